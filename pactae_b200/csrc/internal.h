@@ -259,6 +259,11 @@ struct Ctx {
   // or -1: the enqueue functions then skip the kernels that mode would gate
   // off.  -1 (unknown) enqueues everything and the device picks.
   int known_mode = -1;
+  // A solve in passes (solve_begin / solve_advance): the pass enqueued last,
+  // and where its match goes.
+  int pass = 0;
+  uint32_t pass_flags = 0;
+  int32_t *pass_match = nullptr;
 
   DeviceBuf d_pref_m, d_pref_w, d_rank, d_rankT, d_pr, d_prefix, d_bid, d_tailq, d_seen, d_ctrl, d_match;
   DeviceBuf d_pw16, d_pm16;  // pref_w and pref_m packed to uint16 (host-input solves)
@@ -333,10 +338,17 @@ inline cudaError_t allow_dynamic_smem(const Ctx &c, Kernel kernel) {
   return allow_dynamic_smem_ptr(c, reinterpret_cast<const void *>(kernel));
 }
 
-// smp_b200.cu: a whole solve split into its asynchronous part and its
-// completion (the public smp_b200_solve is the two with a sync between).
+// smp_b200.cu: a whole solve split into its asynchronous parts and its
+// completion.  solve_enqueue needs no host round trip (a captured step);
+// solve_begin enqueues the first of at most three passes and solve_advance,
+// called when the stream has drained, the next (more = false: none is left,
+// call solve_finish).
+enum Pass : int { kPassLast = 0, kPassQuery = 1, kPassPrecheck = 2, kPassScreen = 3 };
 int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
                   uint32_t flags);
+int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
+                uint32_t flags);
+int solve_advance(Ctx &c, bool &more);
 int solve_finish(Ctx &c, uint32_t flags, smp_stats *st);
 int reserve_buffers(Ctx &c, int32_t n);
 

@@ -305,6 +305,13 @@ int init_buffers(Ctx &c) {
   return SMP_OK;
 }
 
+// Buffers of the women-proposing solve.
+int swap_buffers(Ctx &c) {
+  int rc = c.d_swap_pos.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
+  if (!rc) rc = c.d_bid.ensure(sizeof(unsigned long long) * static_cast<size_t>(c.n));
+  return rc ? rc : c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
+}
+
 int enqueue_init(Ctx &c) {
   int rc = init_buffers(c);
   if (rc) return rc;
@@ -630,6 +637,7 @@ int reserve_buffers(Ctx &c, int32_t n) {
   if (!rc && c.query_ok) rc = c.d_qcnt.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && c.query_ok)
     rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * query_capacity(n, c.K));
+  if (!rc) rc = swap_buffers(c);
   if (!rc) rc = c.d_husband.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc) rc = c.d_prank.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc) rc = c.sync("reserve");
@@ -668,111 +676,60 @@ int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t 
   return rc;
 }
 
-// The synchronous solve, in one pass when the precheck picks the query mode
-// (uniform-like inputs): the pass enqueues only that mode's kernels -- the
+// A solve in passes: solve_begin enqueues the first, and each time the stream
+// has drained solve_advance reads the control block back and enqueues the
+// next one, if any.  The first pass assumes that the precheck picks the query
+// mode (uniform-like inputs) and enqueues that mode's kernels only -- the
 // bulk restricted to it, so a rank-mode instance cannot start proposing
-// before its ranks exist -- through the match copy, and the host waits once.
+// before its ranks exist -- through the match copy: most solves end there.
 // If the precheck chose the rank mode, or a man went beyond his prefix, a
-// second pass enqueues what remains and copies the match again.  Kernels a
-// mode gates off would still cost a launch and a pass of every CTA over the
-// gate: 14 of them took about 0.1 ms of a 2.6 ms uniform solve at
+// second pass enqueues what remains and copies the match again; men who all
+// make the same first choice are screened for a shared list before it.
+// Kernels a mode gates off would still cost a launch and a pass of every CTA
+// over the gate: 14 of them took about 0.1 ms of a 2.6 ms uniform solve at
 // n = 30000, where a wait for the precheck costs about 30 us.  The kernels
-// keep their gates, so the device still decides what runs.  The checker
-// (SMP_F_CHECK) must see the final matching: those solves take the fully
-// gated pipeline.
-int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped, bool men_screened = false);
+// keep their gates, so the device still decides what runs.
+//   The checker (SMP_F_CHECK) must see the final matching; it, a disabled tail
+// and a configured tail window (whose tail kernel serves either mode) take
+// the fully gated pipeline, in one pass.
 
-int solve_staged(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
-                 uint32_t flags, smp_stats *st) {
-  // the checker, a disabled tail or a configured tail window (whose tail
-  // kernel serves either mode) take the fully gated pipeline.  The tail is
-  // this n's (plan), not the previous solve's: a fresh context's first solve
-  // would otherwise always take the gated pipeline.
-  if (n > 0 && n <= SMP_B200_MAX_N) {
-    c.n = n;
-    plan(c);
-  }
-  if ((flags & SMP_F_CHECK) || !(c.tail_threshold > 0) || c.tail_window_cfg > 0) {
-    int rc = solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
-    if (!rc) rc = c.sync("solve");
-    return rc ? rc : solve_finish(c, flags, st);
-  }
-  int rc = do_stage(c, pref_m, pref_w, n, flags);
-  if (rc) return rc;
-  const auto finish_pass = [&]() {
-    int r = SMP_OK;
-    if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) r = c.fail_cuda("event");
-    if (!r) r = enqueue_post(c);
-    if (!r && (flags & SMP_F_DEVICE_PTRS)) r = copy_match_out(c, match_out, true);
-    if (!r && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) r = c.fail_cuda("event");
-    if (!r && !(flags & SMP_F_DEVICE_PTRS)) r = copy_match_out(c, match_out, false);
-    if (!r) r = read_control(c);
-    if (!r) r = c.sync("solve");
-    return r;
-  };
-  // pass 1: as if the precheck picks the query mode
-  rc = enqueue_precheck(c, (flags & SMP_F_NO_PRECHECK) == 0);
-  if (!rc && (flags & SMP_F_VALIDATE)) rc = enqueue_validate(c);
-  if (!rc && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  const bool speculate = c.query_ok;
-  if (speculate) {
-    c.known_mode = kModeQuery;
-    if (!rc) rc = enqueue_init(c);
-    if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-    if (!rc) rc = enqueue_core(c);
-    if (!rc) rc = finish_pass();
-  } else {
-    if (!rc) rc = read_control(c);
-    if (!rc) rc = c.sync("precheck");
-  }
-  if (rc) return rc;
-  const Control &h = *c.h_ctrl;
-  const bool done = speculate && !h.status && (h.perfect || (h.mode == kModeQuery && !h.retry));
-  if (!done && !h.status) {
-    // pass 2: the rank mode, or the rank-mode retry of a query-mode round 0
-    bool swapped = false;
-    if (speculate && h.mode == kModeQuery && h.retry) {
-      c.known_mode = -1;
-      rc = c.rank_bytes == 2 ? enqueue_retry_round<uint16_t>(c) : enqueue_retry_round<int32_t>(c);
-    } else {
-      // one first choice for every man: perhaps one list for every man
-      if (!h.perfect && h.mode == kModeRank && h.distinct == 1 && n >= 2 && c.mode_cfg == 0)
-        rc = solve_swapped(c, flags, match_out, swapped);
-      if (!rc && !swapped) {
-        c.known_mode = h.perfect ? -1 : h.mode;
-        rc = enqueue_init(c);
-        if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-        if (!rc) rc = enqueue_core(c);
-      }
-    }
-    if (!rc && !swapped) rc = finish_pass();
-    if (rc) return rc;
-  }
-  return solve_finish(c, flags, st);
+namespace {
+
+// Ends a pass: post, the match copy, the control block's readback.
+int enqueue_pass_end(Ctx &c) {
+  const bool device = (c.pass_flags & SMP_F_DEVICE_PTRS) != 0;
+  if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
+  int rc = enqueue_post(c);
+  if (!rc && device) rc = copy_match_out(c, c.pass_match, true);
+  if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (!rc && !device) rc = copy_match_out(c, c.pass_match, false);
+  return rc ? rc : read_control(c);
 }
 
-// A rank-mode solve whose men all make the same first choice may have men
-// who share one list.  The screen checks that on all SMs (and that pref_w's
-// rows are permutations); if so, the women propose and `swapped` is set,
-// else the caller runs the men's rank-mode pass.  Stops after the screen,
-// with `swapped` set, when it found invalid input.
-int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped, bool men_screened) {
-  swapped = false;
+// Init and core of the mode the control block names (either, if unknown).
+int enqueue_pass_mode(Ctx &c, int mode) {
+  c.known_mode = mode;
+  int rc = enqueue_init(c);
+  if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (!rc) rc = enqueue_core(c);
+  return rc ? rc : enqueue_pass_end(c);
+}
+
+// Rank-mode men who all make the same first choice may share one list.  The
+// screen checks that on all SMs (and that pref_w's rows are permutations).
+bool swap_screen_fits(const Ctx &c) { return swap_screen_smem(c.n) <= c.smem_optin; }
+
+int enqueue_swap_screen(Ctx &c, bool men_screened) {
   const int n = c.n;
-  const size_t screen_smem = swap_screen_smem(n);
-  if (screen_smem > c.smem_optin) return SMP_OK;
-  int rc = c.d_swap_pos.ensure(sizeof(int32_t) * static_cast<size_t>(n));
-  if (!rc) rc = c.d_bid.ensure(sizeof(unsigned long long) * static_cast<size_t>(n));
-  if (!rc) rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(n));
+  int rc = swap_buffers(c);
   if (rc) return rc;
   Control *ctrl = c.d_ctrl.as<Control>();
   int32_t *pos = c.d_swap_pos.as<int32_t>();
-  unsigned long long *bid = c.d_bid.as<unsigned long long>();
-  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
   if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("swap reset");
-  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl);
+  k_swap_pos<<<std::max(1, std::min(c.sm_count * 4, (n + 255) / 256)), 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl);
   if (allow_dynamic_smem(c, k_swap_screen) != cudaSuccess) return c.fail_cuda("k_swap_screen smem attribute");
+  const size_t screen_smem = swap_screen_smem(n);
   int per_sm = 0;  // one wave: every CTA resident
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_swap_screen, 256, screen_smem) != cudaSuccess) {
     cudaGetLastError();
@@ -784,16 +741,19 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped, boo
   c.launches += 2;
   rc = c.check_launch("k_swap_screen");
   if (!rc && cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (!rc) rc = read_control(c);
-  if (!rc) rc = c.sync("swap screen");
-  if (rc) return rc;
-  if (c.h_ctrl->status) {
-    swapped = true;
-    return SMP_OK;
-  }
-  if (c.h_ctrl->swap_fail) return SMP_OK;
-  swapped = true;
+  return rc ? rc : read_control(c);
+}
+
+// The screen found one shared list: the women propose, or, when they share
+// one list too, the sides pair rank for rank.
+int enqueue_swap_solve(Ctx &c) {
+  const int n = c.n;
   c.swapped = true;
+  Control *ctrl = c.d_ctrl.as<Control>();
+  int32_t *pos = c.d_swap_pos.as<int32_t>();
+  unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
+  int rc;
   if (!c.h_ctrl->w_differ) {  // the women share one list too: pair rank for rank
     if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
     if (cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
@@ -816,9 +776,88 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped, boo
     c.launches++;
     rc = c.check_launch("k_swap_match");
   }
-  if (!rc) rc = copy_match_out(c, match_out, (flags & SMP_F_DEVICE_PTRS) != 0);
+  if (!rc) rc = copy_match_out(c, c.pass_match, (c.pass_flags & SMP_F_DEVICE_PTRS) != 0);
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (!rc) rc = read_control(c);
+  return rc ? rc : read_control(c);
+}
+
+}  // namespace
+
+int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
+                uint32_t flags) {
+  // The tail is this n's (plan), not the previous solve's: a fresh context's
+  // first solve would otherwise always take the gated pipeline.
+  if (n > 0 && n <= SMP_B200_MAX_N) {
+    c.n = n;
+    plan(c);
+  }
+  c.pass_flags = flags;
+  c.pass_match = match_out;
+  if ((flags & SMP_F_CHECK) || !(c.tail_threshold > 0) || c.tail_window_cfg > 0) {
+    c.pass = kPassLast;
+    return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
+  }
+  int rc = do_stage(c, pref_m, pref_w, n, flags);
+  if (!rc) rc = enqueue_precheck(c, (flags & SMP_F_NO_PRECHECK) == 0);
+  if (!rc && (flags & SMP_F_VALIDATE)) rc = enqueue_validate(c);
+  if (!rc && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (rc) return rc;
+  c.pass = c.query_ok ? kPassQuery : kPassPrecheck;
+  return c.query_ok ? enqueue_pass_mode(c, kModeQuery) : read_control(c);
+}
+
+int solve_advance(Ctx &c, bool &more) {
+  more = false;
+  const Control &h = *c.h_ctrl;
+  if (c.pass == kPassLast || h.status) return SMP_OK;
+  const bool queried = c.pass == kPassQuery;
+  if (queried && (h.perfect || (h.mode == kModeQuery && !h.retry))) return SMP_OK;
+  more = true;
+  if (c.pass == kPassScreen && !h.swap_fail) {
+    c.pass = kPassLast;
+    return enqueue_swap_solve(c);
+  }
+  if (queried && h.mode == kModeQuery) {  // the rank-mode retry of a query-mode round 0
+    c.pass = kPassLast;
+    c.known_mode = -1;
+    const int rc = c.rank_bytes == 2 ? enqueue_retry_round<uint16_t>(c) : enqueue_retry_round<int32_t>(c);
+    return rc ? rc : enqueue_pass_end(c);
+  }
+  // one first choice for every man: perhaps one list for every man
+  if (c.pass != kPassScreen && !h.perfect && h.mode == kModeRank && h.distinct == 1 && c.n >= 2 && c.mode_cfg == 0 &&
+      swap_screen_fits(c)) {
+    c.pass = kPassScreen;
+    return enqueue_swap_screen(c, false);
+  }
+  c.pass = kPassLast;
+  return enqueue_pass_mode(c, h.perfect ? -1 : h.mode);
+}
+
+// The synchronous solve.
+int solve_staged(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
+                 uint32_t flags, smp_stats *st) {
+  int rc = solve_begin(c, pref_m, pref_w, n, match_out, flags);
+  for (bool more = true; !rc && more;) {
+    rc = c.sync("solve");
+    if (!rc) rc = solve_advance(c, more);
+  }
+  return rc ? rc : solve_finish(c, flags, st);
+}
+
+// The screen and the solve after it, for a host-input solve whose host
+// threads have compared the men's rows.  `swapped` is set when it solved the
+// instance or found invalid input; else the caller runs the men's rank mode.
+int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
+  swapped = false;
+  if (!swap_screen_fits(c)) return SMP_OK;
+  c.pass_flags = flags;
+  c.pass_match = match_out;
+  int rc = enqueue_swap_screen(c, true);
+  if (!rc) rc = c.sync("swap screen");
+  if (rc) return rc;
+  swapped = c.h_ctrl->status || !c.h_ctrl->swap_fail;
+  if (!swapped || c.h_ctrl->status) return SMP_OK;
+  rc = enqueue_swap_solve(c);
   if (!rc) rc = c.sync("solve");
   return rc;
 }
@@ -1210,7 +1249,7 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
     }
     if (!rc && !swapped && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess)
       rc = c.fail_cuda("event");
-    if (!rc && shared && !swapped) rc = solve_swapped(c, flags, match_out, swapped, true);
+    if (!rc && shared && !swapped) rc = solve_swapped(c, flags, match_out, swapped);
     if (!rc && !swapped) rc = enqueue_init(c);
     if (!rc && !swapped && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
     if (!rc && !swapped) rc = enqueue_core(c);
