@@ -51,6 +51,8 @@ struct Control {
   int32_t swap_next;      // k_swap_gs: next woman that has not proposed yet
   int32_t w_differ;       // k_swap_screen: a pref_w row differs from row 0
   int32_t swap_over;      // k_swap_gs: women stopped at the end of what the device holds of their rows
+  int32_t round_done;     // k_round: the matching is complete and written
+  int32_t round_pad;
   int2 coop_chain[32];
 };
 

@@ -264,6 +264,12 @@ struct Ctx {
   int pass = 0;
   uint32_t pass_flags = 0;
   int32_t *pass_match = nullptr;
+  // Rank mode in rounds: the steps enqueued so far and their gate; with
+  // poll_rounds the caller reads the control block back and adds steps until
+  // the matching is complete.
+  bool poll_rounds = false;
+  int round_step = 0;
+  int round_gate = 0;
 
   DeviceBuf d_pref_m, d_pref_w, d_rank, d_rankT, d_pr, d_prefix, d_bid, d_tailq, d_seen, d_ctrl, d_match;
   DeviceBuf d_pw16, d_pm16;  // pref_w and pref_m packed to uint16 (host-input solves)
@@ -276,6 +282,8 @@ struct Ctx {
   std::unique_ptr<HostPool> pack_pool;
   std::unique_ptr<HostLink> link;
   DeviceBuf d_husband, d_prank;
+  // rank mode: the men's starting order and the rounds' state (round_kernels.cuh)
+  DeviceBuf d_order, d_score, d_round;
   DeviceBuf d_qcnt, d_qlist;
   DeviceBuf gen_keys_a, gen_keys_b, gen_seg, gen_temp, gen_aux;
   Control *h_ctrl = nullptr;  // pinned host copy of the control block
@@ -285,11 +293,11 @@ struct Ctx {
   static constexpr int kCopyChunks = 16;
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t ev_chunk[kCopyChunks] = {};
-  std::array<DeviceBuf *, 26> buffers() {
+  std::array<DeviceBuf *, 29> buffers() {
     return {&d_pref_m, &d_pref_w, &d_pw16, &d_pm16, &d_rank,    &d_rankT,    &d_pr,     &d_prefix, &d_bid,    &d_tailq,
             &d_seen,   &d_ctrl,   &d_match,   &d_husband,  &d_prank,  &d_qcnt,   &d_qlist,
             &gen_keys_a, &gen_keys_b, &gen_seg, &gen_temp, &gen_aux, &d_swap_pos, &d_swap_full, &d_swap_over,
-            &d_swap_rows};
+            &d_swap_rows, &d_order, &d_score, &d_round};
   }
   int launches = 0;  // kernels launched since the last stage / call
   smp_stats stats = {};
@@ -340,7 +348,7 @@ inline cudaError_t allow_dynamic_smem(const Ctx &c, Kernel kernel) {
 
 // smp_b200.cu: a whole solve split into its asynchronous parts and its
 // completion.  solve_enqueue needs no host round trip (a captured step);
-// solve_begin enqueues the first of at most three passes and solve_advance,
+// solve_begin enqueues the first of its passes and solve_advance,
 // called when the stream has drained, the next (more = false: none is left,
 // call solve_finish).
 enum Pass : int { kPassLast = 0, kPassQuery = 1, kPassPrecheck = 2, kPassScreen = 3 };

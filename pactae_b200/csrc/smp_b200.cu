@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "round_kernels.cuh"
 #include "solve_kernels.cuh"
 #include "swap_kernels.cuh"
 
@@ -29,7 +30,6 @@ int query_capacity(int n, int K) { return std::min(n, K + K / 2 + 32); }
 // Rank-mode host-input solves send each list in this many row groups.
 constexpr int kRankGroups = 8;
 constexpr int kStreamMinN = 4096;
-constexpr int kRankTailWindow = 256;
 // Chains left when k_tail hands the rest to k_tail_coop (one at a time, the
 // whole CTA scanning each).
 constexpr int kCoopChains = 4;
@@ -116,7 +116,7 @@ void plan(Ctx &c) {
   c.bulk_window = c.bulk_window_cfg > 0 ? c.bulk_window_cfg : kDefaultBulkWindow;
   c.tail_window = c.tail_window_cfg > 0 ? c.tail_window_cfg : kDefaultTailWindow;
   c.tail_threshold = 0;
-  if (c.tail_threshold_cfg >= 0 && n <= kU16MaxN && tail_smem_bytes(n) <= c.smem_optin)
+  if (c.tail_threshold_cfg >= 0 && n <= kU16MaxN && tail_smem_bytes(n) + 256 <= c.smem_optin)
     c.tail_threshold = c.tail_threshold_cfg > 0 ? c.tail_threshold_cfg : kDefaultTailThreshold;
   c.tail_threshold_rank = c.tail_threshold_cfg > 0 ? c.tail_threshold_cfg : kDefaultRankTailThreshold;
 }
@@ -135,8 +135,19 @@ int enqueue_precheck(Ctx &c, bool allow_perfect) {
   return c.check_launch("k_precheck");
 }
 
+// Entries per row of the rank matrices: uint16 rows are padded to 16 bytes.
+size_t rank_ld(const Ctx &c) {
+  return c.rank_bytes == 2 ? (static_cast<size_t>(c.n) + 7) & ~static_cast<size_t>(7) : static_cast<size_t>(c.n);
+}
+size_t rank_matrix_bytes(const Ctx &c) { return static_cast<size_t>(c.n) * rank_ld(c) * c.rank_bytes; }
+
+// Rank mode runs in rounds (round_kernels.cuh) when the ranks are uint16 and
+// one SM holds the bids; else through k_bulk.
+bool in_rounds(const Ctx &c) { return c.rank_bytes == 2 && c.tail_threshold > 0; }
+
+// Rows of int32 ranks have ld = n.
 template <typename RankT>
-int enqueue_invert(Ctx &c, const int32_t *pref_w, RankT *rank, int gate) {
+int enqueue_invert(Ctx &c, const int32_t *pref_w, RankT *rank, size_t ld, int gate) {
   const int n = c.n;
   const size_t smem16 = row_smem_bytes<uint16_t>(n);  // n <= 65535: at most 131 KB
   if constexpr (std::is_same<RankT, int32_t>::value) {
@@ -170,39 +181,59 @@ int enqueue_invert(Ctx &c, const int32_t *pref_w, RankT *rank, int gate) {
       per_sm = 1;
     }
     const int grid = std::min(n, c.sm_count * std::max(per_sm, 1));
-    k_invert<RankT><<<grid, 512, smem16, c.stream>>>(pref_w, rank, n, c.d_ctrl.as<Control>(), gate);
+    k_invert<RankT><<<grid, 512, smem16, c.stream>>>(pref_w, rank, ld, n, c.d_ctrl.as<Control>(), gate);
     c.launches++;
     return c.check_launch("k_invert");
   }
 }
 
 int enqueue_invert_any(Ctx &c, int gate) {
-  return c.rank_bytes == 2 ? enqueue_invert<uint16_t>(c, c.pref_w, c.d_rank.as<uint16_t>(), gate)
-                           : enqueue_invert<int32_t>(c, c.pref_w, c.d_rank.as<int32_t>(), gate);
+  return c.rank_bytes == 2 ? enqueue_invert<uint16_t>(c, c.pref_w, c.d_rank.as<uint16_t>(), rank_ld(c), gate)
+                           : enqueue_invert<int32_t>(c, c.pref_w, c.d_rank.as<int32_t>(), rank_ld(c), gate);
 }
 
-// The rank matrix a solve's proposals read: inverted (woman-major, kept for
-// the checker) and transposed to man-major (d_rankT).
+// The men's starting order (k_order_*), from the woman-major ranks.
+int enqueue_order(Ctx &c, int gate) {
+  const int n = c.n;
+  Control *ctrl = c.d_ctrl.as<Control>();
+  uint32_t *score = c.d_score.as<uint32_t>();
+  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
+  if (c.rank_bytes == 2)
+    k_order_score<<<grid, 256, 0, c.stream>>>(c.d_rank.as<uint16_t>(), rank_ld(c), score, n, ctrl, gate);
+  else
+    k_order_score<<<grid, 256, 0, c.stream>>>(c.d_rank.as<int32_t>(), rank_ld(c), score, n, ctrl, gate);
+  k_order_sort<<<1, 1024, 0, c.stream>>>(score, c.d_order.as<int32_t>(), n, ctrl, gate);
+  c.launches += 2;
+  return c.check_launch("k_order");
+}
+
+int order_buffers(Ctx &c) {
+  int rc = c.d_order.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
+  return rc ? rc : c.d_score.ensure(sizeof(uint32_t) * static_cast<size_t>(c.n));
+}
+
+// The rank matrices a solve's proposals read: inverted (woman-major, kept for
+// the checker), the men's starting order taken from it, and transposed to
+// man-major (d_rankT); where k_bulk proposes with uint16 ranks, by position too.
 int enqueue_rank(Ctx &c, int gate) {
-  int rc = c.d_rankT.ensure(static_cast<size_t>(c.n) * c.n * c.rank_bytes);
+  int rc = c.d_rankT.ensure(rank_matrix_bytes(c));
+  if (!rc) rc = order_buffers(c);
   if (!rc) rc = enqueue_invert_any(c, gate);
+  if (!rc) rc = enqueue_order(c, gate);
   if (rc) return rc;
   const int tiles = (c.n + 63) / 64;
   const int grid = static_cast<int>(std::min<long long>(static_cast<long long>(c.sm_count) * 4,
                                                         static_cast<long long>(tiles) * tiles));
-  if (c.rank_bytes == 2 && c.n % 2 == 0)
-    k_transpose_u16x2<<<grid, 512, 0, c.stream>>>(c.d_rank.as<uint16_t>(), c.d_rankT.as<uint16_t>(), c.n,
-                                                  c.d_ctrl.as<Control>(), gate);
-  else if (c.rank_bytes == 2)
-    k_transpose<uint16_t><<<grid, 512, 0, c.stream>>>(c.d_rank.as<uint16_t>(), c.d_rankT.as<uint16_t>(), c.n,
-                                                      c.d_ctrl.as<Control>(), gate);
+  if (c.rank_bytes == 2)
+    k_transpose16<<<grid, 512, 0, c.stream>>>(c.d_rank.as<uint16_t>(), c.d_rankT.as<uint16_t>(), rank_ld(c), c.n,
+                                              c.d_ctrl.as<Control>(), gate);
   else
     k_transpose<int32_t><<<grid, 512, 0, c.stream>>>(c.d_rank.as<int32_t>(), c.d_rankT.as<int32_t>(), c.n,
                                                      c.d_ctrl.as<Control>(), gate);
   c.launches++;
   rc = c.check_launch("k_transpose");
-  if (rc || c.rank_bytes != 2) return rc;
-  // uint16 ranks: proposals read them by position (pr)
+  if (rc || c.rank_bytes != 2 || in_rounds(c)) return rc;
+  // uint16 ranks: k_bulk reads them by position (pr)
   rc = c.d_pr.ensure(static_cast<size_t>(c.n) * c.n * 2);
   if (rc) return rc;
   const size_t smem = row_smem_bytes<uint16_t>(c.n);
@@ -213,10 +244,80 @@ int enqueue_rank(Ctx &c, int gate) {
     per_sm = 1;
   }
   k_pr<<<std::min(c.n, c.sm_count * std::max(per_sm, 1)), 512, smem, c.stream>>>(
-      c.pref_m, c.d_rankT.as<uint16_t>(), c.d_pr.as<uint16_t>(), c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr,
-      c.K > 0 ? c.K : 0, c.n, c.d_ctrl.as<Control>(), gate);
+      c.pref_m, c.d_rankT.as<uint16_t>(), rank_ld(c), c.d_pr.as<uint16_t>(),
+      c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr, c.K > 0 ? c.K : 0, c.n, c.d_ctrl.as<Control>(), gate);
   c.launches++;
   return c.check_launch("k_pr");
+}
+
+// The rounds' buffers, one allocation: candidate lists, words and positions,
+// the parked lists and the control block.
+size_t round_bytes(int n) {
+  return 6 * static_cast<size_t>(round_cap(n)) * n + 8 * round_words(n) + 2 * sizeof(int32_t) * round_words(n) +
+         sizeof(RoundCtl);
+}
+RoundBufs round_bufs(const Ctx &c) {
+  const size_t nw = round_words(c.n);
+  unsigned char *p = c.d_round.as<unsigned char>();
+  RoundBufs b;
+  b.cap = round_cap(c.n);
+  const size_t entries = static_cast<size_t>(b.cap) * c.n;  // a multiple of 8
+  b.cand = reinterpret_cast<uint32_t *>(p);
+  b.cpos = reinterpret_cast<uint16_t *>(p + 4 * entries);
+  p += 6 * entries;
+  b.word = reinterpret_cast<uint32_t *>(p);
+  b.cut = reinterpret_cast<uint16_t *>(p + 4 * nw);
+  b.at = reinterpret_cast<uint16_t *>(p + 6 * nw);
+  p += 8 * nw;
+  for (auto &q : b.parkq) {
+    q = reinterpret_cast<int32_t *>(p);
+    p += 4 * nw;
+  }
+  b.ctl = reinterpret_cast<RoundCtl *>(p);
+  return b;
+}
+
+// The rank-mode proposals in rounds: a step per batch of men, and more for
+// parked men and refreshes.  A step after the matching is complete costs an
+// empty launch (about 2 us).  A caller that reads the control block back
+// (c.poll_rounds) gets kRoundExtra more and adds steps until round_done;
+// otherwise kRoundExtraBlind follow, then the last step, which ends any solve.
+constexpr int kRoundExtra = 1;
+constexpr int kRoundExtraBlind = 12;
+constexpr int kRoundMore = 8;
+
+int enqueue_round_steps(Ctx &c, int gate, int count) {
+  const RoundBufs b = round_bufs(c);
+  if (allow_dynamic_smem(c, k_round) != cudaSuccess) return c.fail_cuda("k_round smem attribute");
+  for (int i = 0; i < count; ++i)
+    k_round<<<c.sm_count, kRoundBlock, round_smem_bytes(c.n), c.stream>>>(
+        c.pref_m, c.d_rankT.as<uint16_t>(), rank_ld(c), c.d_order.as<int32_t>(), b, c.d_match.as<int32_t>(), c.n,
+        c.sm_count * kTeams, c.round_step + i, c.d_ctrl.as<Control>(), gate);
+  c.round_step += count;
+  c.launches += count;
+  return c.check_launch("k_round");
+}
+
+int enqueue_rounds(Ctx &c, int gate) {
+  const int n = c.n;
+  int rc = c.d_round.ensure(round_bytes(n));
+  if (rc) return rc;
+  const RoundBufs b = round_bufs(c);
+  Control *ctrl = c.d_ctrl.as<Control>();
+  const int batch = c.sm_count * kTeams;
+  k_round_reset<<<std::max(1, std::min(c.sm_count, (n + 1023) / 1024)), 1024, 0, c.stream>>>(
+      c.pref_m, b, c.d_match.as<int32_t>(), n, batch, ctrl, gate);
+  c.launches++;
+  c.round_step = 0;
+  c.round_gate = gate;
+  rc = enqueue_round_steps(c, gate, (n + batch - 1) / batch + (c.poll_rounds ? kRoundExtra : kRoundExtraBlind));
+  if (rc || c.poll_rounds) return rc;
+  if (allow_dynamic_smem(c, k_round_last) != cudaSuccess) return c.fail_cuda("k_round_last smem attribute");
+  k_round_last<<<1, kRoundBlock, round_smem_bytes(n), c.stream>>>(c.pref_m, c.d_rankT.as<uint16_t>(), rank_ld(c),
+                                                                  c.d_order.as<int32_t>(), b, c.d_match.as<int32_t>(),
+                                                                  n, c.round_step, ctrl, gate);
+  c.launches++;
+  return c.check_launch("k_round_last");
 }
 
 // The matrix rank-mode proposals read, as rank_layout<RankT>() says.
@@ -293,8 +394,7 @@ int enqueue_query(Ctx &c) {
 // fills partner_rank with n, smp_engine_bamboo.cu:37).
 int init_buffers(Ctx &c) {
   const int n = c.n;
-  const size_t nn = static_cast<size_t>(n) * n;
-  int rc = c.d_rank.ensure(nn * c.rank_bytes);
+  int rc = c.d_rank.ensure(rank_matrix_bytes(c));
   if (!rc) rc = c.d_bid.ensure(sizeof(unsigned long long) * n);
   if (!rc && c.K > 0) rc = c.d_prefix.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * c.K);
   if (!rc) rc = c.d_tailq.ensure(sizeof(int2) * static_cast<size_t>(n));
@@ -332,7 +432,7 @@ int launch_bulk(Ctx &c, int round) {
   const uint32_t *prefix = c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr;
   const int rank_threshold = c.tail_threshold > 0 ? std::min(c.tail_threshold, c.tail_threshold_rank) : 0;
   const size_t filter = sizeof(uint32_t) * static_cast<size_t>(c.n);
-  if (round == 0 && c.known_mode != kModeQuery && filter + 1024 <= c.smem_optin) {  // the filter fits
+  if (!in_rounds(c) && round == 0 && c.known_mode != kModeQuery && filter + 1024 <= c.smem_optin) {  // the filter fits
     // k_wdistinct decides on the device which of the two variants runs
     k_wdistinct<<<1, 1024, sizeof(uint32_t) * ((c.n + 31) / 32), c.stream>>>(c.pref_w, c.n, c.d_ctrl.as<Control>());
     c.launches++;
@@ -349,14 +449,14 @@ int launch_bulk(Ctx &c, int round) {
     }
     kernel<<<c.sm_count * std::max(per_sm, 1), kFilterBlock, filter, c.stream>>>(
         c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-        c.n, c.tail_threshold, rank_threshold, round, -1);
+        c.d_order.as<int32_t>(), c.n, c.tail_threshold, rank_threshold, round, -1);
     c.launches++;
     rc = c.check_launch("k_bulk (filtered)");
     if (rc) return rc;
   }
   k_bulk<RankT, kSub><<<resident_grid(c, k_bulk<RankT, kSub>, 256), 256, 0, c.stream>>>(
       c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-      c.n, c.tail_threshold, rank_threshold, round, c.known_mode);
+      c.d_order.as<int32_t>(), c.n, c.tail_threshold, rank_threshold, round, in_rounds(c) ? kModeQuery : c.known_mode);
   c.launches++;
   return c.check_launch("k_bulk");
 }
@@ -369,7 +469,7 @@ int launch_tail(Ctx &c, int round, int only_mode) {
   if (allow_dynamic_smem(c, k_tail<RankT, kSub>) != cudaSuccess) return c.fail_cuda("k_tail smem attribute");
   k_tail<RankT, kSub><<<1, 1024, smem, c.stream>>>(c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(),
                                                    c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-                                                   c.d_match.as<int32_t>(), c.n, round, only_mode, kCoopChains);
+                                                   c.d_order.as<int32_t>(), c.d_match.as<int32_t>(), c.n, round, only_mode, kCoopChains);
   c.launches++;
   int rc = c.check_launch("k_tail");
   if (rc) return rc;
@@ -404,24 +504,42 @@ int launch_tail_window(Ctx &c, int window, int round, int only_mode) {
 }
 
 template <typename RankT>
-int enqueue_round(Ctx &c, int round) {
-  int rc;
+int enqueue_bulk(Ctx &c, int round) {
   switch (subs_for(c.bulk_window)) {
-    case 1: rc = launch_bulk<RankT, 1>(c, round); break;
-    case 2: rc = launch_bulk<RankT, 2>(c, round); break;
-    case 4: rc = launch_bulk<RankT, 4>(c, round); break;
-    default: rc = launch_bulk<RankT, 8>(c, round); break;
+    case 1: return launch_bulk<RankT, 1>(c, round);
+    case 2: return launch_bulk<RankT, 2>(c, round);
+    case 4: return launch_bulk<RankT, 4>(c, round);
+    default: return launch_bulk<RankT, 8>(c, round);
   }
+}
+
+// uint16 ranks with a tail: the query mode is k_bulk and k_tail_q, the rank
+// mode the rounds; with the mode unknown both are enqueued and the device
+// runs one.
+int enqueue_round_rounds(Ctx &c, int round) {
+  int rc = SMP_OK;
+  const bool query = round == 0 && c.query_ok && c.known_mode != kModeRank;
+  if (query) rc = enqueue_bulk<uint16_t>(c, round);
+  if (!rc && !query && c.known_mode != kModeQuery) rc = enqueue_rounds(c, round == 0 ? kGateModeRank : kGateRetry);
   if (rc) return rc;
   if (round == 0 && cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  if (c.tail_threshold <= 0) return SMP_OK;
-  if (round == 1 || !c.query_ok || c.tail_window_cfg > 0) return launch_tail_window<RankT>(c, c.tail_window, round, -1);
-  // Query-mode instances end in short chains, every choice in the prefix
-  // (k_tail_q); rank-mode ones in deep scans (wide look-ahead).  Both are
-  // enqueued and the device runs the one for the mode the precheck chose.
-  if (c.known_mode != kModeRank) rc = launch_tail_query(c);
-  if (!rc && c.known_mode != kModeQuery) rc = launch_tail_window<RankT>(c, kRankTailWindow, round, kModeRank);
+  if (query) {
+    rc = launch_tail_query(c);
+    if (!rc && c.known_mode != kModeQuery) rc = enqueue_rounds(c, kGateModeRank);
+  }
   return rc;
+}
+
+template <typename RankT>
+int enqueue_round(Ctx &c, int round) {
+  if (in_rounds(c)) return enqueue_round_rounds(c, round);
+  int rc = enqueue_bulk<RankT>(c, round);
+  if (rc) return rc;
+  if (round == 0 && cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
+  if constexpr (std::is_same<RankT, int32_t>::value) {
+    if (c.tail_threshold > 0) return launch_tail_window<RankT>(c, c.tail_window, round, -1);
+  }
+  return SMP_OK;
 }
 
 // Rank-mode retry round; every kernel of it returns at once unless the
@@ -434,6 +552,12 @@ int enqueue_retry_round(Ctx &c) {
   if (!rc) rc = enqueue_rank(c, kGateRetry);
   if (!rc) rc = enqueue_round<RankT>(c, 1);
   return rc;
+}
+
+// Rounds of a polled solve that has been read back are not finished.
+bool rounds_left(const Ctx &c) {
+  const Control &h = *c.h_ctrl;
+  return c.poll_rounds && c.round_step > 0 && !h.status && !h.perfect && !h.round_done;
 }
 
 template <typename RankT>
@@ -500,9 +624,9 @@ int enqueue_check_t(Ctx &c, const int32_t *match) {
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
   k_check_husband<<<grid, 256, 0, c.stream>>>(match, c.d_husband.as<int32_t>(), n, c.d_ctrl.as<Control>());
   k_check_prank<RankT><<<grid, 256, 0, c.stream>>>(c.d_husband.as<int32_t>(), reinterpret_cast<const RankT *>(c.d_rank.ptr),
-                                                  c.d_prank.as<int32_t>(), n, c.d_ctrl.as<Control>());
+                                                  rank_ld(c), c.d_prank.as<int32_t>(), n, c.d_ctrl.as<Control>());
   const int sgrid = std::max(1, std::min(c.sm_count * 8, (n * 32 + 255) / 256));
-  k_check_scan<RankT><<<sgrid, 256, 0, c.stream>>>(c.pref_m, reinterpret_cast<const RankT *>(c.d_rank.ptr), match,
+  k_check_scan<RankT><<<sgrid, 256, 0, c.stream>>>(c.pref_m, reinterpret_cast<const RankT *>(c.d_rank.ptr), rank_ld(c), match,
                                                   c.d_prank.as<int32_t>(), n, c.d_ctrl.as<Control>());
   c.launches += 3;
   return c.check_launch("k_check");
@@ -523,6 +647,8 @@ int stage_reset(Ctx &c, int32_t n) {
   c.stats.blocking_pairs = -1;
   c.launches = 0;
   c.known_mode = -1;
+  c.poll_rounds = false;
+  c.round_step = 0;
   c.swapped = false;
   plan(c);
   return SMP_OK;
@@ -628,12 +754,13 @@ void trim_device_pool(int device) {
 int reserve_buffers(Ctx &c, int32_t n) {
   if (n <= 0 || n > SMP_B200_MAX_N) return SMP_ERR_INVALID_ARG;
   stage_reset(c, n);
-  const size_t nn = static_cast<size_t>(n) * n;
   int rc = c.d_ctrl.ensure(sizeof(Control));
   if (!rc) rc = c.d_seen.ensure(((static_cast<size_t>(n) + 31) / 32) * 4);
   if (!rc) rc = init_buffers(c);
-  if (!rc) rc = c.d_rankT.ensure(nn * c.rank_bytes);
-  if (!rc && c.rank_bytes == 2) rc = c.d_pr.ensure(nn * 2);
+  if (!rc) rc = c.d_rankT.ensure(rank_matrix_bytes(c));
+  if (!rc) rc = order_buffers(c);
+  if (!rc && in_rounds(c)) rc = c.d_round.ensure(round_bytes(n));
+  if (!rc && c.rank_bytes == 2 && !in_rounds(c)) rc = c.d_pr.ensure(static_cast<size_t>(n) * n * 2);
   if (!rc && c.query_ok) rc = c.d_qcnt.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && c.query_ok)
     rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * query_capacity(n, c.K));
@@ -809,10 +936,17 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
 int solve_advance(Ctx &c, bool &more) {
   more = false;
   const Control &h = *c.h_ctrl;
-  if (c.pass == kPassLast || h.status) return SMP_OK;
+  if (h.status) return SMP_OK;
+  if (c.pass == kPassLast) {
+    if (!rounds_left(c)) return SMP_OK;
+    more = true;  // parked men the enqueued steps did not reach
+    const int rc = enqueue_round_steps(c, c.round_gate, kRoundMore);
+    return rc ? rc : enqueue_pass_end(c);
+  }
   const bool queried = c.pass == kPassQuery;
   if (queried && (h.perfect || (h.mode == kModeQuery && !h.retry))) return SMP_OK;
   more = true;
+  c.poll_rounds = in_rounds(c);
   if (c.pass == kPassScreen && !h.swap_fail) {
     c.pass = kPassLast;
     return enqueue_swap_solve(c);
@@ -1207,6 +1341,7 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
   };
   const bool query = c.h_ctrl->mode == kModeQuery && !c.h_ctrl->perfect;
   if (!c.h_ctrl->perfect) c.known_mode = c.h_ctrl->mode;  // enqueue only this mode's kernels
+  c.poll_rounds = in_rounds(c);
   bool swapped = false;
   if (!query) {
     // One first choice for every man: perhaps one list for every man.  Then
@@ -1294,12 +1429,16 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
       if (!rc) rc = enqueue_retry_round<uint16_t>(c);
     }
   }
-  if (!swapped) {  // the women-proposing pass has finished its solve
-    if (!rc && cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  while (!rc && !swapped) {  // the women-proposing pass has finished its solve
+    if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
     if (!rc) rc = enqueue_post(c);
     if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
     if (!rc) rc = copy_match_out(c, match_out, false);
     if (!rc) rc = read_control(c);
+    if (rc || c.round_step == 0) break;
+    rc = c.sync("solve");
+    if (rc || !rounds_left(c)) break;
+    rc = enqueue_round_steps(c, c.round_gate, kRoundMore);
   }
   // Both streams drain before returning, even after an error: the copies
   // read the caller's buffers.
@@ -1552,7 +1691,7 @@ int smp_b200_invert(smp_ctx *ctx, const int32_t *pref_w, int32_t n, int32_t *ran
   }
   if (cudaMemsetAsync(c.d_ctrl.ptr, 0, sizeof(Control), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   if (cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  rc = enqueue_invert<int32_t>(c, src, dst, kGateAlways);
+  rc = enqueue_invert<int32_t>(c, src, dst, static_cast<size_t>(n), kGateAlways);
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   if (!(flags & SMP_F_DEVICE_PTRS)) {
@@ -1589,7 +1728,7 @@ int smp_b200_check(smp_ctx *ctx, const int32_t *pref_m, const int32_t *pref_w, i
   rc = enqueue_precheck(c, false);
   if (rc) return rc;
   c.rank_bytes = c.rank_bytes_cfg == 4 ? 4 : rank_bytes_for(n);
-  rc = c.d_rank.ensure(static_cast<size_t>(n) * n * c.rank_bytes);
+  rc = c.d_rank.ensure(rank_matrix_bytes(c));
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvCheckBegin], c.stream) != cudaSuccess) return c.fail_cuda("event");
   rc = enqueue_invert_any(c, kGateAlways);

@@ -206,7 +206,7 @@ __device__ __forceinline__ void load_row(const int32_t *__restrict__ row, RankT 
 
 template <typename RankT>
 __global__ void __launch_bounds__(512) k_invert(const int32_t *__restrict__ pref_w, RankT *__restrict__ rank,
-                                                int n, Control *ctrl, int gate) {
+                                                size_t ld, int n, Control *ctrl, int gate) {
   if (!gate_open(gate, ctrl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RankT *sbuf = reinterpret_cast<RankT *>(smem_raw);
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(512) k_invert(const int32_t *__restrict__ pref
   const RankT unset = rank_unset<RankT>();
   bool bad = false;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
-    RankT *out = rank + static_cast<size_t>(w) * n;
+    RankT *out = rank + static_cast<size_t>(w) * ld;
     const int pre = static_cast<int>((reinterpret_cast<uintptr_t>(out) & 15u) / sizeof(RankT));
     const int chunks = (pre + n + kPerVec - 1) / kPerVec;
     load_row(pref_w + static_cast<size_t>(w) * n, sbuf, sbuf + pre, chunks, n, bad);
@@ -326,37 +326,37 @@ __global__ void k_invert_verify(const int32_t *__restrict__ pref_w, const int32_
 // he scans.  Tiles of 64 x 64 go through shared memory so that both the
 // reads and the writes are coalesced; a persistent grid walks the tiles.
 // ---------------------------------------------------------------------------
-// uint16 with n even: every row starts 4-byte aligned, so pairs of elements
-// move as one 32-bit word and a warp reads or writes 128 bytes of a row.
-__global__ void __launch_bounds__(512) k_transpose_u16x2(const uint16_t *__restrict__ src, uint16_t *__restrict__ dst,
-                                                         int n, Control *ctrl, int gate) {
+// uint16, rows of ld entries (a multiple of 8, so every row starts on a
+// 16-byte boundary whatever n is): one 16-byte load and one 16-byte store per
+// thread and tile, a warp covering four whole 128-byte rows of it.  Entries
+// past n are written as 0xFFFF.
+__global__ void __launch_bounds__(512) k_transpose16(const uint16_t *__restrict__ src, uint16_t *__restrict__ dst,
+                                                     size_t ld, int n, Control *ctrl, int gate) {
   if (!gate_open(gate, ctrl)) return;
   __shared__ uint16_t tile[64][66];
-  const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 16
+  const int row = threadIdx.x >> 3, ch = threadIdx.x & 7;  // 64 rows x 8 chunks of 8 entries
   const int tiles = (n + 63) / 64;
   const long long total = static_cast<long long>(tiles) * tiles;
+  const int t_ld = static_cast<int>(ld);
   for (long long t = blockIdx.x; t < total; t += gridDim.x) {
     const int r0 = static_cast<int>(t / tiles) * 64, c0 = static_cast<int>(t % tiles) * 64;
-    const int c = c0 + 2 * lane;  // even, so c < n implies c + 1 < n
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int r = r0 + ty + 16 * k;
-      if (r < n && c < n) {
-        const uint32_t v = *reinterpret_cast<const uint32_t *>(src + static_cast<size_t>(r) * n + c);
-        tile[ty + 16 * k][2 * lane] = static_cast<uint16_t>(v & 0xFFFFu);
-        tile[ty + 16 * k][2 * lane + 1] = static_cast<uint16_t>(v >> 16);
-      }
-    }
+    const int r = r0 + row, c = c0 + 8 * ch;
+    uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
+    if (r < n && c < t_ld) v = __ldcs(reinterpret_cast<const uint4 *>(src + static_cast<size_t>(r) * ld + c));
+    uint32_t *to = reinterpret_cast<uint32_t *>(&tile[row][8 * ch]);  // rows of 33 words
+    to[0] = v.x;
+    to[1] = v.y;
+    to[2] = v.z;
+    to[3] = v.w;
     __syncthreads();
-    const int oc = r0 + 2 * lane;  // output columns are source rows
+    const int orow = c0 + row, oc = r0 + 8 * ch;  // source column, source rows
+    if (orow < n && oc < t_ld) {
+      uint32_t q[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int orow = c0 + ty + 16 * k;  // output rows are source columns
-      if (orow < n && oc < n) {
-        const uint32_t v = static_cast<uint32_t>(tile[2 * lane][ty + 16 * k]) |
-                           (static_cast<uint32_t>(tile[2 * lane + 1][ty + 16 * k]) << 16);
-        *reinterpret_cast<uint32_t *>(dst + static_cast<size_t>(orow) * n + oc) = v;
-      }
+      for (int h = 0; h < 4; ++h)
+        q[h] = static_cast<uint32_t>(tile[8 * ch + 2 * h][row]) |
+               (static_cast<uint32_t>(tile[8 * ch + 2 * h + 1][row]) << 16);
+      *reinterpret_cast<uint4 *>(dst + static_cast<size_t>(orow) * ld + oc) = make_uint4(q[0], q[1], q[2], q[3]);
     }
     __syncthreads();
   }
@@ -648,7 +648,7 @@ __host__ __device__ constexpr int rank_layout() {
 // it.  An out-of-range woman is reported.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(512) k_pr(const int32_t *__restrict__ pref_m, const uint16_t *__restrict__ rankT,
-                                            uint16_t *__restrict__ pr, uint32_t *__restrict__ prefix, int K, int n,
+                                            size_t ld, uint16_t *__restrict__ pr, uint32_t *__restrict__ prefix, int K, int n,
                                             Control *ctrl, int gate) {
   if (!gate_open(gate, ctrl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(512) k_pr(const int32_t *__restrict__ pref_m, 
   const int nthr = blockDim.x;
   bool bad = false;
   for (int m = blockIdx.x; m < n; m += gridDim.x) {
-    const uint16_t *src = rankT + static_cast<size_t>(m) * n;
+    const uint16_t *src = rankT + static_cast<size_t>(m) * ld;
     const int pre = static_cast<int>((reinterpret_cast<uintptr_t>(src) & 15u) >> 1);
     uint16_t *srow = reinterpret_cast<uint16_t *>(smem_raw) + pre;  // same offset from 16 bytes as src
     const int a0 = min(n, (8 - pre) & 7);                           // first element on a 16-byte boundary
@@ -910,8 +910,8 @@ __global__ void __launch_bounds__(1024) k_wdistinct(const int32_t *__restrict__ 
 template <typename RankT, int kMaxSub, bool kFilter = false>
 __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
     k_bulk(const int32_t *__restrict__ pref_m, const RankT *__restrict__ rank, const uint32_t *__restrict__ prefix,
-           int K, unsigned long long *bid, Control *ctrl, int2 *tail_queue, int n, int tail_threshold_query,
-           int tail_threshold_rank, int round, int only_mode = -1) {
+           int K, unsigned long long *bid, Control *ctrl, int2 *tail_queue, const int32_t *__restrict__ order, int n,
+           int tail_threshold_query, int tail_threshold_rank, int round, int only_mode = -1) {
   using Bids = typename std::conditional<kFilter, FilteredBids, GlobalBids>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *lrank = reinterpret_cast<uint32_t *>(smem_raw);
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
       if (lane == 0 && ld_relaxed_s32(&ctrl->free_count) > tail_threshold) v = atomicAdd(&ctrl->next_man, 1);
       v = __shfl_sync(kFullMask, v, 0);
       if (v >= n) break;
-      m = v;
+      m = query ? v : __ldg(order + v);
       pos = 0;
       S = 1;
     }
@@ -1087,6 +1087,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
                                                   const uint32_t *__restrict__ prefix, int K,
                                                   unsigned long long *bid, Control *ctrl,
                                                   const int2 *__restrict__ tail_queue,
+                                                  const int32_t *__restrict__ order,
                                                   int32_t *__restrict__ match, int n, int round,
                                                   int only_mode, int coop_chains) {
   if (only_mode >= 0 && round == 0 && ld_volatile_s32(&ctrl->mode) != only_mode) return;
@@ -1138,6 +1139,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
         pos = e.y;
       } else {
         m = first_unstarted + (i - queued);
+        if (!query) m = __ldg(order + m);
         pos = 0;
       }
       S = 1;
@@ -1598,7 +1600,7 @@ __global__ void k_check_husband(const int32_t *__restrict__ match, int32_t *husb
 }
 
 template <typename RankT>
-__global__ void k_check_prank(const int32_t *__restrict__ husband, const RankT *__restrict__ rank,
+__global__ void k_check_prank(const int32_t *__restrict__ husband, const RankT *__restrict__ rank, size_t ld,
                               int32_t *__restrict__ prank, int n, Control *ctrl) {
   const int stride = gridDim.x * blockDim.x;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += stride) {
@@ -1608,12 +1610,12 @@ __global__ void k_check_prank(const int32_t *__restrict__ husband, const RankT *
       prank[w] = -1;
       continue;
     }
-    prank[w] = static_cast<int32_t>(rank[static_cast<size_t>(w) * n + h]);
+    prank[w] = static_cast<int32_t>(rank[static_cast<size_t>(w) * ld + h]);
   }
 }
 
 template <typename RankT>
-__global__ void k_check_scan(const int32_t *__restrict__ pref_m, const RankT *__restrict__ rank,
+__global__ void k_check_scan(const int32_t *__restrict__ pref_m, const RankT *__restrict__ rank, size_t ld,
                              const int32_t *__restrict__ match, const int32_t *__restrict__ prank, int n,
                              Control *ctrl) {
   const int lane = threadIdx.x & 31;
@@ -1630,7 +1632,7 @@ __global__ void k_check_scan(const int32_t *__restrict__ pref_m, const RankT *__
       const int limit = hit ? (__ffs(hit) - 1) : 32;  // lanes before the wife
       if (lane < limit && r < n && static_cast<unsigned>(w) < static_cast<unsigned>(n)) {
         const int32_t pr = prank[w];
-        if (pr >= 0 && static_cast<int32_t>(rank[static_cast<size_t>(w) * n + m]) < pr) blocking++;
+        if (pr >= 0 && static_cast<int32_t>(rank[static_cast<size_t>(w) * ld + m]) < pr) blocking++;
       }
       if (hit) {
         found = true;
