@@ -281,7 +281,7 @@ struct Ctx {
   // that sends packed rows through them (created on first use).
   std::unique_ptr<HostPool> pack_pool;
   std::unique_ptr<HostLink> link;
-  DeviceBuf d_husband, d_prank;
+  DeviceBuf d_husband, d_prank, d_bits;  // the checker's
   // rank mode: the men's starting order and the rounds' state (round_kernels.cuh)
   DeviceBuf d_order, d_score, d_round;
   DeviceBuf d_qcnt, d_qlist;
@@ -293,11 +293,11 @@ struct Ctx {
   static constexpr int kCopyChunks = 16;
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t ev_chunk[kCopyChunks] = {};
-  std::array<DeviceBuf *, 29> buffers() {
+  std::array<DeviceBuf *, 30> buffers() {
     return {&d_pref_m, &d_pref_w, &d_pw16, &d_pm16, &d_rank,    &d_rankT,    &d_pr,     &d_prefix, &d_bid,    &d_tailq,
             &d_seen,   &d_ctrl,   &d_match,   &d_husband,  &d_prank,  &d_qcnt,   &d_qlist,
             &gen_keys_a, &gen_keys_b, &gen_seg, &gen_temp, &gen_aux, &d_swap_pos, &d_swap_full, &d_swap_over,
-            &d_swap_rows, &d_order, &d_score, &d_round};
+            &d_swap_rows, &d_order, &d_score, &d_round, &d_bits};
   }
   int launches = 0;  // kernels launched since the last stage / call
   smp_stats stats = {};

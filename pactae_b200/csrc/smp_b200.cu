@@ -9,6 +9,7 @@
 #include <thread>
 #include <type_traits>
 
+#include "check_kernels.cuh"
 #include "common.cuh"
 #include "internal.h"
 #include "round_kernels.cuh"
@@ -612,28 +613,54 @@ int control_status(Ctx &c) {
   return s;
 }
 
-// Checker body: needs c.pref_m, c.d_rank valid for c.n.
-template <typename RankT>
-int enqueue_check_t(Ctx &c, const int32_t *match) {
-  const int n = c.n;
-  int rc = c.d_husband.ensure(sizeof(int32_t) * static_cast<size_t>(n));
-  if (!rc) rc = c.d_prank.ensure(sizeof(int32_t) * static_cast<size_t>(n));
-  if (rc) return rc;
-  if (cudaMemsetAsync(c.d_husband.ptr, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess)
-    return c.fail_cuda("husband reset");
-  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
-  k_check_husband<<<grid, 256, 0, c.stream>>>(match, c.d_husband.as<int32_t>(), n, c.d_ctrl.as<Control>());
-  k_check_prank<RankT><<<grid, 256, 0, c.stream>>>(c.d_husband.as<int32_t>(), reinterpret_cast<const RankT *>(c.d_rank.ptr),
-                                                  rank_ld(c), c.d_prank.as<int32_t>(), n, c.d_ctrl.as<Control>());
-  const int sgrid = std::max(1, std::min(c.sm_count * 8, (n * 32 + 255) / 256));
-  k_check_scan<RankT><<<sgrid, 256, 0, c.stream>>>(c.pref_m, reinterpret_cast<const RankT *>(c.d_rank.ptr), rank_ld(c), match,
-                                                  c.d_prank.as<int32_t>(), n, c.d_ctrl.as<Control>());
-  c.launches += 3;
-  return c.check_launch("k_check");
+// Checker body: reads c.pref_m and c.pref_w; above n = 65535 also c.d_rank.
+int check_buffers(Ctx &c) {
+  const size_t n = static_cast<size_t>(c.n);
+  int rc = c.d_husband.ensure(sizeof(int32_t) * n);
+  if (!rc && c.n > kU16MaxN) rc = c.d_prank.ensure(sizeof(int32_t) * n);
+  if (!rc && c.n <= kU16MaxN) rc = c.d_bits.ensure(2 * n * check_row_bytes(c.n));
+  return rc;
 }
 
 int enqueue_check(Ctx &c, const int32_t *match) {
-  return c.rank_bytes == 2 ? enqueue_check_t<uint16_t>(c, match) : enqueue_check_t<int32_t>(c, match);
+  const int n = c.n;
+  int rc = check_buffers(c);
+  if (rc) return rc;
+  Control *ctrl = c.d_ctrl.as<Control>();
+  int32_t *husband = c.d_husband.as<int32_t>();
+  if (cudaMemsetAsync(c.d_husband.ptr, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess)
+    return c.fail_cuda("husband reset");
+  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
+  k_check_husband<<<grid, 256, 0, c.stream>>>(match, husband, n, ctrl);
+  if (n > kU16MaxN) {
+    k_check_prank<<<grid, 256, 0, c.stream>>>(husband, c.d_rank.as<int32_t>(), c.d_prank.as<int32_t>(), n, ctrl);
+    k_check_scan_rank<<<c.sm_count * 8, 256, 0, c.stream>>>(c.pref_m, c.d_rank.as<int32_t>(), match,
+                                                            c.d_prank.as<int32_t>(), n, ctrl);
+    c.launches += 3;
+    return c.check_launch("k_check");
+  }
+  unsigned char *bits = c.d_bits.as<unsigned char>();
+  unsigned char *bits_t = bits + static_cast<size_t>(n) * check_row_bytes(n);
+  const size_t row_smem = row_smem_bytes<uint16_t>(n);
+  const size_t scan_smem = kCheckWarps * check_row_bytes(n);
+  if (allow_dynamic_smem(c, k_check_bits) != cudaSuccess || allow_dynamic_smem(c, k_check_scan) != cudaSuccess)
+    return c.fail_cuda("k_check smem attribute");
+  const auto per_sm = [&](auto kernel, int block, size_t smem) {
+    int k = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, block, smem) != cudaSuccess) {
+      cudaGetLastError();
+      k = 1;
+    }
+    return c.sm_count * std::max(k, 1);
+  };
+  k_check_bits<<<std::min(n, per_sm(k_check_bits, 512, row_smem)), 512, row_smem, c.stream>>>(c.pref_w, husband, bits,
+                                                                                             n, ctrl);
+  const int tiles = (n + 255) / 256;
+  k_check_transpose<<<dim3(tiles, tiles), 256, 0, c.stream>>>(bits, bits_t, n);
+  k_check_scan<<<std::min((n + kCheckWarps - 1) / kCheckWarps, per_sm(k_check_scan, 32 * kCheckWarps, scan_smem)),
+                 32 * kCheckWarps, scan_smem, c.stream>>>(c.pref_m, bits_t, match, n, ctrl);
+  c.launches += 4;
+  return c.check_launch("k_check");
 }
 
 // Per-solve state reset and plan for size n.
@@ -765,8 +792,7 @@ int reserve_buffers(Ctx &c, int32_t n) {
   if (!rc && c.query_ok)
     rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * query_capacity(n, c.K));
   if (!rc) rc = swap_buffers(c);
-  if (!rc) rc = c.d_husband.ensure(sizeof(int32_t) * static_cast<size_t>(n));
-  if (!rc) rc = c.d_prank.ensure(sizeof(int32_t) * static_cast<size_t>(n));
+  if (!rc) rc = check_buffers(c);
   if (!rc) rc = c.sync("reserve");
   c.n = 0;
   return rc;
@@ -793,9 +819,9 @@ int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t 
   if (!rc && !(flags & SMP_F_DEVICE_PTRS)) rc = copy_match_out(c, match_out, false);
   if (!rc && (flags & SMP_F_CHECK)) {
     if (cudaEventRecord(c.ev[kEvCheckBegin], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-    // The checker reuses the solve's rank matrix; only a solve that built
-    // none (perfect, or query mode) builds it here.
-    if (!rc) rc = enqueue_invert_any(c, kGateNoRank);
+    // Above n = 65535 the checker reuses the solve's rank matrix; only a
+    // solve that built none (perfect) builds it here.
+    if (!rc && n > kU16MaxN) rc = enqueue_invert_any(c, kGateNoRank);
     if (!rc) rc = enqueue_check(c, c.d_match.as<int32_t>());
     if (!rc && cudaEventRecord(c.ev[kEvCheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   }
@@ -1725,13 +1751,13 @@ int smp_b200_check(smp_ctx *ctx, const int32_t *pref_m, const int32_t *pref_w, i
       return c.fail_cuda("match copy");
     dmatch = c.d_match.as<int32_t>();
   }
-  rc = enqueue_precheck(c, false);
-  if (rc) return rc;
-  c.rank_bytes = c.rank_bytes_cfg == 4 ? 4 : rank_bytes_for(n);
-  rc = c.d_rank.ensure(rank_matrix_bytes(c));
-  if (rc) return rc;
+  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, sizeof(Control), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   if (cudaEventRecord(c.ev[kEvCheckBegin], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  rc = enqueue_invert_any(c, kGateAlways);
+  if (n > kU16MaxN) {
+    rc = enqueue_precheck(c, false);  // reports first choices out of range
+    if (!rc) rc = c.d_rank.ensure(rank_matrix_bytes(c));
+    if (!rc) rc = enqueue_invert_any(c, kGateAlways);
+  }
   if (!rc) rc = enqueue_check(c, dmatch);
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvCheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");

@@ -14,7 +14,7 @@
 //                                                          src/smp/smp_engine_bamboo.cu:197-287)
 //   k_match       match[m] = w                           (SmpEngineBamboo::PostProc,
 //                                                          smp_engine_bamboo.cu:289-306)
-//   k_check_*     stability checker (no counterpart in the reference)
+//   k_check_*     stability checker (check_kernels.cuh; no counterpart in the reference)
 //
 // Layouts (row-major, 64-bit offsets):
 //   pref_m, pref_w  int32 [n][n]
@@ -45,14 +45,12 @@ enum Gate : int {
   kGateModeRank = 2,   // round 0 in rank mode
   kGateModeQuery = 3,  // round 0 in query mode
   kGateRetry = 4,      // the rank-mode round after a query-mode abort
-  kGateIfPerfect = 5,  // the checker after a perfect solve (needs its own inversion)
   kGateNoRank = 6,     // the checker after a solve that built no rank matrix
 };
 
 __device__ __forceinline__ bool gate_open(int gate, const Control *c) {
   if (gate == kGateAlways) return true;
   const int perfect = ld_volatile_s32(&c->perfect);
-  if (gate == kGateIfPerfect) return perfect != 0;
   if (gate == kGateNoRank) return perfect != 0 || ld_volatile_s32(&c->mode) == kModeQuery;
   if (perfect || ld_volatile_s32(&c->status)) return false;
   switch (gate) {
@@ -1579,77 +1577,6 @@ __global__ void k_match(const int32_t *__restrict__ pref_m, const unsigned long 
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) props += __shfl_down_sync(kFullMask, props, off);
   if ((threadIdx.x & 31) == 0 && props) atomicAdd(&ctrl->proposals, props);
-}
-
-// ---------------------------------------------------------------------------
-// Stability checker.
-//   k_check_husband: husband[w] = m for match[m] = w (husband pre-filled
-//     with -1); a woman matched twice or an out-of-range wife is reported.
-//   k_check_prank:   prank[w] = rank[w][husband[w]].
-//   k_check_scan:    warp per man; every woman before his wife in his list
-//     is a blocking pair if she ranks him above her husband.  Also sums the
-//     proposal count (position of the wife + 1).
-// ---------------------------------------------------------------------------
-__global__ void k_check_husband(const int32_t *__restrict__ match, int32_t *husband, int n, Control *ctrl) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += stride) {
-    const int w = match[m];
-    if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicExch(husband + w, m) != -1)
-      report(ctrl, kStatusInvalidInput, w);
-  }
-}
-
-template <typename RankT>
-__global__ void k_check_prank(const int32_t *__restrict__ husband, const RankT *__restrict__ rank, size_t ld,
-                              int32_t *__restrict__ prank, int n, Control *ctrl) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += stride) {
-    const int h = husband[w];
-    if (h < 0) {
-      report(ctrl, kStatusInvalidInput, w);
-      prank[w] = -1;
-      continue;
-    }
-    prank[w] = static_cast<int32_t>(rank[static_cast<size_t>(w) * ld + h]);
-  }
-}
-
-template <typename RankT>
-__global__ void k_check_scan(const int32_t *__restrict__ pref_m, const RankT *__restrict__ rank, size_t ld,
-                             const int32_t *__restrict__ match, const int32_t *__restrict__ prank, int n,
-                             Control *ctrl) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  unsigned long long blocking = 0, props = 0;
-  for (int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; m < n; m += warps) {
-    const int wife = match[m];
-    const int32_t *row = pref_m + static_cast<size_t>(m) * n;
-    bool found = false;
-    for (int base = 0; base < n && !found; base += 32) {
-      const int r = base + lane;
-      const int w = r < n ? __ldg(row + r) : -1;
-      const unsigned hit = __ballot_sync(kFullMask, r < n && w == wife);
-      const int limit = hit ? (__ffs(hit) - 1) : 32;  // lanes before the wife
-      if (lane < limit && r < n && static_cast<unsigned>(w) < static_cast<unsigned>(n)) {
-        const int32_t pr = prank[w];
-        if (pr >= 0 && static_cast<int32_t>(rank[static_cast<size_t>(w) * ld + m]) < pr) blocking++;
-      }
-      if (hit) {
-        found = true;
-        if (lane == 0) props += static_cast<unsigned long long>(base + limit + 1);
-      }
-    }
-    if (!found && lane == 0) report(ctrl, kStatusInvalidInput, m);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    blocking += __shfl_down_sync(kFullMask, blocking, off);
-    props += __shfl_down_sync(kFullMask, props, off);
-  }
-  if (lane == 0) {
-    if (blocking) atomicAdd(&ctrl->blocking, blocking);
-    if (props) atomicAdd(&ctrl->check_proposals, props);
-  }
 }
 
 }  // namespace smpb200
