@@ -427,7 +427,7 @@ int smp_b200_batch_create(smp_ctx *ctx, const smp_instance *inst, int32_t count,
     delete b;
     return SMP_ERR_UNSUPPORTED;
   }
-  b->slab_elems = static_cast<size_t>(b->max_n) * b->max_n;
+  b->slab_elems = batch_slab_elems(b->max_n);
   const size_t slab_bytes = b->slab_elems * sizeof(uint16_t);
   const int by_budget = static_cast<int>(std::max<size_t>(1, kSlabBudget / slab_bytes));
   const int max_grid = std::max(1, std::min({c.sm_count * 4, by_budget, count}));  // any tuned shape fits

@@ -343,7 +343,7 @@ int smp_b200_server_create(const smp_server_cfg *cfg, smp_server **out) {
   const int max_wave = s->cfg.max_wave > 0 ? s->cfg.max_wave : 256;
   const int per_sm = s->cfg.ctas_per_sm > 0 ? s->cfg.ctas_per_sm : 2;
   s->grid = std::max(1, std::min(max_wave, c.sm_count * per_sm));
-  s->slab_elems = static_cast<size_t>(s->cfg.route_n) * s->cfg.route_n;
+  s->slab_elems = batch_slab_elems(s->cfg.route_n);
   s->waves.resize(s->cfg.waves);
   for (Wave &w : s->waves) {
     if (cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) != cudaSuccess ||

@@ -39,7 +39,8 @@ __device__ __forceinline__ uint32_t issue_choice(const int32_t *__restrict__ pre
 //              load does not wait for that one;
 //   3          one rank per proposer, rank[m]: every receiver ranks the
 //              proposers the same way (a batch instance solved with the
-//              roles swapped because all men share one list).
+//              roles swapped because all men share one list);
+//   4          woman-major with rows padded to 8 entries (the batch kernel).
 template <bool kLdg = true, int kManMajor = 0, typename RankT>
 __device__ __forceinline__ int finish_choice(uint32_t raw, const RankT *__restrict__ rank, int K, int n, bool query,
                                              int m, int r, int &w, uint32_t &rk) {
@@ -52,7 +53,8 @@ __device__ __forceinline__ int finish_choice(uint32_t raw, const RankT *__restri
   if (query) return 1;
   w = static_cast<int>(raw);
   if (static_cast<unsigned>(w) >= static_cast<unsigned>(n)) return 2;
-  const RankT *p = kManMajor == 3   ? rank + m
+  const RankT *p = kManMajor == 4   ? rank + static_cast<size_t>(w) * ((n + 7) & ~7) + m
+                   : kManMajor == 3 ? rank + m
                    : kManMajor == 2 ? rank + static_cast<size_t>(m) * n + r
                    : kManMajor == 1 ? rank + static_cast<size_t>(m) * n + w
                                     : rank + static_cast<size_t>(w) * n + m;

@@ -232,3 +232,58 @@ def test_autotuned_threshold_is_reported(ctx):
         pm, pw, mt = insts[k]
         want, wst = ctx.solve(pm, pw)
         assert np.array_equal(mt.cpu().numpy(), want.cpu().numpy()) and props[k] == wst["proposals"]
+
+
+@pytest.mark.parametrize("block,region", [(512, 32), (128, 64), (96, 32)])
+def test_batch_hard_instances(ctx, block, region):
+    # Few distinct first choices and too large for the shared rank region:
+    # solved 64 men at a time through candidate lists (batch_hard).  Sizes at
+    # the edges of that, of the 32-women bit words and of the 16-byte rows;
+    # lists alike in every way the generator knows; one order of starting
+    # that is the worst one (every man displaces all before him and uses his
+    # list up).
+    import torch
+
+    insts, wants = [], []
+    cases = [(pb.SMP_GEN_CORRELATED, 500, n) for n in (182, 191, 193, 255, 256, 257, 512, 1001, 2050)]
+    cases += [(pb.SMP_GEN_CORRELATED, 20, 640), (pb.SMP_GEN_GROUPED, 5, 321), (pb.SMP_GEN_GROUPED, 50, 1000)]
+    lists = [oracle.generate(kind, n, 70 + n, 0, param) for kind, param, n in cases]
+    n = 700
+    pm = np.tile(np.arange(n, dtype=np.int32), (n, 1))
+    pm[n // 2, [n - 2, n - 1]] = pm[n // 2, [n - 1, n - 2]]
+    pw = np.tile(np.arange(n, dtype=np.int32)[::-1], (n, 1))
+    pw[[i * n // 32 for i in range(32)]] = np.arange(n, dtype=np.int32)
+    lists.append((pm, pw))
+    for pm, pw in lists:
+        wants.append(oracle.gs_seq(pm, pw))
+        insts.append((torch.from_numpy(pm).cuda(), torch.from_numpy(pw).cuda(),
+                      torch.full((pm.shape[0],), -1, dtype=torch.int32, device="cuda")))
+    with pb.Batch(ctx, insts, tune=False, block_threads=block, rank_smem_kb=region) as batch:
+        for _ in range(2):
+            status, props, st = batch.run()
+            assert all(s == 0 for s in status)
+            for (_, _, mt), (want, wp), p in zip(insts, wants, props):
+                assert np.array_equal(mt.cpu().numpy(), want) and p == wp
+
+
+def test_batch_hard_instance_bad_entries(ctx):
+    # An entry out of range counts only if a man's proposals reach it.
+    import torch
+
+    n = 400
+    pm, pw = oracle.generate(pb.SMP_GEN_CORRELATED, n, 3, 0, 500)
+    want, wp = oracle.gs_seq(pm, pw)
+    pos = np.argmax(pm == want[:, None], axis=1)
+    m = int(np.argmax(pos < n - 2))
+    reached, not_reached, bad_w = pm.copy(), pm.copy(), pw.copy()
+    reached[m, 0] = n
+    not_reached[m, n - 1] = -5
+    bad_w[n - 1, 0] = bad_w[n - 1, 1]
+    insts = [(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(),
+              torch.full((n,), -1, dtype=torch.int32, device="cuda"))
+             for a, b in ((reached, pw), (not_reached, pw), (pm, bad_w), (pm, pw))]
+    with pb.Batch(ctx, insts, tune=False) as batch:
+        status, props, _ = batch.run()
+    assert status == [pb.SMP_ERR_INVALID_INPUT, 0, pb.SMP_ERR_INVALID_INPUT, 0]
+    for i in (1, 3):
+        assert np.array_equal(insts[i][2].cpu().numpy(), want) and props[i] == wp
