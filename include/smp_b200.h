@@ -202,7 +202,8 @@ typedef struct smp_instance {
 #define SMP_B200_BATCH_MAX_N 16384
 
 typedef struct smp_batch_cfg {
-  int32_t block_threads;   /* threads per CTA (64..512); 0 = auto            */
+  int32_t block_threads;   /* threads per CTA (64..512); 0 = auto (which may */
+                           /* choose 1024)                                   */
   int32_t ctas_per_sm;     /* resident CTAs per SM (1..4); 0 = auto          */
   int32_t window;          /* look-ahead choices per warp step; 0 = auto     */
   int32_t use_graph;       /* 1 (default, also 0 here) = replay a captured   */

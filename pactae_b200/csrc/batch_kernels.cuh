@@ -429,7 +429,7 @@ __device__ __forceinline__ void batch_hard(const int32_t *__restrict__ pref_m, c
 // whose n*n rank matrix fits there keeps it on chip (small instances), the
 // others use the CTA's slab in global memory.
 template <int kMaxSub>
-__global__ void __launch_bounds__(512, 2) k_batch(BatchInstance *__restrict__ table, const int32_t *__restrict__ order,
+__global__ void __launch_bounds__(1024, 1) k_batch(BatchInstance *__restrict__ table, const int32_t *__restrict__ order,
                                                int count, int *queue, uint16_t *__restrict__ slabs,
                                                size_t slab_elems, int max_n, int dynamic, int rank_smem_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
