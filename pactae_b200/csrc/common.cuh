@@ -52,7 +52,14 @@ struct Control {
   int32_t w_differ;       // k_swap_screen: a pref_w row differs from row 0
   int32_t swap_over;      // k_swap_gs: women stopped at the end of what the device holds of their rows
   int32_t round_done;     // k_round: the matching is complete and written
-  int32_t round_pad;
+  // the women-proposing screen with the proposals beside it (swap_kernels.cuh)
+  int32_t w_first;        // the women's first choices differ
+  int32_t screen_next;    // rows its CTAs have taken beyond their first
+  int32_t screen_ctas;    // CTAs of it that have finished
+  int32_t screen_done;    // all have
+  int32_t swap_out;       // match[] is written
+  int32_t swap_quit;      // a warp of the proposals beside it gave up
+  int32_t swap_pad;
   int2 coop_chain[32];
 };
 

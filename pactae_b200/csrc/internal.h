@@ -273,6 +273,7 @@ struct Ctx {
 
   DeviceBuf d_pref_m, d_pref_w, d_rank, d_rankT, d_pr, d_prefix, d_bid, d_tailq, d_seen, d_ctrl, d_match;
   DeviceBuf d_pw16, d_pm16;  // pref_w and pref_m packed to uint16 (host-input solves)
+  DeviceBuf d_swap_near;  // women-proposing solves: each woman's first choices in 16 bits
   DeviceBuf d_swap_pos;  // women-proposing solves: position of each woman in the men's shared list
   // host-input women-proposing solves: which women's rows are whole on the
   // device, the women stopped at the end of theirs (two lists), row ids
@@ -293,11 +294,13 @@ struct Ctx {
   static constexpr int kCopyChunks = 16;
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t ev_chunk[kCopyChunks] = {};
-  std::array<DeviceBuf *, 30> buffers() {
+  cudaStream_t side_stream = nullptr;  // the women's proposals beside their screen
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  std::array<DeviceBuf *, 31> buffers() {
     return {&d_pref_m, &d_pref_w, &d_pw16, &d_pm16, &d_rank,    &d_rankT,    &d_pr,     &d_prefix, &d_bid,    &d_tailq,
             &d_seen,   &d_ctrl,   &d_match,   &d_husband,  &d_prank,  &d_qcnt,   &d_qlist,
             &gen_keys_a, &gen_keys_b, &gen_seg, &gen_temp, &gen_aux, &d_swap_pos, &d_swap_full, &d_swap_over,
-            &d_swap_rows, &d_order, &d_score, &d_round, &d_bits};
+            &d_swap_rows, &d_order, &d_score, &d_round, &d_bits, &d_swap_near};
   }
   int launches = 0;  // kernels launched since the last stage / call
   smp_stats stats = {};

@@ -406,10 +406,24 @@ int init_buffers(Ctx &c) {
   return SMP_OK;
 }
 
+// The stream that runs beside the context's, with its fork and join events
+// (created on first use).
+int side_stream(Ctx &c) {
+  if (c.side_stream) return SMP_OK;
+  if (!c.ev_fork && cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming) != cudaSuccess)
+    return c.fail_cuda("fork event");
+  if (!c.ev_join && cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming) != cudaSuccess)
+    return c.fail_cuda("join event");
+  if (cudaStreamCreateWithFlags(&c.side_stream, cudaStreamNonBlocking) != cudaSuccess)
+    return c.fail_cuda("side stream");
+  return SMP_OK;
+}
+
 // Buffers of the women-proposing solve.
 int swap_buffers(Ctx &c) {
   int rc = c.d_swap_pos.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
   if (!rc) rc = c.d_bid.ensure(sizeof(unsigned long long) * static_cast<size_t>(c.n));
+  if (!rc && c.n <= kU16MaxN) rc = c.d_swap_near.ensure(sizeof(uint16_t) * kSwapNear * static_cast<size_t>(c.n));
   return rc ? rc : c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
 }
 
@@ -870,65 +884,85 @@ int enqueue_pass_mode(Ctx &c, int mode) {
 
 // Rank-mode men who all make the same first choice may share one list.  The
 // screen checks that on all SMs (and that pref_w's rows are permutations).
+constexpr int kSwapBeside = 1;  // CTAs per SM of the proposals
 bool swap_screen_fits(const Ctx &c) { return swap_screen_smem(c.n) <= c.smem_optin; }
 
 int enqueue_swap_screen(Ctx &c, bool men_screened) {
   const int n = c.n;
   int rc = swap_buffers(c);
+  if (!rc) rc = side_stream(c);
   if (rc) return rc;
   Control *ctrl = c.d_ctrl.as<Control>();
   int32_t *pos = c.d_swap_pos.as<int32_t>();
-  if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess)
+  unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
+  if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
+      cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("swap reset");
-  k_swap_pos<<<std::max(1, std::min(c.sm_count * 4, (n + 255) / 256)), 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl);
-  if (allow_dynamic_smem(c, k_swap_screen) != cudaSuccess) return c.fail_cuda("k_swap_screen smem attribute");
+  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl, c.pref_w);
+  uint16_t *near = n <= kU16MaxN ? c.d_swap_near.as<uint16_t>() : nullptr;
+  if (near) k_swap_near<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_w, near, n);
+  // the women's proposals beside the screen, which leaves a CTA's place on
+  // each SM: where it fills them, the proposals may not start before it ends
+  if (cudaEventRecord(c.ev_fork, c.stream) != cudaSuccess ||
+      cudaStreamWaitEvent(c.side_stream, c.ev_fork, 0) != cudaSuccess)
+    return c.fail_cuda("swap fork");
+  k_swap_gs<<<c.sm_count * kSwapBeside, 256, 0, c.side_stream>>>(c.pref_m, c.pref_w, pos, bid, n, ctrl, nullptr, n, nullptr,
+                                                       nullptr, 0, 1, near);
+  rc = c.check_launch("k_swap_gs");
+  if (!rc && allow_dynamic_smem(c, k_swap_screen) != cudaSuccess) rc = c.fail_cuda("k_swap_screen smem attribute");
   const size_t screen_smem = swap_screen_smem(n);
-  int per_sm = 0;  // one wave: every CTA resident
+  int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_swap_screen, 256, screen_smem) != cudaSuccess) {
     cudaGetLastError();
     per_sm = 1;
   }
   const int t0 = men_screened ? n : 1;  // the host compared the men's rows already
-  k_swap_screen<<<std::max(1, std::min(2 * n - t0, c.sm_count * std::max(per_sm, 1))), 256, screen_smem, c.stream>>>(
-      c.pref_m, c.pref_w, n, ctrl, t0);
-  c.launches += 2;
-  rc = c.check_launch("k_swap_screen");
-  if (!rc && cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (!rc) {
+    k_swap_screen<<<std::max(1, std::min(2 * n - t0, c.sm_count * std::max(per_sm - kSwapBeside, 1))), 256, screen_smem,
+                    c.stream>>>(c.pref_m, c.pref_w, n, ctrl, t0);
+    rc = c.check_launch("k_swap_screen");
+  }
+  c.launches += near ? 5 : 4;
+  if (!rc && (cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess ||
+              cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess))
+    rc = c.fail_cuda("event");
+  // join the side stream, even after an error: its kernel uses the buffers
+  if (cudaEventRecord(c.ev_join, c.side_stream) != cudaSuccess ||
+      cudaStreamWaitEvent(c.stream, c.ev_join, 0) != cudaSuccess)
+    return c.fail_cuda("swap join");
+  if (!rc && (cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess ||
+              cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess))
+    rc = c.fail_cuda("event");
+  if (rc) return rc;
+  k_swap_outcome<<<grid, 256, 0, c.stream>>>(c.pref_m, c.pref_w, bid, c.d_match.as<int32_t>(), n, ctrl);
+  rc = c.check_launch("k_swap_outcome");
+  if (!rc) rc = copy_match_out(c, c.pass_match, (c.pass_flags & SMP_F_DEVICE_PTRS) != 0);
+  if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   return rc ? rc : read_control(c);
 }
 
-// The screen found one shared list: the women propose, or, when they share
-// one list too, the sides pair rank for rank.
+// The screen found one shared list, and proposals still to be made: the women
+// differ, but not in their first choices, so those beside the screen gave up.
 int enqueue_swap_solve(Ctx &c) {
   const int n = c.n;
-  c.swapped = true;
   Control *ctrl = c.d_ctrl.as<Control>();
-  int32_t *pos = c.d_swap_pos.as<int32_t>();
   unsigned long long *bid = c.d_bid.as<unsigned long long>();
-  const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
-  int rc;
-  if (!c.h_ctrl->w_differ) {  // the women share one list too: pair rank for rank
-    if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-    if (cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-    if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-    k_swap_direct<<<grid, 256, 0, c.stream>>>(c.pref_m, c.pref_w, c.d_match.as<int32_t>(), n, ctrl);
-    c.launches++;
-    rc = c.check_launch("k_swap_direct");
-  } else {
-    if (cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
-      return c.fail_cuda("swap bid reset");
-    if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-    k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_m, c.pref_w, pos, bid, n, ctrl, nullptr, n, nullptr,
-                                                    nullptr, 0);
-    c.launches++;
-    rc = c.check_launch("k_swap_gs");
-    if (!rc && cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-    if (!rc && cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-    if (rc) return rc;
-    k_swap_match<<<grid, 256, 0, c.stream>>>(c.pref_m, bid, c.d_match.as<int32_t>(), n, ctrl);
-    c.launches++;
-    rc = c.check_launch("k_swap_match");
-  }
+  if (cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
+      cudaMemsetAsync(&ctrl->swap_next, 0, sizeof(int32_t), c.stream) != cudaSuccess)
+    return c.fail_cuda("swap bid reset");
+  if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
+  k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_m, c.pref_w, c.d_swap_pos.as<int32_t>(), bid, n, ctrl, nullptr,
+                                                  n, nullptr, nullptr, 0, 0, nullptr);
+  c.launches++;
+  int rc = c.check_launch("k_swap_gs");
+  if (!rc && cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (!rc && cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (rc) return rc;
+  k_swap_match<<<std::max(1, std::min(c.sm_count * 4, (n + 255) / 256)), 256, 0, c.stream>>>(
+      c.pref_m, bid, c.d_match.as<int32_t>(), n, ctrl);
+  c.launches++;
+  rc = c.check_launch("k_swap_match");
   if (!rc) rc = copy_match_out(c, c.pass_match, (c.pass_flags & SMP_F_DEVICE_PTRS) != 0);
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   return rc ? rc : read_control(c);
@@ -971,12 +1005,14 @@ int solve_advance(Ctx &c, bool &more) {
   }
   const bool queried = c.pass == kPassQuery;
   if (queried && (h.perfect || (h.mode == kModeQuery && !h.retry))) return SMP_OK;
-  more = true;
-  c.poll_rounds = in_rounds(c);
   if (c.pass == kPassScreen && !h.swap_fail) {
     c.pass = kPassLast;
-    return enqueue_swap_solve(c);
+    c.swapped = true;
+    more = !h.swap_out;
+    return more ? enqueue_swap_solve(c) : SMP_OK;
   }
+  more = true;
+  c.poll_rounds = in_rounds(c);
   if (queried && h.mode == kModeQuery) {  // the rank-mode retry of a query-mode round 0
     c.pass = kPassLast;
     c.known_mode = -1;
@@ -1017,6 +1053,8 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
   if (rc) return rc;
   swapped = c.h_ctrl->status || !c.h_ctrl->swap_fail;
   if (!swapped || c.h_ctrl->status) return SMP_OK;
+  c.swapped = true;
+  if (c.h_ctrl->swap_out) return SMP_OK;
   rc = enqueue_swap_solve(c);
   if (!rc) rc = c.sync("solve");
   return rc;
@@ -1288,7 +1326,7 @@ int solve_shared_host(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, uint
   if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   if (!rc) rc = reset_queue();
   if (rc) return rc;
-  k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(dm, dw, pos, bid, n, ctrl, full, kw, over[0], nullptr, 0);
+  k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(dm, dw, pos, bid, n, ctrl, full, kw, over[0], nullptr, 0, 0, nullptr);
   c.launches++;
   rc = c.check_launch("k_swap_gs");
   for (int round = 0; !rc; ++round) {
@@ -1309,7 +1347,7 @@ int solve_shared_host(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, uint
     if (!rc) rc = reset_queue();
     if (rc) break;
     k_swap_gs<<<std::max(1, std::min(c.sm_count * 4, (stopped + 7) / 8)), 256, 0, c.stream>>>(
-        dm, dw, pos, bid, n, ctrl, full, kw, over[(round + 1) & 1], over[round & 1], stopped);
+        dm, dw, pos, bid, n, ctrl, full, kw, over[(round + 1) & 1], over[round & 1], stopped, 0, nullptr);
     c.launches++;
     rc = c.check_launch("k_swap_gs");
   }
@@ -1564,6 +1602,7 @@ void smp_b200_destroy(smp_ctx *ctx) {
   {
     DeviceGuard g(c.device);
     if (c.copy_stream) cudaStreamSynchronize(c.copy_stream);
+    if (c.side_stream) cudaStreamSynchronize(c.side_stream);
     if (c.stream) cudaStreamSynchronize(c.stream);
     for (DeviceBuf *b : c.buffers()) b->release();
     if (c.stream) cudaStreamSynchronize(c.stream);
@@ -1573,6 +1612,9 @@ void smp_b200_destroy(smp_ctx *ctx) {
     for (auto &e : c.ev_chunk)
       if (e) cudaEventDestroy(e);
     if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
+    if (c.side_stream) cudaStreamDestroy(c.side_stream);
+    if (c.ev_fork) cudaEventDestroy(c.ev_fork);
+    if (c.ev_join) cudaEventDestroy(c.ev_join);
     if (c.h_ctrl) cudaFreeHost(c.h_ctrl);
     c.link.reset();
     c.pack_pool.reset();

@@ -28,12 +28,16 @@
 namespace smpb200 {
 
 // pos[L[r]] = r, with pos preset to -1; an entry out of range or seen twice
-// makes row 0 no permutation.
-__global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl) {
+// makes row 0 no permutation.  With pref_w given, w_first says whether the
+// women's first choices differ.
+__global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl,
+                           const int32_t *__restrict__ pref_w = nullptr) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const int w = __ldg(pref_m + r);
     if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1)
       report(ctrl, kStatusInvalidInput, w);
+    if (pref_w && __ldg(pref_w + static_cast<size_t>(r) * n) != __ldg(pref_w) && !ld_volatile_s32(&ctrl->w_first))
+      ctrl->w_first = 1;
   }
 }
 
@@ -45,8 +49,40 @@ __global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restri
 // when n is not a multiple of 4).  Once a pref_m row differs, the solve
 // takes the men's rank-mode pass, which checks pref_w itself: the CTAs stop.
 // (One colour byte per man with plain stores and a check pass, instead of the
-// bitmap's shared atomics, took 1.85 ms against 1.47 ms at n = 30000.)
+// bitmap's shared atomics, took 1.85 ms against 1.47 ms at n = 30000.  Where the
+// women share one list too, comparing with row 0 instead of marking: 1.96 -> 1.30.)
 __host__ __device__ constexpr size_t swap_screen_smem(int n) { return ((static_cast<size_t>(n) + 31) / 32) * 4; }
+
+// Does this thread's share of row t differ from row 0?  Chunk by chunk where
+// both rows start at the same 16-byte offset (all rows when n is a multiple of
+// 4), else each chunk against four entries of row 0.
+__device__ __forceinline__ bool row_differs(const int32_t *__restrict__ pref, int t, int n) {
+  const int tid = threadIdx.x;
+  const int nthr = blockDim.x;
+  const RowSpan s = row_span(pref, t, n);
+  bool differs = false;
+  const auto other = [](int4 v, int4 u) { return v.x != u.x || v.y != u.y || v.z != u.z || v.w != u.w; };
+  int i = tid;
+  if (s.head == row_span(pref, 0, n).head) {
+    const int4 *q0 = reinterpret_cast<const int4 *>(pref + s.head);
+    for (; i + nthr < s.nq; i += 2 * nthr) {
+      const int4 v = __ldcs(s.rq + i);
+      const int4 v2 = __ldcs(s.rq + i + nthr);
+      differs |= other(v, __ldg(q0 + i)) || other(v2, __ldg(q0 + i + nthr));
+    }
+    if (i < s.nq) differs |= other(__ldcs(s.rq + i), __ldg(q0 + i));
+  } else {
+    for (; i < s.nq; i += nthr) {
+      const int c = s.head + 4 * i;
+      differs |= other(__ldcs(s.rq + i),
+                       make_int4(__ldg(pref + c), __ldg(pref + c + 1), __ldg(pref + c + 2), __ldg(pref + c + 3)));
+    }
+  }
+  if (tid < s.head) differs |= __ldcs(s.row + tid) != __ldg(pref + tid);
+  const int c0 = s.head + 4 * s.nq;
+  if (tid < s.tail) differs |= __ldcs(s.row + c0 + tid) != __ldg(pref + c0 + tid);
+  return differs;
+}
 
 __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__ pref_m,
                                                      const int32_t *__restrict__ pref_w, int n, Control *ctrl,
@@ -54,89 +90,99 @@ __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *seen = reinterpret_cast<uint32_t *>(smem_raw);
   __shared__ int s_stop;
+  __shared__ int s_row;
   __shared__ int s_wsame;  // no pref_w row has differed from row 0 yet
   const int tid = threadIdx.x;
   const int nthr = blockDim.x;
   const int words = (n + 31) >> 5;
   bool bad = false;
   int bad_value = 0;
-  for (int t = t0 + static_cast<int>(blockIdx.x); t < 2 * n; t += gridDim.x) {
+  // Rows are taken in turn, each CTA's next one while it works on the last: a
+  // CTA that waits for the proposals' CTA to leave its SM then takes fewer.
+  int next = t0 + static_cast<int>(blockIdx.x);
+  for (;;) {
     if (tid == 0) {
-      s_stop = ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status);
+      s_row = next;
+      s_stop = next >= 2 * n || ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status);
       s_wsame = !ld_volatile_s32(&ctrl->w_differ);
+      next = t0 + static_cast<int>(gridDim.x) + atomicAdd(&ctrl->screen_next, 1);
     }
     __syncthreads();
     if (s_stop) break;
+    const int t = s_row;
     if (t < n) {
-      // pref_m row t against row 0: chunk by chunk where both rows start at
-      // the same 16-byte offset (all rows when n is a multiple of 4), else
-      // each chunk against four entries of row 0
-      const RowSpan s = row_span(pref_m, t, n);
-      bool differs = false;
-      if (s.head == row_span(pref_m, 0, n).head) {
-        const int4 *q0 = reinterpret_cast<const int4 *>(pref_m + s.head);
-        for (int i = tid; i < s.nq; i += nthr) {
-          const int4 v = __ldcs(s.rq + i);
-          const int4 u = __ldg(q0 + i);
-          differs |= v.x != u.x || v.y != u.y || v.z != u.z || v.w != u.w;
-        }
-      } else {
-        for (int i = tid; i < s.nq; i += nthr) {
-          const int4 v = __ldcs(s.rq + i);
-          const int c = s.head + 4 * i;
-          differs |= v.x != __ldg(pref_m + c) || v.y != __ldg(pref_m + c + 1) || v.z != __ldg(pref_m + c + 2) ||
-                     v.w != __ldg(pref_m + c + 3);
-        }
-      }
-      if (tid < s.head) differs |= __ldcs(s.row + tid) != __ldg(pref_m + tid);
-      const int c0 = s.head + 4 * s.nq;
-      if (tid < s.tail) differs |= __ldcs(s.row + c0 + tid) != __ldg(pref_m + c0 + tid);
-      if (__syncthreads_or(differs) && tid == 0) atomicExch(&ctrl->swap_fail, 1);
+      // pref_m row t against row 0
+      if (__syncthreads_or(row_differs(pref_m, t, n)) && tid == 0) atomicExch(&ctrl->swap_fail, 1);
     } else {
-      // pref_w row t - n: every value in range and seen once; while no
-      // row has differed, also compared with row 0 (the women may share one
-      // list as well)
+      // pref_w row t - n: every value in range and seen once.  While no row
+      // has differed it is compared with row 0 first (the women may share one
+      // list as well): a row equal to row 0 needs no check of its own.
+      if (s_wsame && t > n) {
+        if (!__syncthreads_or(row_differs(pref_w, t - n, n))) continue;
+        if (tid == 0) atomicExch(&ctrl->w_differ, 1);  // one flag per CTA and row
+      }
       for (int i = tid; i < words; i += nthr) seen[i] = 0u;
       __syncthreads();
       const RowSpan s = row_span(pref_w, t - n, n);
-      if (s_wsame && t > n) {
-        bool differs = false;
-        for (int i = tid; i < s.nq; i += nthr) {
-          const int4 v = __ldcs(s.rq + i);
-          const int c = s.head + 4 * i;
-          differs |= v.x != __ldg(pref_w + c) || v.y != __ldg(pref_w + c + 1) || v.z != __ldg(pref_w + c + 2) ||
-                     v.w != __ldg(pref_w + c + 3);
-        }
-        if (tid < s.head) differs |= __ldcs(s.row + tid) != __ldg(pref_w + tid);
-        const int c0 = s.head + 4 * s.nq;
-        if (tid < s.tail) differs |= __ldcs(s.row + c0 + tid) != __ldg(pref_w + c0 + tid);
-        if (__syncthreads_or(differs) && tid == 0) atomicExch(&ctrl->w_differ, 1);  // one flag per CTA and row
-      }
+      // n entries in range that set n bits are a permutation: no atomic's
+      // result is waited for, the bits are counted at the end
       const auto mark = [&](int v) {
-        if (static_cast<unsigned>(v) >= static_cast<unsigned>(n)) {
-          bad = true;
-          bad_value = v;
-          return;
-        }
-        const uint32_t bit = 1u << (v & 31);
-        if (atomicOr(seen + (v >> 5), bit) & bit) {
+        if (static_cast<unsigned>(v) < static_cast<unsigned>(n)) {
+          atomicOr(seen + (v >> 5), 1u << (v & 31));
+        } else {
           bad = true;
           bad_value = v;
         }
       };
-      for (int i = tid; i < s.nq; i += nthr) {
-        const int4 v = __ldcs(s.rq + i);
+      const auto mark4 = [&](int4 v) {
         mark(v.x);
         mark(v.y);
         mark(v.z);
         mark(v.w);
+      };
+      int i = tid;
+      for (; i + nthr < s.nq; i += 2 * nthr) {
+        const int4 v = __ldcs(s.rq + i);
+        const int4 u = __ldcs(s.rq + i + nthr);
+        mark4(v);
+        mark4(u);
       }
+      if (i < s.nq) mark4(__ldcs(s.rq + i));
       if (tid < s.head) mark(__ldcs(s.row + tid));
       if (tid < s.tail) mark(__ldcs(s.row + s.head + 4 * s.nq + tid));
+      __syncthreads();
+      for (int k = tid; k < words; k += nthr) {
+        const uint32_t full = k < n / 32 ? 0xFFFFFFFFu : (1u << (n & 31)) - 1u;
+        if (seen[k] != full) {  // someone is named twice, and this man not at all
+          bad = true;
+          bad_value = 32 * k + __ffs(~seen[k]) - 1;
+        }
+      }
       __syncthreads();  // the bitmap is cleared for the next row only after this one
     }
   }
   if (bad) report(ctrl, kStatusInvalidInput, bad_value);
+  // the last CTA tells the proposals running beside the screen that it is over
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(&ctrl->screen_ctas, 1) == static_cast<int>(gridDim.x) - 1) atomicExch(&ctrl->screen_done, 1);
+  }
+}
+
+// near[w][r] = woman w's r-th choice for r < kSwapNear, in 16 bits (0xFFFF where
+// it is out of range).  A displaced woman's next choices are then in a table of
+// 128 bytes per woman that stays in L2; her row is a DRAM access, which takes
+// several microseconds while the screen streams both lists.
+constexpr int kSwapNear = 64;
+__global__ void __launch_bounds__(256) k_swap_near(const int32_t *__restrict__ pref_w, uint16_t *__restrict__ near, int n) {
+  const size_t total = static_cast<size_t>(n) * kSwapNear;
+  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+  for (size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const int w = static_cast<int>(t / kSwapNear);
+    const int r = static_cast<int>(t % kSwapNear);
+    if (r < n) near[t] = static_cast<uint16_t>(min(static_cast<uint32_t>(__ldg(pref_w + static_cast<size_t>(w) * n + r)), 0xFFFFu));
+  }
 }
 
 // The women's proposals.  A man's bid word is pos[w] << 32 | r for the woman
@@ -155,18 +201,39 @@ __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__
 // position 0).  Gale-Shapley's result does not depend on that order.  An
 // entry out of range is reported; a woman who runs out of her whole row
 // (input that is not a permutation) too.
+//   beside: the screen runs at the same time.  The proposals are a chain of L2
+// round trips that leaves the memory idle, the screen a stream that leaves
+// the SMs idle: n = 30000 congested took 1.31 ms and then 0.82 ms.  An entry
+// that is not a permutation's is the screen's to report here; the proposals
+// give up when it has found that the men's lists differ, that the input is
+// invalid, or that the women share one list too (they would make n (n + 1) / 2
+// contended proposals) -- at once if even their first choices are all alike.
 __global__ void __launch_bounds__(256) k_swap_gs(const int32_t *__restrict__ pref_m,
                                                  const int32_t *__restrict__ pref_w,
                                                  const int32_t *__restrict__ pos,
                                                  unsigned long long *__restrict__ bid, int n, Control *ctrl,
                                                  const uint8_t *__restrict__ full, int depth,
                                                  int2 *__restrict__ over, const int2 *__restrict__ start,
-                                                 int start_count) {
+                                                 int start_count, int beside, const uint16_t *__restrict__ near) {
   const int lane = threadIdx.x & 31;
   const int total = start ? start_count : n;
   int w = -1, r0 = 0;
   uint32_t key = 0;
+  unsigned steps = 0;
+  if (beside && !ld_volatile_s32(&ctrl->w_first)) return;
   for (;;) {
+    // Now and then only: thousands of warps reading these flags at every step
+    // would queue at one L2 slice.
+    if (beside && (++steps & 31) == 0) {
+      int stop = 0;
+      if (lane == 0)
+        stop = ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status) ||
+               (ld_volatile_s32(&ctrl->screen_done) && !ld_volatile_s32(&ctrl->w_differ));
+      if (__shfl_sync(kFullMask, stop, 0)) {
+        if (lane == 0) atomicExch(&ctrl->swap_quit, 1);
+        return;
+      }
+    }
     if (w < 0) {
       int i = 0;
       if (lane == 0) i = atomicAdd(&ctrl->swap_next, 1);
@@ -202,7 +269,9 @@ __global__ void __launch_bounds__(256) k_swap_gs(const int32_t *__restrict__ pre
     }
     const int r = r0 + lane;
     const bool in_row = r < lim;
-    const int m = in_row ? __ldg(pref_w + static_cast<size_t>(w) * n + r) : 0;
+    const int m = !in_row                ? 0
+                  : near && r < kSwapNear ? static_cast<int>(__ldg(near + w * kSwapNear + r))
+                                          : __ldg(pref_w + static_cast<size_t>(w) * n + r);
     const bool valid = static_cast<unsigned>(m) < static_cast<unsigned>(n);
     const bool open = in_row && valid && static_cast<uint32_t>(ld_relaxed_u64(bid + m) >> 32) > key;
     const unsigned hit = __ballot_sync(kFullMask, open);
@@ -280,6 +349,34 @@ __global__ void k_swap_mark_full(uint8_t *__restrict__ full, const int32_t *__re
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     const int w = __ldg(rows + i);
     if (static_cast<unsigned>(w) < static_cast<unsigned>(n)) full[w] = 1;
+  }
+}
+
+// The outcome of the screen and the proposals beside it: nothing where the
+// men's lists differ or the input is invalid; the pairing rank for rank where
+// the women share one list too; else match[m] = the woman m holds.  swap_out
+// says that match[] is complete (the host runs the proposals alone if they
+// gave up without cause: women who differ, but not in their first choice).
+__global__ void k_swap_outcome(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
+                               const unsigned long long *__restrict__ bid, int32_t *__restrict__ match, int n,
+                               Control *ctrl) {
+  if (ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status)) return;
+  const bool alike = !ld_volatile_s32(&ctrl->w_differ);
+  if (!alike && (!ld_volatile_s32(&ctrl->w_first) || ld_volatile_s32(&ctrl->swap_quit))) return;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    if (alike) {
+      match[__ldg(pref_w + k)] = __ldg(pref_m + k);
+    } else {
+      const unsigned long long b = bid[k];
+      // (a man left without a woman: reported by the proposals)
+      match[k] = b == ~0ull ? -1 : __ldg(pref_m + static_cast<uint32_t>(b >> 32));
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctrl->swap_out = 1;
+    ctrl->proposals = static_cast<unsigned long long>(n) * (static_cast<unsigned long long>(n) + 1) / 2;
+    ctrl->bulk_proposals = ctrl->proposals;
+    ctrl->tail_proposals = 0;
   }
 }
 
