@@ -202,8 +202,7 @@ typedef struct smp_instance {
 #define SMP_B200_BATCH_MAX_N 16384
 
 typedef struct smp_batch_cfg {
-  int32_t block_threads;   /* threads per CTA (64..512); 0 = auto (which may */
-                           /* choose 1024)                                   */
+  int32_t block_threads;   /* threads per CTA (64..512); 0 = auto            */
   int32_t ctas_per_sm;     /* resident CTAs per SM (1..4); 0 = auto          */
   int32_t window;          /* look-ahead choices per warp step; 0 = auto     */
   int32_t use_graph;       /* 1 (default, also 0 here) = replay a captured   */
@@ -219,7 +218,9 @@ typedef struct smp_batch_cfg {
                            /* beside the persistent kernel; 0 = auto (the    */
                            /* autotuner times none and the largest 8, 32 and */
                            /* 128; with tune = -1: none), -1 = none          */
-  int32_t reserved;
+  int32_t cta_width;       /* out of smp_b200_batch_config: 2 where the      */
+                           /* autotuner runs CTAs of twice block_threads     */
+                           /* (one per SM), else 1; ignored on input         */
 } smp_batch_cfg;
 
 typedef struct smp_batch_stats {

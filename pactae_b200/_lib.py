@@ -138,11 +138,11 @@ class smp_batch_cfg(ctypes.Structure):
         ("rank_smem_kb", ctypes.c_int32),
         ("tune", ctypes.c_int32),
         ("threshold_n", ctypes.c_int32),
-        ("reserved", ctypes.c_int32),
+        ("cta_width", ctypes.c_int32),
     ]
 
     def as_dict(self) -> dict:
-        return {name: getattr(self, name) for name, _ in self._fields_ if name != "reserved"}
+        return {name: getattr(self, name) for name, _ in self._fields_ if name != "cta_width"}
 
 
 class smp_batch_stats(ctypes.Structure):

@@ -23,7 +23,8 @@ struct smp_batch {
   smp_ctx *ctx = nullptr;
   int count = 0;
   int max_n = 0;
-  int block = 512;
+  int block = 512;         // threads of a CTA
+  int width = 1;           // of which block / width are the shape's
   int grid = 0;
   int subs = 8;
   int per_sm = 2;
@@ -105,13 +106,14 @@ int launch_batch(smp_batch &b, cudaStream_t s, int grid, const int32_t *order, i
 // Shapes and the autotuner.  A shape is the CTA size, CTAs per SM, the
 // look-ahead window and the shared rank region (the size threshold below
 // which an instance's rank matrix stays on chip: n*n*2 bytes must fit).  The
-// kernel is compiled for at most 64 registers, so block * ctas_per_sm <= 1024:
-// two 512-thread CTAs per SM suit batches with many more instances than CTAs
+// kernel is compiled for at most 64 registers, so block * width * ctas_per_sm
+// <= 1024: two 512-thread CTAs per SM suit batches with many more instances than CTAs
 // (6000 instances of the mix), one of 1024 threads those whose largest
-// instances set the time (1024 instances: 9.1 -> 6.8 ms).
+// instances set the time (width 2; 1024 instances: 9.1 -> 6.8 ms).
 // ---------------------------------------------------------------------------
 struct Shape {
   int block, per_sm, subs, rank_kb;
+  int width = 1;  // 2: CTAs of twice `block` threads
 };
 
 size_t shape_smem(int max_n, int rank_kb) {
@@ -123,12 +125,13 @@ bool shape_fits(const Ctx &c, int max_n, const Shape &sh) {
   int per_sm_bytes = 0;
   cudaDeviceGetAttribute(&per_sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c.device);
   return smem <= c.smem_optin && static_cast<size_t>(sh.per_sm) * (smem + 1024) <= static_cast<size_t>(per_sm_bytes) &&
-         sh.block * sh.per_sm <= 1024 && sh.block >= 64 && sh.block <= 1024;
+         sh.block * sh.width * sh.per_sm <= 1024 && sh.block >= 64 && sh.block <= 512;
 }
 
 int apply_shape(smp_batch &b, const Shape &sh) {
   const Ctx &c = b.ctx->c;
-  b.block = sh.block;
+  b.block = sh.block * sh.width;
+  b.width = sh.width;
   b.per_sm = sh.per_sm;
   b.subs = sh.subs;
   b.rank_kb = sh.rank_kb;
@@ -187,12 +190,12 @@ Shape autotune(smp_batch &b, Shape start, const smp_batch_cfg *cfg) {
     }
   };
   if (!(cfg && cfg->window > 0))
-    for (int subs : {1, 2, 4, 8}) consider({best.block, best.per_sm, subs, best.rank_kb});
+    for (int subs : {1, 2, 4, 8}) consider({best.block, best.per_sm, subs, best.rank_kb, best.width});
   if (!(cfg && (cfg->block_threads > 0 || cfg->ctas_per_sm > 0)))
-    for (auto bp : {std::pair<int, int>{1024, 1}, {512, 1}, {512, 2}, {256, 2}, {256, 4}})
-      consider({bp.first, bp.second, best.subs, best.rank_kb});
+    for (const Shape &sh : {Shape{512, 1, 1, 0, 2}, {512, 1, 1, 0, 1}, {512, 2, 1, 0, 1}, {256, 2, 1, 0, 1}, {256, 4, 1, 0, 1}})
+      consider({sh.block, sh.per_sm, best.subs, best.rank_kb, sh.width});
   if (!(cfg && cfg->rank_smem_kb != 0))
-    for (int kb : {0, 32, 64}) consider({best.block, best.per_sm, best.subs, kb});
+    for (int kb : {0, 32, 64}) consider({best.block, best.per_sm, best.subs, kb, best.width});
   return best;
 }
 
@@ -589,7 +592,8 @@ int smp_b200_batch_run_plain(smp_batch *b, smp_instance *results, smp_batch_stat
 int smp_b200_batch_config(const smp_batch *b, smp_batch_cfg *out) {
   if (!b || !out) return SMP_ERR_INVALID_ARG;
   *out = smp_batch_cfg{};
-  out->block_threads = b->block;
+  out->block_threads = b->block / b->width;
+  out->cta_width = b->width;
   out->ctas_per_sm = b->per_sm;
   out->window = 32 * b->subs;
   out->use_graph = b->exec ? 1 : -1;
