@@ -59,7 +59,9 @@ struct Control {
   int32_t screen_done;    // all have
   int32_t swap_out;       // match[] is written
   int32_t swap_quit;      // a warp of the proposals beside it gave up
-  int32_t swap_pad;
+  int32_t tail_left;      // k_tail_q: chains that have not ended
+  int32_t tail_done;      // none are left and the words are final
+  int32_t tail_pad;
   int2 coop_chain[32];
 };
 

@@ -268,6 +268,9 @@ struct Ctx {
   // poll_rounds the caller reads the control block back and adds steps until
   // the matching is complete.
   bool poll_rounds = false;
+  // The same for the query-mode tail's segments.
+  bool poll_tail = false;
+  int tail_segment = 0;
   int round_step = 0;
   int round_gate = 0;
 
@@ -283,6 +286,7 @@ struct Ctx {
   std::unique_ptr<HostPool> pack_pool;
   std::unique_ptr<HostLink> link;
   DeviceBuf d_husband, d_prank, d_bits;  // the checker's
+  DeviceBuf d_tail;                      // query mode: the tail's lists and state
   // rank mode: the men's starting order and the rounds' state (round_kernels.cuh)
   DeviceBuf d_order, d_score, d_round;
   DeviceBuf d_qcnt, d_qlist;
@@ -296,11 +300,11 @@ struct Ctx {
   cudaEvent_t ev_chunk[kCopyChunks] = {};
   cudaStream_t side_stream = nullptr;  // the women's proposals beside their screen
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  std::array<DeviceBuf *, 31> buffers() {
+  std::array<DeviceBuf *, 32> buffers() {
     return {&d_pref_m, &d_pref_w, &d_pw16, &d_pm16, &d_rank,    &d_rankT,    &d_pr,     &d_prefix, &d_bid,    &d_tailq,
             &d_seen,   &d_ctrl,   &d_match,   &d_husband,  &d_prank,  &d_qcnt,   &d_qlist,
             &gen_keys_a, &gen_keys_b, &gen_seg, &gen_temp, &gen_aux, &d_swap_pos, &d_swap_full, &d_swap_over,
-            &d_swap_rows, &d_order, &d_score, &d_round, &d_bits, &d_swap_near};
+            &d_swap_rows, &d_order, &d_score, &d_round, &d_bits, &d_swap_near, &d_tail};
   }
   int launches = 0;  // kernels launched since the last stage / call
   smp_stats stats = {};

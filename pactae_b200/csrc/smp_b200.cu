@@ -15,6 +15,7 @@
 #include "round_kernels.cuh"
 #include "solve_kernels.cuh"
 #include "swap_kernels.cuh"
+#include "tail_kernels.cuh"
 
 using namespace smpb200;
 
@@ -497,15 +498,95 @@ int launch_tail(Ctx &c, int round, int only_mode) {
   return c.check_launch("k_tail_coop");
 }
 
-int launch_tail_query(Ctx &c) {
-  const size_t smem = tail_smem_bytes(c.n);
-  if (allow_dynamic_smem(c, k_tail_q) !=
-      cudaSuccess)
+TailBufs tail_bufs(const Ctx &c) {
+  const size_t np = tail_people(c.n);
+  unsigned char *p = c.d_tail.as<unsigned char>();
+  TailBufs b;
+  b.list = reinterpret_cast<uint32_t *>(p);
+  b.word = b.list + np * kTailCand;
+  b.park[0] = reinterpret_cast<int32_t *>(b.word + np);
+  b.park[1] = b.park[0] + np;
+  b.first = reinterpret_cast<uint16_t *>(b.park[1] + np);
+  b.from = b.first + np;
+  b.end = b.from + np;
+  return b;
+}
+
+// Segment after segment: the candidate lists on all SMs, then the chains in
+// one CTA with as many list entries per man in shared memory as fit.  Where
+// none do, a segment ends when a thread has read kTailSlow lists from L2
+// (about 0.3 us more each than a step in shared memory; making the lists anew
+// takes about 20 us); where some do, when it has used up kTailSlowExact whole
+// lists and searched the prefix beyond them.  A caller that reads the control block back (c.poll_tail) adds
+// segments until tail_done; otherwise the last one has no limit.  A segment
+// after the tail has ended costs two empty launches, about 4 us.
+constexpr int kTailSlow = 80;
+constexpr int kTailSlowExact = 6;
+constexpr int kTailSegments = 5;       // lists in L2
+constexpr int kTailSegmentsExact = 1;
+constexpr int kTailMore = 6;
+constexpr int kTailMoreExact = 2;
+
+template <int E>
+int enqueue_tail_segments(Ctx &c, int count, bool unlimited) {
+  const TailBufs b = tail_bufs(c);
+  const uint32_t *prefix = c.d_prefix.as<uint32_t>();
+  const unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  Control *ctrl = c.d_ctrl.as<Control>();
+  if (allow_dynamic_smem(c, k_tail_q<E>) != cudaSuccess || allow_dynamic_smem(c, k_tail_lists<true>) != cudaSuccess ||
+      allow_dynamic_smem(c, k_tail_lists<false>) != cudaSuccess)
     return c.fail_cuda("k_tail_q smem attribute");
-  k_tail_q<<<1, 1024, smem, c.stream>>>(c.pref_m, c.d_prefix.as<uint32_t>(), c.K, c.d_bid.as<unsigned long long>(),
-                                        c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(), c.d_match.as<int32_t>(), c.n);
-  c.launches++;
+  const int grid = std::max(1, std::min(c.sm_count * 2, (c.n + kTailListBlock / 32 - 1) / (kTailListBlock / 32)));
+  const size_t cut = sizeof(uint16_t) * tail_people(c.n);
+  for (int i = 0; i < count; ++i) {
+    const int s = c.tail_segment + i;
+    if (s == 0)
+      k_tail_lists<true><<<grid, kTailListBlock, cut, c.stream>>>(prefix, c.K, bid, c.d_tailq.as<int2>(), b, c.n, ctrl);
+    else
+      k_tail_lists<false><<<grid, kTailListBlock, cut, c.stream>>>(prefix, c.K, bid, c.d_tailq.as<int2>(), b, c.n, ctrl);
+    k_tail_q<E><<<1, 1024, tail_q_smem(c.n, E), c.stream>>>(
+        c.pref_m, prefix, c.K, bid, ctrl, b, c.d_match.as<int32_t>(), c.n, s,
+        unlimited && i + 1 == count ? 0 : E > 0 ? kTailSlowExact : kTailSlow);
+  }
+  k_tail_out<<<std::max(1, std::min(c.sm_count * 8, (c.n + 7) / 8)), 256, 0, c.stream>>>(prefix, c.K, b,
+                                                                                        c.d_match.as<int32_t>(), c.n, ctrl);
+  c.tail_segment += count;
+  c.launches += 2 * count + 1;
   return c.check_launch("k_tail_q");
+}
+
+int enqueue_tail(Ctx &c, bool more) {
+  const size_t room = c.smem_optin - 256;  // beside the kernel's static shared memory
+  const bool unlimited = !c.poll_tail || c.tail_segment >= 64;
+  const int exact = more ? kTailMoreExact : kTailSegmentsExact;
+  if (tail_q_smem(c.n, 16) <= room) return enqueue_tail_segments<16>(c, exact, unlimited);
+  if (tail_q_smem(c.n, 8) <= room) return enqueue_tail_segments<8>(c, exact, unlimited);
+  if (tail_q_smem(c.n, 4) <= room) return enqueue_tail_segments<4>(c, exact, unlimited);
+  return enqueue_tail_segments<0>(c, more ? kTailMore : kTailSegments, unlimited);
+}
+
+// Below this n the three launches cost more than their shorter steps save
+// (n = 500: 46 us in one launch, 52 in three; n = 1000: 90 and 75).
+constexpr int kTailMinN = 768;
+
+int launch_tail_query(Ctx &c) {
+  if (c.n > kTailMaxN || c.n < kTailMinN) {
+    if (allow_dynamic_smem(c, k_tail_qw) != cudaSuccess) return c.fail_cuda("k_tail_qw smem attribute");
+    k_tail_qw<<<1, 1024, tail_smem_bytes(c.n), c.stream>>>(c.pref_m, c.d_prefix.as<uint32_t>(), c.K,
+                                                           c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(),
+                                                           c.d_tailq.as<int2>(), c.d_match.as<int32_t>(), c.n);
+    c.launches++;
+    return c.check_launch("k_tail_qw");
+  }
+  const int rc = c.d_tail.ensure(tail_bytes(c.n));
+  c.tail_segment = 0;
+  return rc ? rc : enqueue_tail(c, false);
+}
+
+// Segments of a polled solve that has been read back are not over.
+bool tail_over(const Ctx &c) {
+  const Control &h = *c.h_ctrl;
+  return !(c.poll_tail && c.tail_segment > 0 && h.mode == kModeQuery && !h.status && !h.perfect && !h.retry && !h.tail_done);
 }
 
 template <typename RankT>
@@ -688,8 +769,8 @@ int stage_reset(Ctx &c, int32_t n) {
   c.stats.blocking_pairs = -1;
   c.launches = 0;
   c.known_mode = -1;
-  c.poll_rounds = false;
-  c.round_step = 0;
+  c.poll_rounds = c.poll_tail = false;
+  c.round_step = c.tail_segment = 0;
   c.swapped = false;
   plan(c);
   return SMP_OK;
@@ -729,6 +810,8 @@ int do_stage(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, ui
 void fill_stats(Ctx &c, bool timed_phases) {
   c.stats.proposals = static_cast<int64_t>(c.h_ctrl->proposals);
   c.stats.tail_proposals = static_cast<int64_t>(c.h_ctrl->tail_proposals);
+  if (c.h_ctrl->tail_done && c.h_ctrl->proposals > c.h_ctrl->bulk_proposals)  // k_tail_q counts no proposals
+    c.stats.tail_proposals = static_cast<int64_t>(c.h_ctrl->proposals - c.h_ctrl->bulk_proposals);
   c.stats.bulk_hops = static_cast<int32_t>(c.h_ctrl->bulk_hops);
   c.stats.tail_hops = static_cast<int32_t>(c.h_ctrl->tail_hops);
   c.stats.perfect = c.h_ctrl->perfect;
@@ -802,6 +885,7 @@ int reserve_buffers(Ctx &c, int32_t n) {
   if (!rc) rc = order_buffers(c);
   if (!rc && in_rounds(c)) rc = c.d_round.ensure(round_bytes(n));
   if (!rc && c.rank_bytes == 2 && !in_rounds(c)) rc = c.d_pr.ensure(static_cast<size_t>(n) * n * 2);
+  if (!rc && c.query_ok && n <= kTailMaxN) rc = c.d_tail.ensure(tail_bytes(n));
   if (!rc && c.query_ok) rc = c.d_qcnt.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && c.query_ok)
     rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * query_capacity(n, c.K));
@@ -990,6 +1074,7 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
   if (!rc && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   if (rc) return rc;
   c.pass = c.query_ok ? kPassQuery : kPassPrecheck;
+  c.poll_tail = true;
   return c.query_ok ? enqueue_pass_mode(c, kModeQuery) : read_control(c);
 }
 
@@ -1004,6 +1089,11 @@ int solve_advance(Ctx &c, bool &more) {
     return rc ? rc : enqueue_pass_end(c);
   }
   const bool queried = c.pass == kPassQuery;
+  if (queried && !tail_over(c)) {  // more of the tail than the segments enqueued
+    more = true;
+    const int rc = enqueue_tail(c, true);
+    return rc ? rc : enqueue_pass_end(c);
+  }
   if (queried && (h.perfect || (h.mode == kModeQuery && !h.retry))) return SMP_OK;
   if (c.pass == kPassScreen && !h.swap_fail) {
     c.pass = kPassLast;
@@ -1481,9 +1571,14 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
     if (!rc && cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
     if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
     c.tail_ran = true;
+    c.poll_tail = true;
     if (!rc) rc = enqueue_round<uint16_t>(c, 0);
-    if (!rc) rc = read_control(c);
-    if (!rc) rc = c.sync("round 0");
+    for (bool again = true; !rc && again;) {
+      rc = read_control(c);
+      if (!rc) rc = c.sync("round 0");
+      again = !rc && !tail_over(c);
+      if (again) rc = enqueue_tail(c, true);
+    }
     if (!rc && c.h_ctrl->retry && !c.h_ctrl->status) {
       c.known_mode = -1;
       rc = copy_rest_of_m();

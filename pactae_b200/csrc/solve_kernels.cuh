@@ -1366,8 +1366,10 @@ __global__ void __launch_bounds__(1024, 1) k_tail_coop(const int32_t *__restrict
 }
 
 // ---------------------------------------------------------------------------
-// Query-mode tail.  The same job as k_tail for the mode uniform-like inputs
-// take, where every choice a man reaches lies in his prefix, written for the
+// Query-mode tail where the one of tail_kernels.cuh does not serve: above n =
+// kTailMaxN a man does not fit the 15 bits it gives him, below kTailMinN its
+// three launches cost more than they save.  The same job as k_tail for the mode uniform-like
+// inputs take, where every choice a man reaches lies in his prefix, written for the
 // shortest chain of dependent operations per displacement: the last free
 // man's chain is the critical path of the whole solve (thousands of steps,
 // one after the other, on one SM).  Per step, every lane
@@ -1386,7 +1388,7 @@ __device__ __forceinline__ uint32_t prefix_word(const uint32_t *__restrict__ pre
   return r < Kn ? __ldg(prefix + static_cast<size_t>(m) * K + r) : 0u;
 }
 
-__global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ pref_m,
+__global__ void __launch_bounds__(1024, 1) k_tail_qw(const int32_t *__restrict__ pref_m,
                                                     const uint32_t *__restrict__ prefix, int K,
                                                     const unsigned long long *__restrict__ bid, Control *ctrl,
                                                     const int2 *__restrict__ tail_queue,
