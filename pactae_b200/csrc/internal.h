@@ -358,7 +358,7 @@ inline cudaError_t allow_dynamic_smem(const Ctx &c, Kernel kernel) {
 // solve_begin enqueues the first of its passes and solve_advance,
 // called when the stream has drained, the next (more = false: none is left,
 // call solve_finish).
-enum Pass : int { kPassLast = 0, kPassQuery = 1, kPassPrecheck = 2, kPassScreen = 3 };
+enum Pass : int { kPassLast = 0, kPassQuery = 1, kPassPrecheck = 2, kPassScreen = 3, kPassSmall = 4 };
 int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
                   uint32_t flags);
 int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,

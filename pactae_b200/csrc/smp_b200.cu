@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "round_kernels.cuh"
+#include "small_kernels.cuh"
 #include "solve_kernels.cuh"
 #include "swap_kernels.cuh"
 #include "tail_kernels.cuh"
@@ -769,6 +770,7 @@ int stage_reset(Ctx &c, int32_t n) {
   c.stats.blocking_pairs = -1;
   c.launches = 0;
   c.known_mode = -1;
+  c.pass = kPassLast;
   c.poll_rounds = c.poll_tail = false;
   c.round_step = c.tail_segment = 0;
   c.swapped = false;
@@ -828,7 +830,7 @@ void fill_stats(Ctx &c, bool timed_phases) {
     c.stats.total_ms = elapsed(c, kEvStageEnd, kEvPostEnd);
   }
   // Kernel-level times exist when the inversion and proposal kernels ran.
-  if (c.phase >= 3 && !c.h_ctrl->perfect) {
+  if (c.phase >= 3 && !c.h_ctrl->perfect && c.pass != kPassSmall) {
     c.stats.invert_ms = elapsed(c, kEvPrecheckEnd, kEvInvertEnd);
     c.stats.bulk_ms = elapsed(c, kEvInitEnd, kEvBulkEnd);
     c.stats.tail_ms = c.tail_ran && !c.swapped ? elapsed(c, kEvBulkEnd, kEvCoreEnd) : 0.f;
@@ -1054,6 +1056,34 @@ int enqueue_swap_solve(Ctx &c) {
 
 }  // namespace
 
+namespace {
+
+// One launch does it (small_kernels.cuh): small n, and nothing configured
+// that only the larger pipelines heed.
+bool solve_is_small(const Ctx &c, uint32_t flags) {
+  return c.n >= 1 && c.n <= kSmallMaxN && small_smem(c.n) + 256 <= c.smem_optin && c.prefix_k_cfg == 0 &&
+         c.tail_threshold_cfg == 0 && c.bulk_window_cfg == 0 && c.tail_window_cfg == 0 && c.mode_cfg == 0 &&
+         c.rank_bytes_cfg == 0 && !(flags & (SMP_F_CHECK | SMP_F_VALIDATE));
+}
+
+int enqueue_small(Ctx &c, int32_t *match_out, uint32_t flags) {
+  const bool device = (flags & SMP_F_DEVICE_PTRS) != 0;
+  if (!device) {
+    const int rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
+    if (rc) return rc;
+  }
+  if (allow_dynamic_smem(c, k_small) != cudaSuccess) return c.fail_cuda("k_small smem attribute");
+  k_small<<<1, 1024, small_smem(c.n), c.stream>>>(c.pref_m, c.pref_w, c.n, c.K, (flags & SMP_F_NO_PRECHECK) == 0,
+                                                  device ? match_out : c.d_match.as<int32_t>(), c.h_ctrl);
+  c.launches++;
+  int rc = c.check_launch("k_small");
+  if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (!rc && !device) rc = copy_match_out(c, match_out, false);
+  return rc;
+}
+
+}  // namespace
+
 int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
                 uint32_t flags) {
   // The tail is this n's (plan), not the previous solve's: a fresh context's
@@ -1069,6 +1099,10 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }
   int rc = do_stage(c, pref_m, pref_w, n, flags);
+  if (!rc && solve_is_small(c, flags)) {
+    c.pass = kPassSmall;
+    return enqueue_small(c, match_out, flags);
+  }
   if (!rc) rc = enqueue_precheck(c, (flags & SMP_F_NO_PRECHECK) == 0);
   if (!rc && (flags & SMP_F_VALIDATE)) rc = enqueue_validate(c);
   if (!rc && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
@@ -1081,7 +1115,8 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
 int solve_advance(Ctx &c, bool &more) {
   more = false;
   const Control &h = *c.h_ctrl;
-  if (h.status) return SMP_OK;
+  if (c.pass == kPassSmall) c.swapped = h.swap_out != 0;
+  if (h.status || c.pass == kPassSmall) return SMP_OK;
   if (c.pass == kPassLast) {
     if (!rounds_left(c)) return SMP_OK;
     more = true;  // parked men the enqueued steps did not reach
@@ -1153,7 +1188,11 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
 // Statistics and status of a solve whose stream has completed.
 int solve_finish(Ctx &c, uint32_t flags, smp_stats *st) {
   c.phase = 3;
-  fill_stats(c, true);
+  fill_stats(c, c.pass != kPassSmall);
+  if (c.pass == kPassSmall) {  // one launch, all of it the core
+    c.stats.stage_ms = elapsed(c, kEvStageBegin, kEvStageEnd);
+    c.stats.core_ms = c.stats.total_ms = elapsed(c, kEvStageEnd, kEvPostEnd);
+  }
   c.phase = 4;
   if (flags & SMP_F_CHECK) {
     c.stats.blocking_pairs = static_cast<int64_t>(c.h_ctrl->blocking);
