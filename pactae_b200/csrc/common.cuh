@@ -61,7 +61,7 @@ struct Control {
   int32_t swap_quit;      // a warp of the proposals beside it gave up
   int32_t tail_left;      // k_tail_q: chains that have not ended
   int32_t tail_done;      // none are left and the words are final
-  int32_t tail_pad;
+  int32_t check_deep;     // k_check_near: some man's wife is not among his first choices
   int2 coop_chain[32];
 };
 

@@ -264,6 +264,7 @@ struct Ctx {
   int pass = 0;
   uint32_t pass_flags = 0;
   int32_t *pass_match = nullptr;
+  bool match_direct = false;  // a kernel may write pass_match
   // Rank mode in rounds: the steps enqueued so far and their gate; with
   // poll_rounds the caller reads the control block back and adds steps until
   // the matching is complete.
@@ -274,7 +275,9 @@ struct Ctx {
   int round_step = 0;
   int round_gate = 0;
 
-  DeviceBuf d_pref_m, d_pref_w, d_rank, d_rankT, d_pr, d_prefix, d_bid, d_tailq, d_seen, d_ctrl, d_match;
+  DeviceBuf d_pref_m, d_pref_w, d_rank, d_rankT, d_pr, d_prefix, d_bid, d_tailq, d_match;
+  DeviceBuf d_ctrl;  // the control block, the query buckets' counts and the precheck's bitmap
+  bool qcnt_clean = false, bid_clean = false;  // the precheck reset them and nothing has used them since
   DeviceBuf d_pw16, d_pm16;  // pref_w and pref_m packed to uint16 (host-input solves)
   DeviceBuf d_swap_near;  // women-proposing solves: each woman's first choices in 16 bits
   DeviceBuf d_swap_pos;  // women-proposing solves: position of each woman in the men's shared list
@@ -289,7 +292,7 @@ struct Ctx {
   DeviceBuf d_tail;                      // query mode: the tail's lists and state
   // rank mode: the men's starting order and the rounds' state (round_kernels.cuh)
   DeviceBuf d_order, d_score, d_round;
-  DeviceBuf d_qcnt, d_qlist;
+  DeviceBuf d_qlist;
   DeviceBuf gen_keys_a, gen_keys_b, gen_seg, gen_temp, gen_aux;
   Control *h_ctrl = nullptr;  // pinned host copy of the control block
   cudaEvent_t ev[10] = {};
@@ -300,9 +303,9 @@ struct Ctx {
   cudaEvent_t ev_chunk[kCopyChunks] = {};
   cudaStream_t side_stream = nullptr;  // the women's proposals beside their screen
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  std::array<DeviceBuf *, 32> buffers() {
+  std::array<DeviceBuf *, 30> buffers() {
     return {&d_pref_m, &d_pref_w, &d_pw16, &d_pm16, &d_rank,    &d_rankT,    &d_pr,     &d_prefix, &d_bid,    &d_tailq,
-            &d_seen,   &d_ctrl,   &d_match,   &d_husband,  &d_prank,  &d_qcnt,   &d_qlist,
+            &d_ctrl,   &d_match,   &d_husband,  &d_prank,  &d_qlist,
             &gen_keys_a, &gen_keys_b, &gen_seg, &gen_temp, &gen_aux, &d_swap_pos, &d_swap_full, &d_swap_over,
             &d_swap_rows, &d_order, &d_score, &d_round, &d_bits, &d_swap_near, &d_tail};
   }

@@ -124,16 +124,25 @@ void plan(Ctx &c) {
   c.tail_threshold_rank = c.tail_threshold_cfg > 0 ? c.tail_threshold_cfg : kDefaultRankTailThreshold;
 }
 
+// What a solve needs zeroed, in one buffer and one reset: the control block,
+// the query buckets' counts and the precheck's bitmap.
+constexpr size_t kCtrlBytes = (sizeof(Control) + 255) & ~static_cast<size_t>(255);
+size_t zero_bytes(int n) {
+  return kCtrlBytes + sizeof(int32_t) * (static_cast<size_t>(n) + (static_cast<size_t>(n) + 31) / 32);
+}
+int32_t *qcnt_of(const Ctx &c) { return reinterpret_cast<int32_t *>(c.d_ctrl.as<unsigned char>() + kCtrlBytes); }
+uint32_t *seen_of(const Ctx &c) { return reinterpret_cast<uint32_t *>(qcnt_of(c) + c.n); }
+
 int enqueue_precheck(Ctx &c, bool allow_perfect) {
   const int n = c.n;
+  const int rc = c.d_bid.ensure(sizeof(unsigned long long) * static_cast<size_t>(n));
+  if (rc) return rc;
   // zeroed on the device, never copied from the host block (k_precheck)
-  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, sizeof(Control), c.stream) != cudaSuccess)
-    return c.fail_cuda("control reset");
-  const size_t words = (static_cast<size_t>(n) + 31) / 32;
-  if (cudaMemsetAsync(c.d_seen.ptr, 0, words * 4, c.stream) != cudaSuccess) return c.fail_cuda("seen reset");
+  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, zero_bytes(n), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
-  k_precheck<<<grid, 256, 0, c.stream>>>(c.pref_m, n, c.d_seen.as<uint32_t>(), c.d_ctrl.as<Control>(),
-                                         allow_perfect ? 1 : 0, c.query_ok ? 1 : 0);
+  k_precheck<<<grid, 256, 0, c.stream>>>(c.pref_m, n, seen_of(c), c.d_bid.as<unsigned long long>(),
+                                         c.d_ctrl.as<Control>(), allow_perfect ? 1 : 0, c.query_ok ? 1 : 0);
+  c.qcnt_clean = c.bid_clean = true;
   c.launches++;
   return c.check_launch("k_precheck");
 }
@@ -336,13 +345,13 @@ int enqueue_query_index(Ctx &c) {
   const int n = c.n;
   const int qcap = query_capacity(n, c.K);
   const size_t total = static_cast<size_t>(n) * c.K;
-  int rc = c.d_qcnt.ensure(sizeof(int32_t) * static_cast<size_t>(n));
-  if (!rc) rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * qcap);
+  const int rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * qcap);
   if (rc) return rc;
-  if (cudaMemsetAsync(c.d_qcnt.ptr, 0, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess)
+  if (!c.qcnt_clean && cudaMemsetAsync(qcnt_of(c), 0, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("qcnt reset");
+  c.qcnt_clean = false;
   const int grid = static_cast<int>(std::min<size_t>(static_cast<size_t>(c.sm_count) * 16, (total + 255) / 256));
-  k_qscatter<<<grid, 256, 0, c.stream>>>(c.pref_m, n, c.K, qcap, c.d_qcnt.as<int32_t>(), c.d_qlist.as<uint32_t>(),
+  k_qscatter<<<grid, 256, 0, c.stream>>>(c.pref_m, n, c.K, qcap, qcnt_of(c), c.d_qlist.as<uint32_t>(),
                                          c.d_ctrl.as<Control>());
   c.launches++;
   return c.check_launch("k_qscatter");
@@ -364,7 +373,7 @@ int enqueue_qinvert(Ctx &c, int w0, int w1) {
     per_sm = 1;
   }
   const int qgrid = std::max(1, std::min(w1 - w0, c.sm_count * std::max(per_sm, 1)));
-  kernel<<<qgrid, block, smem, c.stream>>>(c.pref_w, c.n, c.K, query_capacity(c.n, c.K), c.d_qcnt.as<int32_t>(),
+  kernel<<<qgrid, block, smem, c.stream>>>(c.pref_w, c.n, c.K, query_capacity(c.n, c.K), qcnt_of(c),
                                          c.d_qlist.as<uint32_t>(), c.d_prefix.as<uint32_t>(), c.d_ctrl.as<Control>(),
                                          w0, w1);
   c.launches++;
@@ -382,7 +391,7 @@ int enqueue_qinvert16(Ctx &c, int w0, int w1) {
   }
   const int qgrid = std::max(1, std::min(w1 - w0, c.sm_count * std::max(per_sm, 1)));
   k_qinvert_p16<<<qgrid, 256, smem, c.stream>>>(c.d_pw16.as<uint16_t>(), c.n, c.K, query_capacity(c.n, c.K),
-                                                c.d_qcnt.as<int32_t>(), c.d_qlist.as<uint32_t>(),
+                                                qcnt_of(c), c.d_qlist.as<uint32_t>(),
                                                 c.d_prefix.as<uint32_t>(), c.d_ctrl.as<Control>(), w0, w1);
   c.launches++;
   return c.check_launch("k_qinvert_p16");
@@ -403,8 +412,9 @@ int init_buffers(Ctx &c) {
   if (!rc) rc = c.d_tailq.ensure(sizeof(int2) * static_cast<size_t>(n));
   if (!rc) rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (rc) return rc;
-  if (cudaMemsetAsync(c.d_bid.ptr, 0xFF, sizeof(unsigned long long) * n, c.stream) != cudaSuccess)
+  if (!c.bid_clean && cudaMemsetAsync(c.d_bid.ptr, 0xFF, sizeof(unsigned long long) * n, c.stream) != cudaSuccess)
     return c.fail_cuda("bid reset");
+  c.bid_clean = false;  // (the precheck frees every woman)
   return SMP_OK;
 }
 
@@ -513,6 +523,22 @@ TailBufs tail_bufs(const Ctx &c) {
   return b;
 }
 
+// Where a query pass and a small solve leave the matching.  The caller's own
+// array where a kernel may write it (this device's memory): the copy it saves
+// took 2 of 105 us of a perfect solve at n = 927.
+bool kernel_may_write(const Ctx &c, const int32_t *p) {
+  cudaPointerAttributes a;
+  if (reinterpret_cast<uintptr_t>(p) % sizeof(int32_t) || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == c.device;
+}
+bool writes_match_here(const Ctx &c) {
+  return c.match_direct && (c.pass == kPassSmall || (c.pass == kPassQuery && in_rounds(c)));
+}
+int32_t *match_here(const Ctx &c) { return writes_match_here(c) ? c.pass_match : c.d_match.as<int32_t>(); }
+
 // Segment after segment: the candidate lists on all SMs, then the chains in
 // one CTA with as many list entries per man in shared memory as fit.  Where
 // none do, a segment ends when a thread has read kTailSlow lists from L2
@@ -546,11 +572,11 @@ int enqueue_tail_segments(Ctx &c, int count, bool unlimited) {
     else
       k_tail_lists<false><<<grid, kTailListBlock, cut, c.stream>>>(prefix, c.K, bid, c.d_tailq.as<int2>(), b, c.n, ctrl);
     k_tail_q<E><<<1, 1024, tail_q_smem(c.n, E), c.stream>>>(
-        c.pref_m, prefix, c.K, bid, ctrl, b, c.d_match.as<int32_t>(), c.n, s,
+        c.pref_m, prefix, c.K, bid, ctrl, b, match_here(c), c.n, s,
         unlimited && i + 1 == count ? 0 : E > 0 ? kTailSlowExact : kTailSlow);
   }
-  k_tail_out<<<std::max(1, std::min(c.sm_count * 8, (c.n + 7) / 8)), 256, 0, c.stream>>>(prefix, c.K, b,
-                                                                                        c.d_match.as<int32_t>(), c.n, ctrl);
+  k_tail_out<<<std::max(1, std::min(c.sm_count * 8, (c.n + 7) / 8)), 256, 0, c.stream>>>(prefix, c.K, b, match_here(c),
+                                                                                        c.n, ctrl);
   c.tail_segment += count;
   c.launches += 2 * count + 1;
   return c.check_launch("k_tail_q");
@@ -575,7 +601,7 @@ int launch_tail_query(Ctx &c) {
     if (allow_dynamic_smem(c, k_tail_qw) != cudaSuccess) return c.fail_cuda("k_tail_qw smem attribute");
     k_tail_qw<<<1, 1024, tail_smem_bytes(c.n), c.stream>>>(c.pref_m, c.d_prefix.as<uint32_t>(), c.K,
                                                            c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(),
-                                                           c.d_tailq.as<int2>(), c.d_match.as<int32_t>(), c.n);
+                                                           c.d_tailq.as<int2>(), match_here(c), c.n);
     c.launches++;
     return c.check_launch("k_tail_qw");
   }
@@ -714,7 +740,7 @@ int check_buffers(Ctx &c) {
   const size_t n = static_cast<size_t>(c.n);
   int rc = c.d_husband.ensure(sizeof(int32_t) * n);
   if (!rc && c.n > kU16MaxN) rc = c.d_prank.ensure(sizeof(int32_t) * n);
-  if (!rc && c.n <= kU16MaxN) rc = c.d_bits.ensure(2 * n * check_row_bytes(c.n));
+  if (!rc && c.n <= kU16MaxN) rc = c.d_bits.ensure(2 * n * check_row_bytes(c.n) + n);
   return rc;
 }
 
@@ -752,10 +778,16 @@ int enqueue_check(Ctx &c, const int32_t *match) {
   k_check_bits<<<std::min(n, per_sm(k_check_bits, 512, row_smem)), 512, row_smem, c.stream>>>(c.pref_w, husband, bits,
                                                                                              n, ctrl);
   const int tiles = (n + 255) / 256;
-  k_check_transpose<<<dim3(tiles, tiles), 256, 0, c.stream>>>(bits, bits_t, n);
-  k_check_scan<<<std::min((n + kCheckWarps - 1) / kCheckWarps, per_sm(k_check_scan, 32 * kCheckWarps, scan_smem)),
-                 32 * kCheckWarps, scan_smem, c.stream>>>(c.pref_m, bits_t, match, n, ctrl);
-  c.launches += 4;
+  unsigned char *deep = bits_t + static_cast<size_t>(n) * check_row_bytes(n);
+  const int warps_grid = (n + kCheckWarps - 1) / kCheckWarps;
+  k_check_near<<<std::min(warps_grid, per_sm(k_check_near, 32 * kCheckWarps, 0)), 32 * kCheckWarps, 0, c.stream>>>(
+      c.pref_m, bits, match, deep, n, ctrl);
+  if (n > kCheckNear) {
+    k_check_transpose<<<dim3(tiles, tiles), 256, 0, c.stream>>>(bits, bits_t, n, ctrl);
+    k_check_scan<<<std::min(warps_grid, per_sm(k_check_scan, 32 * kCheckWarps, scan_smem)), 32 * kCheckWarps, scan_smem,
+                   c.stream>>>(c.pref_m, bits_t, match, deep, n, ctrl);
+  }
+  c.launches += n > kCheckNear ? 5 : 3;
   return c.check_launch("k_check");
 }
 
@@ -769,6 +801,7 @@ int stage_reset(Ctx &c, int32_t n) {
   c.stats.n = n;
   c.stats.blocking_pairs = -1;
   c.launches = 0;
+  c.qcnt_clean = c.bid_clean = false;
   c.known_mode = -1;
   c.pass = kPassLast;
   c.poll_rounds = c.poll_tail = false;
@@ -785,8 +818,7 @@ int do_stage(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, ui
     return SMP_ERR_INVALID_ARG;
   }
   stage_reset(c, n);
-  int rc = c.d_ctrl.ensure(sizeof(Control));
-  if (!rc) rc = c.d_seen.ensure(((static_cast<size_t>(n) + 31) / 32) * 4);
+  int rc = c.d_ctrl.ensure(zero_bytes(n));
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvStageBegin], c.stream) != cudaSuccess) return c.fail_cuda("event");
   if (flags & SMP_F_DEVICE_PTRS) {
@@ -880,15 +912,13 @@ void trim_device_pool(int device) {
 int reserve_buffers(Ctx &c, int32_t n) {
   if (n <= 0 || n > SMP_B200_MAX_N) return SMP_ERR_INVALID_ARG;
   stage_reset(c, n);
-  int rc = c.d_ctrl.ensure(sizeof(Control));
-  if (!rc) rc = c.d_seen.ensure(((static_cast<size_t>(n) + 31) / 32) * 4);
+  int rc = c.d_ctrl.ensure(zero_bytes(n));
   if (!rc) rc = init_buffers(c);
   if (!rc) rc = c.d_rankT.ensure(rank_matrix_bytes(c));
   if (!rc) rc = order_buffers(c);
   if (!rc && in_rounds(c)) rc = c.d_round.ensure(round_bytes(n));
   if (!rc && c.rank_bytes == 2 && !in_rounds(c)) rc = c.d_pr.ensure(static_cast<size_t>(n) * n * 2);
   if (!rc && c.query_ok && n <= kTailMaxN) rc = c.d_tail.ensure(tail_bytes(n));
-  if (!rc && c.query_ok) rc = c.d_qcnt.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && c.query_ok)
     rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * query_capacity(n, c.K));
   if (!rc) rc = swap_buffers(c);
@@ -953,7 +983,7 @@ int enqueue_pass_end(Ctx &c) {
   const bool device = (c.pass_flags & SMP_F_DEVICE_PTRS) != 0;
   if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   int rc = enqueue_post(c);
-  if (!rc && device) rc = copy_match_out(c, c.pass_match, true);
+  if (!rc && device && !writes_match_here(c)) rc = copy_match_out(c, c.pass_match, true);
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   if (!rc && !device) rc = copy_match_out(c, c.pass_match, false);
   return rc ? rc : read_control(c);
@@ -981,6 +1011,7 @@ int enqueue_swap_screen(Ctx &c, bool men_screened) {
   Control *ctrl = c.d_ctrl.as<Control>();
   int32_t *pos = c.d_swap_pos.as<int32_t>();
   unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  c.bid_clean = false;
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
   if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
       cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
@@ -1034,6 +1065,7 @@ int enqueue_swap_solve(Ctx &c) {
   const int n = c.n;
   Control *ctrl = c.d_ctrl.as<Control>();
   unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  c.bid_clean = false;
   if (cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
       cudaMemsetAsync(&ctrl->swap_next, 0, sizeof(int32_t), c.stream) != cudaSuccess)
     return c.fail_cuda("swap bid reset");
@@ -1068,17 +1100,17 @@ bool solve_is_small(const Ctx &c, uint32_t flags) {
 
 int enqueue_small(Ctx &c, int32_t *match_out, uint32_t flags) {
   const bool device = (flags & SMP_F_DEVICE_PTRS) != 0;
-  if (!device) {
+  if (!writes_match_here(c)) {
     const int rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
     if (rc) return rc;
   }
   if (allow_dynamic_smem(c, k_small) != cudaSuccess) return c.fail_cuda("k_small smem attribute");
   k_small<<<1, 1024, small_smem(c.n), c.stream>>>(c.pref_m, c.pref_w, c.n, c.K, (flags & SMP_F_NO_PRECHECK) == 0,
-                                                  device ? match_out : c.d_match.as<int32_t>(), c.h_ctrl);
+                                                  match_here(c), c.h_ctrl);
   c.launches++;
   int rc = c.check_launch("k_small");
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (!rc && !device) rc = copy_match_out(c, match_out, false);
+  if (!rc && !writes_match_here(c)) rc = copy_match_out(c, match_out, device);
   return rc;
 }
 
@@ -1099,6 +1131,7 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }
   int rc = do_stage(c, pref_m, pref_w, n, flags);
+  c.match_direct = (flags & SMP_F_DEVICE_PTRS) && kernel_may_write(c, match_out);
   if (!rc && solve_is_small(c, flags)) {
     c.pass = kPassSmall;
     return enqueue_small(c, match_out, flags);
@@ -1366,6 +1399,7 @@ int solve_shared_host(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, uint
   Control *ctrl = c.d_ctrl.as<Control>();
   int32_t *pos = c.d_swap_pos.as<int32_t>();
   unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  c.bid_clean = false;
   uint8_t *full = c.d_swap_full.as<uint8_t>();
   int2 *over[2] = {c.d_swap_over.as<int2>(), c.d_swap_over.as<int2>() + n};
   int32_t *d_rows = c.d_swap_rows.as<int32_t>();
@@ -1499,8 +1533,7 @@ int solve_shared_host(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, uint
 int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
                    uint32_t flags, smp_stats *st) {
   const size_t row = sizeof(int32_t) * static_cast<size_t>(n);
-  int rc = c.d_ctrl.ensure(sizeof(Control));
-  if (!rc) rc = c.d_seen.ensure(((static_cast<size_t>(n) + 31) / 32) * 4);
+  int rc = c.d_ctrl.ensure(zero_bytes(n));
   if (!rc) rc = c.d_pref_m.ensure(row * n);
   if (!rc) rc = c.d_pref_w.ensure(row * n);
   if (rc) return rc;

@@ -98,8 +98,9 @@ __device__ __forceinline__ bool any_unset<int32_t>(uint4 v) {
 // writes them and the free count into it.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_precheck(const int32_t *__restrict__ pref_m, int n,
-                                                  uint32_t *__restrict__ seen, Control *ctrl, int allow_perfect,
-                                                  int allow_query) {
+                                                  uint32_t *__restrict__ seen,
+                                                  unsigned long long *__restrict__ bid, Control *ctrl,
+                                                  int allow_perfect, int allow_query) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctrl->free_count = n;
     ctrl->allow_perfect = allow_perfect;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(256) k_precheck(const int32_t *__restrict__ pr
   }
   const int stride = gridDim.x * blockDim.x;
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += stride) {
+    bid[m] = kFree;  // every woman, too
     const int w = __ldg(pref_m + static_cast<size_t>(m) * n);
     if (static_cast<unsigned>(w) >= static_cast<unsigned>(n)) {
       report(ctrl, kStatusInvalidInput, w);

@@ -12,7 +12,7 @@ import pactae_b200 as pb
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2, 7, 63, 64, 65, 255, 256, 257, 319, 513, 1030])
+@pytest.mark.parametrize("n", [1, 2, 7, 63, 64, 65, 127, 128, 129, 255, 256, 257, 319, 513, 1030])
 @pytest.mark.parametrize("kind,param", [(pb.SMP_GEN_UNIFORM, 0), (pb.SMP_GEN_CORRELATED, 500)])
 def test_checker_matches_oracle(ctx, kind, param, n):
     pm, pw = oracle.generate(kind, n, 23, 0, param)
