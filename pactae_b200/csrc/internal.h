@@ -2,6 +2,7 @@
 // libsmp_b200.so.  Not part of the public ABI (include/smp_b200.h is).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -31,7 +31,7 @@
 // Measured on one B200 against k_bulk, k_tail and k_tail_coop over ranks by
 // position, which still serve int32 ranks and lists whose bids no SM holds:
 // RANDOM(5) n = 15013 18.7 -> 4.0 ms (18.7 M displacements -> 98 thousand),
-// n = 30000 58.8 -> 9.6; SOLO n = 10007 43.6 -> 6.9; correlated n = 30000
+// n = 30000 58.8 -> 9.6; SOLO n = 10007 43.6 -> 3.3; correlated n = 30000
 // 10.8 -> 8.6, n = 2000 0.57 -> 0.53, n = 97 0.25 -> 0.22.  A step of the
 // n = 30000 correlated solve takes about 37 us to scan (592 rows of two
 // lists: 100 MB, half the copy rate), 2 us to load the state, 75 us to
@@ -176,6 +176,12 @@ __host__ __device__ constexpr size_t round_smem_bytes(int n) {
   const size_t resolve = round_words(n) * 6;
   const size_t scan = round_words(n) * 2 + kTeams * (round_bitmap_bytes(n) + kBallotBytes);
   return resolve > scan ? resolve : scan;
+}
+
+// With the resolver's table of the list entry after each man's position.
+__host__ __device__ constexpr size_t round_table_bytes(int n) {
+  const size_t resolve = round_words(n) * 10;
+  return resolve > round_smem_bytes(n) ? resolve : round_smem_bytes(n);
 }
 
 // Every woman free, no man started, the first men in step 0's slot.  A
@@ -436,7 +442,16 @@ __device__ __forceinline__ void round_finish(const RoundBufs &b, const uint32_t 
   }
 }
 
-// One step.
+// One step.  kTable: the resolver keeps the entry after each man's position in
+// shared memory, and a man dropped tries it without a look at his list: 0.1 us
+// on a displacement instead of 0.5.  That pays in a refresh step, where every
+// list is new, his wife its first entry, and the one after it most often takes
+// him; and it takes L1 from the scans.  So the steps past the first
+// ceil(n / batch), by which all men may have started, are the ones with the
+// table.  (With it in every step, RANDOM(5) n = 15013 took 6.4 ms for 4.0 and
+// correlated n = 30000 10.6 for 8.6: filling it reads a line per man, and two
+// entries in five had been overtaken.)
+template <bool kTable>
 __global__ void __launch_bounds__(kRoundBlock, 1)
     k_round(const int32_t *__restrict__ pref_m, const uint16_t *__restrict__ rankT, size_t ld,
             const int32_t *__restrict__ order, RoundBufs b, int32_t *__restrict__ match, int n, int batch, int t,
@@ -478,12 +493,26 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
   const int cap = b.cap;
   uint32_t *sbid = reinterpret_cast<uint32_t *>(smem_raw);
   uint16_t *spos = reinterpret_cast<uint16_t *>(smem_raw + static_cast<size_t>(nw) * 4);
+  uint32_t *snext = reinterpret_cast<uint32_t *>(smem_raw + static_cast<size_t>(nw) * 6);  // kTable
   int32_t *park = b.parkq[(t & 1) ^ 1];
   round_state_in(b, sbid, spos, nw);
   __syncthreads();
+  if (kTable) {
+    if (slot.refresh) {
+#pragma unroll 8
+      for (int i = tid; i < n; i += kRoundBlock) {
+        const int r = spos[i] + 1;
+        snext[i] = r < cap ? b.cand[static_cast<uint32_t>(i * cap + r)] : kNoCand;
+      }
+    } else {
+      for (int i = tid; i < n; i += kRoundBlock) snext[i] = kNoCand;
+    }
+    __syncthreads();
+  }
   unsigned int hops = 0;
   int m = -1, pos = 0;    // the man and the list entry to try next
   uint32_t raw = 0;       // this lane's entry pos + lane of his list
+  uint32_t one = kNoCand;  // kTable: entry pos, where the table has it (raw is not read then)
   const auto entry = [&](int man, int r) { return r < cap ? b.cand[static_cast<uint32_t>(man * cap + r)] : kNoCand; };
   // Moves on to the first window at or after pos that holds a candidate or
   // the end of the list, looking at kWide windows per round trip.
@@ -517,10 +546,36 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     if (i >= ready || *reinterpret_cast<volatile int *>(&s_stop)) return false;
     m = i < slot.parked ? parkq[i] : __ldg(order + slot.new0 + (i - slot.parked));
     pos = 0;
+    one = kNoCand;
     skip();
     return true;
   };
   for (bool more = next_man(); more;) {
+    if (kTable && one != kNoCand) {
+      const uint32_t rk = one & 0xFFFFu;
+      uint32_t old = 0;
+      if (lane == 0) {
+        spos[m] = static_cast<uint16_t>(pos);
+        snext[m] = kNoCand;
+        old = atom_min_relaxed_shared(sbid + (one >> 16), (rk << 16) | static_cast<uint32_t>(m));
+      }
+      old = __shfl_sync(kFullMask, old, 0);
+      if ((old >> 16) > rk) {
+        hops++;
+        if (old == 0xFFFFFFFFu) {
+          more = next_man();
+          continue;
+        }
+        m = static_cast<int>(old & 0xFFFFu);
+        pos = spos[m] + 1;
+        one = snext[m];
+        if (one != kNoCand) continue;
+      } else {
+        one = kNoCand;
+        pos++;
+      }
+      raw = entry(m, pos + lane);
+    }
     const bool ok = raw != kNoCand;  // a window past a list's end holds nothing else
     const int w = ok ? static_cast<int>(raw >> 16) : 0;
     const uint32_t rk = raw & 0xFFFFu;
@@ -559,8 +614,10 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     uint32_t next_raw = 0;
     if (hw != 0xFFFFFFFFu) next_raw = entry(hm, hpos + lane);
     uint32_t old = 0;
+    const uint32_t after = kTable ? __shfl_down_sync(kFullMask, raw, 1) : kNoCand;
     if (lane == j) {
       spos[m] = static_cast<uint16_t>(pos + j);
+      if (kTable) snext[m] = j < 31 ? after : kNoCand;
       old = atom_min_relaxed_shared(sbid + w, (rk << 16) | static_cast<uint32_t>(m));
     }
     old = __shfl_sync(kFullMask, old, j);
@@ -569,6 +626,7 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
       m = hm;
       pos = hpos;
       raw = next_raw;
+      if (kTable) one = snext[m];
       continue;
     }
     if ((old >> 16) <= rkj) continue;  // someone better got there first: read the bids again
@@ -580,6 +638,7 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     m = static_cast<int>(old & 0xFFFFu);
     pos = spos[m] + 1;
     raw = entry(m, pos + lane);
+    if (kTable) one = snext[m];
   }
   if (lane == 0 && hops) atomicAdd(&s_hops, hops);
   __syncthreads();

@@ -300,11 +300,18 @@ constexpr int kRoundMore = 8;
 
 int enqueue_round_steps(Ctx &c, int gate, int count) {
   const RoundBufs b = round_bufs(c);
-  if (allow_dynamic_smem(c, k_round) != cudaSuccess) return c.fail_cuda("k_round smem attribute");
-  for (int i = 0; i < count; ++i)
-    k_round<<<c.sm_count, kRoundBlock, round_smem_bytes(c.n), c.stream>>>(
-        c.pref_m, c.d_rankT.as<uint16_t>(), rank_ld(c), c.d_order.as<int32_t>(), b, c.d_match.as<int32_t>(), c.n,
-        c.sm_count * kTeams, c.round_step + i, c.d_ctrl.as<Control>(), gate);
+  if (allow_dynamic_smem(c, k_round<false>) != cudaSuccess || allow_dynamic_smem(c, k_round<true>) != cudaSuccess)
+    return c.fail_cuda("k_round smem attribute");
+  const int batch = c.sm_count * kTeams;
+  const bool room = round_table_bytes(c.n) + 256 <= c.smem_optin;  // beside the kernel's static shared memory
+  for (int i = 0; i < count; ++i) {
+    const int t = c.round_step + i;
+    const bool table = room && t >= (c.n + batch - 1) / batch;
+    const auto kernel = table ? k_round<true> : k_round<false>;
+    kernel<<<c.sm_count, kRoundBlock, table ? round_table_bytes(c.n) : round_smem_bytes(c.n), c.stream>>>(
+        c.pref_m, c.d_rankT.as<uint16_t>(), rank_ld(c), c.d_order.as<int32_t>(), b, c.d_match.as<int32_t>(), c.n, batch,
+        t, c.d_ctrl.as<Control>(), gate);
+  }
   c.round_step += count;
   c.launches += count;
   return c.check_launch("k_round");
@@ -524,15 +531,32 @@ TailBufs tail_bufs(const Ctx &c) {
 }
 
 // Where a query pass and a small solve leave the matching.  The caller's own
-// array where a kernel may write it (this device's memory): the copy it saves
-// took 2 of 105 us of a perfect solve at n = 927.
-bool kernel_may_write(const Ctx &c, const int32_t *p) {
+// array where a kernel may write all of it (this device's memory, one
+// allocation; what else a copy takes or refuses stays the copy's): the copy it
+// saves took 2 of 105 us of a perfect solve at n = 927.
+bool kernel_may_write(const Ctx &c, const int32_t *p, size_t bytes) {
+  using AddressRange = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+  static const AddressRange range = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<AddressRange>(f);
+  }();
   cudaPointerAttributes a;
-  if (reinterpret_cast<uintptr_t>(p) % sizeof(int32_t) || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if (!range || at % sizeof(int32_t)) return false;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == c.device;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  return a.type == cudaMemoryTypeDevice && a.device == c.device && range(&base, &size, at) == CUDA_SUCCESS &&
+         at - base + bytes <= size;
 }
 bool writes_match_here(const Ctx &c) {
   return c.match_direct && (c.pass == kPassSmall || (c.pass == kPassQuery && in_rounds(c)));
@@ -1131,7 +1155,7 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }
   int rc = do_stage(c, pref_m, pref_w, n, flags);
-  c.match_direct = (flags & SMP_F_DEVICE_PTRS) && kernel_may_write(c, match_out);
+  c.match_direct = (flags & SMP_F_DEVICE_PTRS) && n > 0 && kernel_may_write(c, match_out, sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && solve_is_small(c, flags)) {
     c.pass = kPassSmall;
     return enqueue_small(c, match_out, flags);

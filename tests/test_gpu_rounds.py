@@ -66,3 +66,13 @@ def test_rounds_refuse_an_entry_out_of_range(where):
             with pytest.raises(pb.SmpError) as e:
                 c.solve(pm, pw, check=check)
             assert e.value.status == pb.SMP_ERR_INVALID_INPUT
+
+
+@pytest.mark.parametrize("n", [23216, 23217])
+def test_rounds_at_the_table_limit(n):
+    # the largest n whose refresh steps have the table of next entries, and the next
+    with pb.Context() as c:
+        pm, pw = c.generate(pb.SMP_GEN_SOLO, n, 3)
+        match, st = c.solve(pm, pw)
+        again, st2 = c.solve(pm, pw, check=True)
+        assert bool((match == again).all()) and st["proposals"] == st2["proposals"] and st2["blocking_pairs"] == 0

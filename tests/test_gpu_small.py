@@ -54,3 +54,16 @@ def test_small_refuses_what_the_pipeline_refuses(ctx, kind, param, n):
                 except pb.SmpError as e:
                     outcome.append(e.status)
             assert outcome[0] == outcome[1], (where, row, col)
+
+
+@pytest.mark.parametrize("n", [97, 300, 927])
+def test_match_where_no_kernel_may_write(n):
+    # pinned host memory as the device solve's output: copied there, as ever
+    import torch
+
+    with pb.Context() as c:
+        pm, pw = c.generate(pb.SMP_GEN_UNIFORM, n, 5)
+        want, _ = c.solve(pm, pw)
+        out = torch.full((n,), -1, dtype=torch.int32).pin_memory()
+        match, _ = c.solve(pm, pw, out=out)
+        assert bool((match == want.cpu()).all())
