@@ -12,7 +12,7 @@
 //            only improve, so a woman left out would reject him at any later
 //            time: this list replaces his preference row;
 //   resolves them on the CTA that finishes scanning last: a warp per
-//            displacement chain, bids and positions in shared memory, every
+//            displacement chain, or eight lanes, bids and positions in shared memory, every
 //            choice read from the candidate lists.  A man whose list is used
 //            up is parked and scanned again, from where he stopped, in the
 //            next step.
@@ -31,19 +31,20 @@
 // Measured on one B200 against k_bulk, k_tail and k_tail_coop over ranks by
 // position, which still serve int32 ranks and lists whose bids no SM holds:
 // RANDOM(5) n = 15013 18.7 -> 4.0 ms (18.7 M displacements -> 98 thousand),
-// n = 30000 58.8 -> 9.6; SOLO n = 10007 43.6 -> 3.3; correlated n = 30000
-// 10.8 -> 8.6, n = 2000 0.57 -> 0.53, n = 97 0.25 -> 0.22.  A step of the
-// n = 30000 correlated solve takes about 37 us to scan (592 rows of two
-// lists: 100 MB, half the copy rate), 2 us to load the state, 75 us to
+// n = 30000 58.8 -> 9.6; SOLO n = 10007 43.6 -> 3.0; correlated n = 30000
+// 10.8 -> 7.9, n = 2000 0.57 -> 0.53, n = 97 0.25 -> 0.22.  A step of the
+// n = 30000 correlated solve takes about 36 us to scan (592 rows of two
+// lists: 100 MB, half the copy rate), 2 us to load the state, 64 us to
 // resolve and 10 us between launches.  The resolver is bound by the latency
-// of a displacement (0.46 us, an L2 read of the next window on it) and, at 32
-// warps, by the SM's issue slots (0.58 us): 24 or 16 warps take 7.4 and
-// 8.6 ms for those proposals where 32 take 6.9.  Batches of 296 and 1184 men
-// were slower than 592 (9.4 and 6.3 against 6.8 ms correlated, 10.6 and 13.3
-// against 8.5 ms RANDOM(5), n = 30000): a man skips those of his own batch
-// one by one, and a step costs what it costs.  Scanning a batch ahead while
-// the last one is resolved does not pay for the same reason: the men then
-// skip two batches.
+// of a displacement (0.46 us by warp, an L2 read of the next window on it; 0.5
+// to 0.74 by eight lanes, where four chains wait for one another) and, at 32
+// warps with a chain each, by the SM's issue slots (0.58 us): 24 or 16 warps
+// take 7.4 and 8.6 ms for RANDOM(5)'s proposals where 32 take 6.9.  Batches of
+// 296 and 1184 men were slower than 592 (9.4 and 6.3 against 6.8 ms
+// correlated, 10.6 and 13.3 against 8.5 ms RANDOM(5), n = 30000): a man skips
+// those of his own batch one by one, and a step costs what it costs.  Scanning
+// a batch ahead while the last one is resolved does not pay for the same
+// reason: the men then skip two batches.
 #pragma once
 
 #include "common.cuh"
@@ -148,6 +149,7 @@ struct RoundCtl {
   int32_t done;        // the matching is complete and written
   int32_t steps;       // steps that ran
   int32_t refreshes;
+  int32_t calm;        // 1: few proposals of the step before came too late; -1: many did at four times the chains
 };
 
 struct RoundBufs {
@@ -442,78 +444,59 @@ __device__ __forceinline__ void round_finish(const RoundBufs &b, const uint32_t 
   }
 }
 
-// One step.  kTable: the resolver keeps the entry after each man's position in
-// shared memory, and a man dropped tries it without a look at his list: 0.1 us
-// on a displacement instead of 0.5.  That pays in a refresh step, where every
-// list is new, his wife its first entry, and the one after it most often takes
-// him; and it takes L1 from the scans.  So the steps past the first
-// ceil(n / batch), by which all men may have started, are the ones with the
-// table.  (With it in every step, RANDOM(5) n = 15013 took 6.4 ms for 4.0 and
-// correlated n = 30000 10.6 for 8.6: filling it reads a line per man, and two
-// entries in five had been overtaken.)
+// What the chains of a step work on.
+struct RoundChains {
+  const int32_t *order;
+  const int32_t *parkq;
+  RoundBufs b;
+  RoundSlot slot;
+  uint32_t *sbid;   // shared: the women's words
+  uint16_t *spos;   // shared: the entries the men have reached
+  uint32_t *snext;  // shared, chains_by_warp: the entries after those
+  int32_t *park;    // the men parked for the next step
+  int *s_next, *s_parked, *s_stop;
+  int ready, n;
+  Control *ctrl;
+};
+
+// Displacements, and proposals that met someone better who had just got there.
+struct RoundCount {
+  unsigned int hops, lost;
+};
+
+// A chain per warp.  kTable: with a table of the list entry after each man's
+// position; a man dropped tries it without a look at his list, 0.1 us on a
+// displacement instead of 0.5.  That pays in a refresh step, where every list
+// is new, his wife its first entry, and the one after it most often takes him.
+// (With the table in every step, RANDOM(5) n = 15013 took 6.4 ms for 4.0 and
+// correlated n = 30000 10.6 for 8.6: filling it reads a line per man, it takes
+// L1 from the scans, and two entries in five had been overtaken.)  Counts in
+// lane 0.
 template <bool kTable>
-__global__ void __launch_bounds__(kRoundBlock, 1)
-    k_round(const int32_t *__restrict__ pref_m, const uint16_t *__restrict__ rankT, size_t ld,
-            const int32_t *__restrict__ order, RoundBufs b, int32_t *__restrict__ match, int n, int batch, int t,
-            Control *ctrl, int gate) {
-  __shared__ int s_go;
-  __shared__ int s_next, s_parked, s_stop;
-  __shared__ unsigned long long s_props;
-  __shared__ unsigned int s_hops;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  if (tid == 0) s_go = gate_open(gate, ctrl) && !ld_volatile_s32(&b.ctl->done);
-  __syncthreads();  // read once: another CTA may report an error meanwhile
-  if (!s_go) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const RoundSlot slot = b.ctl->slot[t & 1];
-  const int32_t *parkq = b.parkq[t & 1];
-  const int ready = slot.parked + (slot.new1 - slot.new0);
-  const int items = slot.refresh ? n : ready;
-  if (static_cast<int>(blockIdx.x) * kTeams < items)
-    round_scan(pref_m, rankT, ld, order, b, slot, parkq, items, n, smem_raw, ctrl);
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_go = atomicAdd(&b.ctl->arrived[t & 1], 1) == static_cast<int>(gridDim.x) - 1;
-    s_next = 0;
-    s_parked = 0;
-    s_stop = 0;
-    s_props = 0;
-    s_hops = 0;
-  }
-  __syncthreads();
-  if (!s_go) {
-    round_check(pref_m, order, slot.new0, slot.new1, &b.ctl->checked[t & 1], n, ctrl);
-    return;
-  }
-  __threadfence();  // the other CTAs' lists
-  // ---- the last CTA resolves ----
-  const int nw = static_cast<int>(round_words(n));
-  const int cap = b.cap;
-  uint32_t *sbid = reinterpret_cast<uint32_t *>(smem_raw);
-  uint16_t *spos = reinterpret_cast<uint16_t *>(smem_raw + static_cast<size_t>(nw) * 4);
-  uint32_t *snext = reinterpret_cast<uint32_t *>(smem_raw + static_cast<size_t>(nw) * 6);  // kTable
-  int32_t *park = b.parkq[(t & 1) ^ 1];
-  round_state_in(b, sbid, spos, nw);
-  __syncthreads();
+__device__ __forceinline__ RoundCount chains_by_warp(const RoundChains &q) {
+  const int n = q.n;
+  const int cap = q.b.cap;
+  const int lane = threadIdx.x & 31;
+  uint32_t *sbid = q.sbid;
+  uint16_t *spos = q.spos;
+  uint32_t *snext = q.snext;
   if (kTable) {
-    if (slot.refresh) {
+    if (q.slot.refresh) {
 #pragma unroll 8
-      for (int i = tid; i < n; i += kRoundBlock) {
+      for (int i = threadIdx.x; i < n; i += kRoundBlock) {
         const int r = spos[i] + 1;
-        snext[i] = r < cap ? b.cand[static_cast<uint32_t>(i * cap + r)] : kNoCand;
+        snext[i] = r < cap ? q.b.cand[static_cast<uint32_t>(i * cap + r)] : kNoCand;
       }
     } else {
-      for (int i = tid; i < n; i += kRoundBlock) snext[i] = kNoCand;
+      for (int i = threadIdx.x; i < n; i += kRoundBlock) snext[i] = kNoCand;
     }
     __syncthreads();
   }
-  unsigned int hops = 0;
+  unsigned int hops = 0, lost = 0;
   int m = -1, pos = 0;    // the man and the list entry to try next
   uint32_t raw = 0;       // this lane's entry pos + lane of his list
   uint32_t one = kNoCand;  // kTable: entry pos, where the table has it (raw is not read then)
-  const auto entry = [&](int man, int r) { return r < cap ? b.cand[static_cast<uint32_t>(man * cap + r)] : kNoCand; };
+  const auto entry = [&](int man, int r) { return r < cap ? q.b.cand[static_cast<uint32_t>(man * cap + r)] : kNoCand; };
   // Moves on to the first window at or after pos that holds a candidate or
   // the end of the list, looking at kWide windows per round trip.
   const auto skip = [&]() {
@@ -541,10 +524,10 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
   };
   const auto next_man = [&]() {
     int i = 0;
-    if (lane == 0) i = atomicAdd(&s_next, 1);
+    if (lane == 0) i = atomicAdd(q.s_next, 1);
     i = __shfl_sync(kFullMask, i, 0);
-    if (i >= ready || *reinterpret_cast<volatile int *>(&s_stop)) return false;
-    m = i < slot.parked ? parkq[i] : __ldg(order + slot.new0 + (i - slot.parked));
+    if (i >= q.ready || *reinterpret_cast<volatile int *>(q.s_stop)) return false;
+    m = i < q.slot.parked ? q.parkq[i] : __ldg(q.order + q.slot.new0 + (i - q.slot.parked));
     pos = 0;
     one = kNoCand;
     skip();
@@ -587,14 +570,14 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
       if (end) {
         if (pos + __ffs(end) - 1 < cap) {  // the list held every woman left: rejected by all of them
           if (lane == 0) {
-            report(ctrl, kStatusInvalidInput, m);
-            s_stop = 1;
+            report(q.ctrl, kStatusInvalidInput, m);
+            *q.s_stop = 1;
           }
           break;
         }
         if (lane == 0) {
           spos[m] = static_cast<uint16_t>(cap - 1);
-          park[atomicAdd(&s_parked, 1)] = m;
+          q.park[atomicAdd(q.s_parked, 1)] = m;
         }
         more = next_man();
       } else {
@@ -629,7 +612,10 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
       if (kTable) one = snext[m];
       continue;
     }
-    if ((old >> 16) <= rkj) continue;  // someone better got there first: read the bids again
+    if ((old >> 16) <= rkj) {  // someone better got there first: read the bids again
+      lost++;
+      continue;
+    }
     hops++;
     if (old == 0xFFFFFFFFu) {
       more = next_man();  // the chain ended at a free woman
@@ -640,7 +626,179 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     raw = entry(m, pos + lane);
     if (kTable) one = snext[m];
   }
-  if (lane == 0 && hops) atomicAdd(&s_hops, hops);
+  return lane == 0 ? RoundCount{hops, lost} : RoundCount{0, 0};
+}
+
+// A chain per eight lanes, four in a warp: a window of a list is 16 bytes per
+// lane.  At 32 chains the SM's issue slots were the bound (0.58 us on a
+// displacement), here a step's longest chain is (70 windows of 0.74 us where
+// the mean is 30 of 1.1): correlated n = 30000 8.6 -> 7.9 ms, n = 8000 1.54 ->
+// 1.37, SOLO n = 10007 3.3 -> 3.0.  Counts in the first lane of each eight.
+__device__ __forceinline__ RoundCount chains_by_group(const RoundChains &q) {
+  const int n = q.n;
+  const int cap = q.b.cap;
+  const int lane = threadIdx.x & 31;
+  const int gl = lane & 7;
+  const int g0 = lane & 24;
+  uint32_t *sbid = q.sbid;
+  uint16_t *spos = q.spos;
+  const auto window = [&](int man, int pos) {  // from the 16-byte boundary at or before pos
+    const int r = (pos & ~3) + 4 * gl;
+    return r < cap ? *reinterpret_cast<const uint4 *>(q.b.cand + static_cast<uint32_t>(man * cap + r))
+                   : make_uint4(kNoCand, kNoCand, kNoCand, kNoCand);
+  };
+  unsigned int hops = 0, lost = 0;
+  bool has = false, out = false;  // a man; no more of them
+  bool fresh = false;             // his window is still to be loaded
+  int m = 0, pos = 0;             // the man and the list entry to try next
+  uint4 v = make_uint4(kNoCand, kNoCand, kNoCand, kNoCand);
+  for (;;) {
+    const bool ask = !has && !out;
+    if (__any_sync(kFullMask, ask)) {
+      int i = 0;
+      if (ask && gl == 0) i = atomicAdd(q.s_next, 1);
+      i = __shfl_sync(kFullMask, i, g0);
+      if (ask) {
+        has = i < q.ready && !*reinterpret_cast<volatile int *>(q.s_stop);
+        out = !has;
+        fresh = has;
+        if (has) m = i < q.slot.parked ? q.parkq[i] : __ldg(q.order + q.slot.new0 + (i - q.slot.parked));
+        pos = 0;
+      }
+    }
+    if (!__any_sync(kFullMask, has)) break;
+    if (fresh) v = window(m, pos);
+    fresh = false;
+    const int at = (pos & ~3) + 4 * gl;
+    const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+    int f = -1;              // this lane's first entry that takes him, and her word
+    uint32_t fe = 0, fw = 0;
+    bool end = false;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      // (a window past a list's end holds nothing else; leftovers are not reached)
+      const uint32_t word = lds_relaxed_u32(sbid + min(e[k] >> 16, static_cast<uint32_t>(n - 1)));
+      end |= e[k] == kNoCand;
+      if (at + k >= pos && e[k] != kNoCand && (e[k] & 0xFFFFu) < (word >> 16)) {
+        f = k;
+        fe = e[k];
+        fw = word;
+      }
+    }
+    const unsigned hits = (__ballot_sync(kFullMask, has && f >= 0) >> g0) & 0xFFu;
+    const unsigned ends = (__ballot_sync(kFullMask, has && end) >> g0) & 0xFFu;
+    const unsigned short_end = (__ballot_sync(kFullMask, has && end && at < cap) >> g0) & 0xFFu;
+    const bool found = hits != 0;
+    const int src = found ? g0 + __ffs(hits) - 1 : lane;
+    const uint32_t rk = __shfl_sync(kFullMask, fe, src) & 0xFFFFu;
+    const uint32_t hw = __shfl_sync(kFullMask, fw, src);
+    if (has && !found) {
+      if (!ends) {
+        pos = (pos & ~3) + 32;
+        fresh = true;
+      } else {
+        if (gl == 0) {
+          if (short_end) {  // the list held every woman left: rejected by all of them
+            report(q.ctrl, kStatusInvalidInput, m);
+            *q.s_stop = 1;
+          } else {
+            spos[m] = static_cast<uint16_t>(cap - 1);
+            q.park[atomicAdd(q.s_parked, 1)] = m;
+          }
+        }
+        has = false;
+      }
+    }
+    // the window of the man she would drop, while the proposal is under way
+    int hpos = 0;
+    uint4 hv = v;
+    if (found && hw != 0xFFFFFFFFu) {
+      hpos = spos[hw & 0xFFFFu] + 1;
+      hv = window(static_cast<int>(hw & 0xFFFFu), hpos);
+    }
+    uint32_t old = 0;
+    if (found && lane == src) {
+      spos[m] = static_cast<uint16_t>(at + f);
+      old = atom_min_relaxed_shared(sbid + (fe >> 16), (fe << 16) | static_cast<uint32_t>(m));
+    }
+    old = __shfl_sync(kFullMask, old, src);
+    if (found && (old >> 16) <= rk) lost++;  // someone better got there first: read the bids again
+    if (found && (old >> 16) > rk) {
+      hops++;
+      has = old != 0xFFFFFFFFu;  // else the chain ended at a free woman
+      m = static_cast<int>(old & 0xFFFFu);
+      if (old == hw) {
+        pos = hpos;
+        v = hv;
+      } else if (has) {
+        pos = spos[m] + 1;
+        fresh = true;
+      }
+    }
+  }
+  return gl == 0 ? RoundCount{hops, lost} : RoundCount{0, 0};
+}
+
+// One step.  kTable: the steps past the first ceil(n / batch), by which all men
+// may have started, if the table fits.  The others work their chains by warp
+// or by eight lanes, as the step before found the men calm or crowded.  Where
+// many make for the same women, four times the chains at a time triple the
+// displacements (RANDOM(5) n = 15013: 101 to 308 thousand, 4.0 to 6.4 ms) and
+// a quarter of the proposals come too late; in correlated lists one in 200
+// does by warp and one in 50 by eight lanes.
+constexpr unsigned int kCalmWarp = 64;   // fewer than one in so many late
+constexpr unsigned int kCalmGroup = 16;
+template <bool kTable>
+__global__ void __launch_bounds__(kRoundBlock, 1)
+    k_round(const int32_t *__restrict__ pref_m, const uint16_t *__restrict__ rankT, size_t ld,
+            const int32_t *__restrict__ order, RoundBufs b, int32_t *__restrict__ match, int n, int batch, int t,
+            Control *ctrl, int gate) {
+  __shared__ int s_go;
+  __shared__ int s_next, s_parked, s_stop;
+  __shared__ unsigned long long s_props;
+  __shared__ unsigned int s_hops, s_lost;
+  const int tid = threadIdx.x;
+  if (tid == 0) s_go = gate_open(gate, ctrl) && !ld_volatile_s32(&b.ctl->done);
+  __syncthreads();  // read once: another CTA may report an error meanwhile
+  if (!s_go) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const RoundSlot slot = b.ctl->slot[t & 1];
+  const int32_t *parkq = b.parkq[t & 1];
+  const int ready = slot.parked + (slot.new1 - slot.new0);
+  const int items = slot.refresh ? n : ready;
+  if (static_cast<int>(blockIdx.x) * kTeams < items)
+    round_scan(pref_m, rankT, ld, order, b, slot, parkq, items, n, smem_raw, ctrl);
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_go = atomicAdd(&b.ctl->arrived[t & 1], 1) == static_cast<int>(gridDim.x) - 1;
+    s_next = 0;
+    s_parked = 0;
+    s_stop = 0;
+    s_props = 0;
+    s_hops = 0;
+    s_lost = 0;
+  }
+  __syncthreads();
+  if (!s_go) {
+    round_check(pref_m, order, slot.new0, slot.new1, &b.ctl->checked[t & 1], n, ctrl);
+    return;
+  }
+  __threadfence();  // the other CTAs' lists
+  // ---- the last CTA resolves ----
+  const int nw = static_cast<int>(round_words(n));
+  uint32_t *sbid = reinterpret_cast<uint32_t *>(smem_raw);
+  uint16_t *spos = reinterpret_cast<uint16_t *>(smem_raw + static_cast<size_t>(nw) * 4);
+  uint32_t *snext = reinterpret_cast<uint32_t *>(smem_raw + static_cast<size_t>(nw) * 6);  // kTable
+  int32_t *park = b.parkq[(t & 1) ^ 1];
+  round_state_in(b, sbid, spos, nw);
+  __syncthreads();
+  const RoundChains q = {order,   parkq,     b,       slot,  sbid, spos,
+                         snext,   park,      &s_next, &s_parked, &s_stop, ready, n, ctrl};
+  const bool calm = !kTable && b.ctl->calm > 0;
+  const RoundCount count = kTable ? chains_by_warp<true>(q) : calm ? chains_by_group(q) : chains_by_warp<false>(q);
+  if (count.hops) atomicAdd(&s_hops, count.hops);
+  if (count.lost) atomicAdd(&s_lost, count.lost);
   __syncthreads();
   if (tid == 0 && ld_volatile_s32(&ctrl->status)) s_stop = 1;  // read once
   __syncthreads();
@@ -658,6 +816,11 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     b.ctl->checked[(t & 1) ^ 1] = 0;
     b.ctl->steps = t + 1;
     b.ctl->refreshes += nx.refresh;
+    const bool few = s_lost * (calm ? kCalmGroup : kCalmWarp) < s_hops;
+    if (few && b.ctl->calm == 0)
+      b.ctl->calm = 1;
+    else if (!few && calm)
+      b.ctl->calm = -1;  // for good
     b.ctl->done = done;
     ctrl->round_done = done;
     ctrl->bulk_hops += s_hops;

@@ -76,3 +76,17 @@ def test_rounds_at_the_table_limit(n):
         match, st = c.solve(pm, pw)
         again, st2 = c.solve(pm, pw, check=True)
         assert bool((match == again).all()) and st["proposals"] == st2["proposals"] and st2["blocking_pairs"] == 0
+
+
+@pytest.mark.parametrize("kind,n,param", [
+    (pb.SMP_GEN_UNIFORM, 3001, 0), (pb.SMP_GEN_CORRELATED, 5003, 1000), (pb.SMP_GEN_CORRELATED, 4100, 3000),
+    (pb.SMP_GEN_GROUPED, 3301, 400), (pb.SMP_GEN_SOLO, 1777, 0),
+])
+def test_rounds_by_eight_lanes(kind, n, param):
+    # steps after the first work their chains by eight lanes where few proposals come too late
+    pm, pw = lists(kind, n, param)
+    want, props = oracle.gs_seq(pm, pw)
+    with pb.Context(mode=1) as c:
+        for check in (False, True):
+            match, st = c.solve(pm, pw, check=check)
+            assert np.array_equal(match, want) and st["proposals"] == props
