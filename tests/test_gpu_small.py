@@ -67,3 +67,26 @@ def test_match_where_no_kernel_may_write(n):
         out = torch.full((n,), -1, dtype=torch.int32).pin_memory()
         match, _ = c.solve(pm, pw, out=out)
         assert bool((match == want.cpu()).all())
+
+
+@pytest.mark.parametrize("n", [257, 767, 768, 4097])
+def test_perfect_without_the_tail(n):
+    # every man a first choice of his own; then two who share one
+    import torch
+
+    def device(*lists):
+        return [torch.from_numpy(x).cuda() for x in lists]
+
+    rng = np.random.default_rng(n)
+    pm = np.stack([rng.permutation(n) for _ in range(n)]).astype(np.int32)
+    pw = np.stack([rng.permutation(n) for _ in range(n)]).astype(np.int32)
+    for m, w in enumerate(rng.permutation(n)):
+        k = int(np.nonzero(pm[m] == w)[0][0])
+        pm[m, [0, k]] = pm[m, [k, 0]]
+    with pb.Context() as c:
+        match, st = c.solve(*device(pm, pw))
+        assert np.array_equal(match.cpu().numpy(), pm[:, 0]) and st["proposals"] == n
+        pm[0] = pm[1]
+        want, props = oracle.gs_seq(pm, pw)
+        match, st = c.solve(*device(pm, pw))
+        assert np.array_equal(match.cpu().numpy(), want) and st["proposals"] == props
