@@ -297,7 +297,8 @@ struct Ctx {
   DeviceBuf gen_keys_a, gen_keys_b, gen_seg, gen_temp, gen_aux;
   Control *h_ctrl = nullptr;  // pinned host copy of the control block
   int32_t *h_verdict = nullptr;  // pinned, behind it: the precheck's verdict
-  bool await_verdict = false;    // the caller waits for it (synchronous solves)
+  bool synchronous = false;      // the caller waits for it, and for every pass
+  bool check_after = false;      // and runs the checker after the last one
   cudaEvent_t ev[10] = {};
   // Host-pointer solves: pref_w arrives on copy_stream in kCopyChunks row
   // chunks, each signalled by its event (created on first use).

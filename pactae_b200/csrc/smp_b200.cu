@@ -141,10 +141,10 @@ int enqueue_precheck(Ctx &c, bool allow_perfect) {
   // zeroed on the device, never copied from the host block (k_precheck)
   if (cudaMemsetAsync(c.d_ctrl.ptr, 0, zero_bytes(n), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
-  if (c.await_verdict) *static_cast<volatile int32_t *>(c.h_verdict) = kVerdictNone;
+  if (c.synchronous) *static_cast<volatile int32_t *>(c.h_verdict) = kVerdictNone;
   k_precheck<<<grid, 256, 0, c.stream>>>(c.pref_m, n, seen_of(c), c.d_bid.as<unsigned long long>(),
                                          c.d_ctrl.as<Control>(), allow_perfect ? 1 : 0, c.query_ok ? 1 : 0,
-                                         c.await_verdict ? c.h_verdict : nullptr);
+                                         c.synchronous ? c.h_verdict : nullptr);
   c.qcnt_clean = c.bid_clean = true;
   c.launches++;
   return c.check_launch("k_precheck");
@@ -629,7 +629,7 @@ constexpr int kTailMinN = 768;
 // 0.131 ms on the device with eleven of them, 0.053 without).  Bounded: without a verdict the tail is
 // enqueued and gated on the device, as it is where nobody waits.
 int32_t precheck_verdict(const Ctx &c) {
-  if (!c.await_verdict || c.pass != kPassQuery) return kVerdictNone;
+  if (!c.synchronous || c.pass != kPassQuery) return kVerdictNone;
   const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
   const volatile int32_t *verdict = c.h_verdict;
   while (*verdict == kVerdictNone && std::chrono::steady_clock::now() < until) {
@@ -1021,9 +1021,12 @@ int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t 
 // over the gate: 14 of them took about 0.1 ms of a 2.6 ms uniform solve at
 // n = 30000, where a wait for the precheck costs about 30 us.  The kernels
 // keep their gates, so the device still decides what runs.
-//   The checker (SMP_F_CHECK) must see the final matching; it, a disabled tail
-// and a configured tail window (whose tail kernel serves either mode) take
-// the fully gated pipeline, in one pass.
+//   The checker (SMP_F_CHECK) must see the final matching: a synchronous solve
+// runs it after its passes, the others enqueue it behind the fully gated
+// pipeline, in one pass.  So do a disabled tail and a configured tail window
+// (whose tail kernel serves either mode), and int32 ranks with the checker,
+// which reads them.  (Checked solves in the gated pipeline: uniform n = 1500
+// 0.49 ms for 0.28 in passes, congested n = 6000 3.1 for 0.52.)
 
 namespace {
 
@@ -1175,7 +1178,9 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
   }
   c.pass_flags = flags;
   c.pass_match = match_out;
-  if ((flags & SMP_F_CHECK) || !(c.tail_threshold > 0) || c.tail_window_cfg > 0) {
+  c.check_after = (flags & SMP_F_CHECK) && c.synchronous && n <= kU16MaxN;
+  if (((flags & SMP_F_CHECK) && !c.check_after) || !(c.tail_threshold > 0) || c.tail_window_cfg > 0) {
+    c.check_after = false;
     c.pass = kPassLast;
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }
@@ -1233,18 +1238,28 @@ int solve_advance(Ctx &c, bool &more) {
     return enqueue_swap_screen(c, false);
   }
   c.pass = kPassLast;
-  return enqueue_pass_mode(c, h.perfect ? -1 : h.mode);
+  if (!h.perfect) return enqueue_pass_mode(c, h.mode);
+  c.tail_ran = false;  // k_match writes the first choices
+  if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
+  return enqueue_pass_end(c);
 }
 
 // The synchronous solve.
 int solve_staged(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, int32_t *match_out,
                  uint32_t flags, smp_stats *st) {
-  c.await_verdict = true;
+  c.synchronous = true;
   int rc = solve_begin(c, pref_m, pref_w, n, match_out, flags);
-  c.await_verdict = false;
+  c.synchronous = false;
   for (bool more = true; !rc && more;) {
     rc = c.sync("solve");
     if (!rc) rc = solve_advance(c, more);
+  }
+  if (!rc && c.check_after) {  // the matching is final now
+    if (cudaEventRecord(c.ev[kEvCheckBegin], c.stream) != cudaSuccess) return c.fail_cuda("event");
+    if (!c.h_ctrl->status) rc = enqueue_check(c, match_here(c));
+    if (!rc && cudaEventRecord(c.ev[kEvCheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+    if (!rc) rc = read_control(c);
+    if (!rc) rc = c.sync("check");
   }
   return rc ? rc : solve_finish(c, flags, st);
 }
@@ -1662,9 +1677,11 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
     if (!rc && !swapped && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess)
       rc = c.fail_cuda("event");
     if (!rc && shared && !swapped) rc = solve_swapped(c, flags, match_out, swapped);
-    if (!rc && !swapped) rc = enqueue_init(c);
+    const bool perfect = c.h_ctrl->perfect != 0;
+    if (perfect) c.tail_ran = false;  // k_match writes the first choices
+    if (!rc && !swapped && !perfect) rc = enqueue_init(c);
     if (!rc && !swapped && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-    if (!rc && !swapped) rc = enqueue_core(c);
+    if (!rc && !swapped && !perfect) rc = enqueue_core(c);
   } else {
     if (cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
     rc = init_buffers(c);

@@ -90,3 +90,29 @@ def test_rounds_by_eight_lanes(kind, n, param):
         for check in (False, True):
             match, st = c.solve(pm, pw, check=check)
             assert np.array_equal(match, want) and st["proposals"] == props
+
+
+@pytest.mark.parametrize("kind,n,param", [
+    ("worst", 5000, 0), (pb.SMP_GEN_SOLO, 1777, 0), (pb.SMP_GEN_CORRELATED, 3001, 500), (pb.SMP_GEN_UNIFORM, 3001, 0),
+    (pb.SMP_GEN_UNIFORM, 9001, 0), (pb.SMP_GEN_PERFECT, 900, 0),
+])
+def test_fixed_sequences(kind, n, param):
+    # phase by phase nothing is read back in the middle of one: a fixed number of
+    # steps and a last one, or of the tail's segments and one without a limit
+    if kind == "worst":
+        pm = np.tile(np.arange(n, dtype=np.int32), (n, 1))
+        pm[n // 2, [n - 2, n - 1]] = pm[n // 2, [n - 1, n - 2]]
+        pw = np.tile(np.arange(n, dtype=np.int32)[::-1], (n, 1))
+        for i in range(64):
+            pw[i * n // 64] = np.arange(n, dtype=np.int32)
+    else:
+        pm, pw = lists(kind, n, param)
+    want, props = oracle.gs_seq(pm, pw)
+    with pb.Context() as c:
+        c.stage(pm, pw, n)
+        if not c.precheck():
+            c.init()
+            c.core()
+        assert np.array_equal(c.post(), want)
+        match, st = c.solve(pm, pw, check=True)  # the checker after the passes
+        assert np.array_equal(match, want) and st["proposals"] == props and st["blocking_pairs"] == 0
