@@ -1886,6 +1886,8 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
   c.phase = 1;
   c.stats.precheck_ms = elapsed(c, kEvStageEnd, kEvPrecheckEnd);
   if (is_perfect) *is_perfect = c.h_ctrl->perfect;
+  // init and core enqueue this mode's kernels only
+  c.known_mode = in_rounds(c) && !c.h_ctrl->status && !c.h_ctrl->perfect ? c.h_ctrl->mode : -1;
   return control_status(c);
 }
 
@@ -1910,11 +1912,27 @@ int smp_b200_core(smp_ctx *ctx) {
   Ctx &c = ctx->c;
   DeviceGuard g(c.device);
   if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
+  const bool query = c.known_mode == kModeQuery;
+  c.poll_tail = c.poll_rounds = c.known_mode >= 0;
   int rc = enqueue_core(c);
-  if (rc) return rc;
-  if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  rc = read_control(c);
-  if (!rc) rc = c.sync("core");
+  for (bool more = true; !rc && more;) {
+    if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
+    rc = read_control(c);
+    if (!rc) rc = c.sync("core");
+    if (rc) break;
+    more = c.poll_tail && !c.h_ctrl->status;
+    if (!more) break;
+    if (!tail_over(c)) {
+      rc = enqueue_tail(c, true);
+    } else if (rounds_left(c)) {
+      rc = enqueue_round_steps(c, c.round_gate, kRoundMore);
+    } else if (query && c.known_mode == kModeQuery && c.h_ctrl->retry) {
+      c.known_mode = -1;  // the rank-mode retry of a query-mode round 0
+      rc = enqueue_retry_round<uint16_t>(c);
+    } else {
+      more = false;
+    }
+  }
   if (rc) return rc;
   c.phase = 3;
   c.stats.core_ms = elapsed(c, kEvInitEnd, kEvCoreEnd);
