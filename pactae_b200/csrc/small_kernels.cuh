@@ -106,9 +106,9 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
         list[t] = static_cast<uint16_t>((w << 8) | rank[w * n + m]);
     }
     if (differ) s_differ = 1;
-    __syncthreads();
-    // the chains: a warp each, 32 choices at a time
-    if (!s_status) {
+    // the chains: a warp each, 32 choices at a time (all warps or none: one that
+    // refuses a man in there must not keep lanes of a later one out)
+    if (!__syncthreads_or(s_status != 0)) {
       unsigned int hops = 0;
       int m = -1, pos = 0;
       for (;;) {
