@@ -840,6 +840,14 @@ int enqueue_check(Ctx &c, const int32_t *match) {
   return c.check_launch("k_check");
 }
 
+// What the last solve or phase sequence on the context left of its rounds and
+// segments: the next one starts without.
+void reset_progress(Ctx &c) {
+  c.poll_rounds = c.poll_tail = false;
+  c.round_step = c.tail_segment = 0;
+  c.swapped = false;
+}
+
 // Per-solve state reset and plan for size n.
 int stage_reset(Ctx &c, int32_t n) {
   c.n = n;
@@ -853,9 +861,7 @@ int stage_reset(Ctx &c, int32_t n) {
   c.qcnt_clean = c.bid_clean = false;
   c.known_mode = -1;
   c.pass = kPassLast;
-  c.poll_rounds = c.poll_tail = false;
-  c.round_step = c.tail_segment = 0;
-  c.swapped = false;
+  reset_progress(c);
   plan(c);
   return SMP_OK;
 }
@@ -1876,6 +1882,7 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
   if (!valid_ctx(ctx) || !ctx->c.staged) return SMP_ERR_INVALID_ARG;
   Ctx &c = ctx->c;
   DeviceGuard g(c.device);
+  reset_progress(c);
   if (cudaEventRecord(c.ev[kEvStageEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   int rc = enqueue_precheck(c, true);
   if (!rc) rc = read_control(c);
@@ -1914,6 +1921,7 @@ int smp_b200_core(smp_ctx *ctx) {
   if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   const bool query = c.known_mode == kModeQuery;
   c.poll_tail = c.poll_rounds = c.known_mode >= 0;
+  c.round_step = c.tail_segment = 0;  // this call waits for what it enqueues itself
   int rc = enqueue_core(c);
   for (bool more = true; !rc && more;) {
     if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");

@@ -1,0 +1,46 @@
+"""The phase calls on a context that has already done something: the whole
+sequence again on one staging, and after a solve on the same context."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+import pactae_b200 as pb
+from pactae_b200._lib import lib
+
+pytestmark = pytest.mark.gpu
+
+
+def phases(c, n):
+    """precheck .. post of what the context holds; the matching on the host."""
+    perfect = ctypes.c_int32()
+    assert lib.smp_b200_precheck(c.handle, ctypes.byref(perfect)) == pb.SMP_OK
+    if not perfect.value:
+        assert lib.smp_b200_init(c.handle) == pb.SMP_OK
+        assert lib.smp_b200_core(c.handle) == pb.SMP_OK
+    return post(c, n)
+
+
+def post(c, n):
+    match = np.full(n, -1, dtype=np.int32)
+    assert lib.smp_b200_post(c.handle, ctypes.c_void_p(match.ctypes.data), 0) == pb.SMP_OK
+    return match
+
+
+# with a prefix too short for the query mode (the rank-mode retry), in the query
+# mode to its end, in the rank mode, and with distinct first choices
+@pytest.mark.parametrize("kind,n,param,prefix_k", [
+    (pb.SMP_GEN_UNIFORM, 1500, 0, 6), (pb.SMP_GEN_UNIFORM, 400, 0, 6), (pb.SMP_GEN_UNIFORM, 1500, 0, 0),
+    (pb.SMP_GEN_CORRELATED, 1300, 500, 0), (pb.SMP_GEN_CONGESTED, 600, 0, 0), (pb.SMP_GEN_PERFECT, 700, 0, 0),
+])
+def test_phases_again_on_one_staging(kind, n, param, prefix_k):
+    pm, pw = oracle.generate(kind, n, 8, 0, param)
+    want, props = oracle.gs_seq(pm, pw)
+    with pb.Context(prefix_k=prefix_k) as c:
+        engine = pb.SmpEngineB200(pb.SmpObj(pm, pw), n, c)
+        for _ in range(3):
+            assert np.array_equal(engine.FindStableMatching(), want)
+            assert c.stats()["proposals"] == props
