@@ -23,7 +23,7 @@
 // she holds).  Where she has changed the list is read.  Lists age as women
 // change, so a thread that has read enough of them ends the segment: all
 // chains are parked and the lists made anew (one more pair of launches).
-//   The last few chains are followed by one warp, one after the other: with
+//   The last few chains are followed by one thread, one after the other: with
 // nobody else writing, a proposal is a plain store, and steps go four to a
 // branch, each predicated on the one before.
 //   k_tail_out writes the matching and finds the positions.
@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(kTailListBlock) k_tail_lists(const uint32_t *_
   }
 }
 
-// Why the chains stop: few are left (one warp goes on with them), the lists
+// Why the chains stop: few are left (one thread goes on with them), the lists
 // are too old (the segment ends), the solve cannot go on here.
 constexpr int kTailFew = 1, kTailOld = 2, kTailOver = 3;
-// Chains that one warp follows one after the other.  With the lists in L2 a
+// Chains that one thread follows one after the other.  With the lists in L2 a
 // step costs it about 0.4 of what it costs threads that must propose
 // atomically; with exact lists the two differ little, and only the last one
 // gains.
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ 
   } else {
 #pragma unroll 4
     for (int i = tid; i < np / 4; i += 1024)
-      reinterpret_cast<uint4 *>(sbid)[i] = __ldg(reinterpret_cast<const uint4 *>(b.word) + i);
+      reinterpret_cast<uint4 *>(sbid)[i] = __ldcg(reinterpret_cast<const uint4 *>(b.word) + i);  // (written below)
   }
   if (kExact) {
     constexpr int kGroups = kExact ? E / 4 : 1;
@@ -367,17 +367,15 @@ __global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ 
   const int why = s_stop;
   __syncthreads();
   if (why == kTailOver) return;
-  if (why == kTailFew && tid < 32) {
-    // the parked men and those nobody took up, one after the other; every lane
-    // of the warp does the same
+  if (why == kTailFew && tid == 0) {
+    // the parked men and those nobody took up, one after the other
     const int few = s_parked;
     const int taken = min(s_next, total);
     const int count = few + (total - taken);
     int over = 0, kept = 0;
-    slow = 0;  // the same in every lane (lane 0 has counted before)
-    __syncwarp();
+    slow = 0;
     for (int i = 0; i < count; ++i) {
-      int m = i < few ? __ldcg(parked + i) : waiting[taken + i - few];
+      int m = i < few ? parked[i] : waiting[taken + i - few];
       for (bool on = !over; on;) {
         uint32_t e, seen = 0;
         if constexpr (kExact) {
@@ -411,7 +409,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ 
           e = w < static_cast<uint32_t>(np) ? search(m, 0, seen) : kTailNone;
         }
         if (e == kTailNone) {
-          if (tid == 0) nobody(m);
+          nobody(m);
           over = 1;
           break;
         }
@@ -423,24 +421,15 @@ __global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ 
           // the lists are too old; the men left go to the front of the next
           // segment's list
           on = false;
-          if (tid == 0) parked[kept] = m;
-          kept++;
-          for (int j = i + 1; j < count; ++j, ++kept) {
-            const int other = j < few ? __ldcg(parked + j) : waiting[taken + j - few];
-            __syncwarp();
-            if (tid == 0) parked[kept] = other;
-            __syncwarp();
-          }
+          parked[kept++] = m;  // (entry i or before: read already)
+          for (int j = i + 1; j < count; ++j) parked[kept++] = j < few ? parked[j] : waiting[taken + j - few];
           i = count;
         }
       }
     }
-    if (tid == 0) {
-      s_parked = kept;
-      s_next = total;
-      if (over) s_stop = kTailOver;
-    }
-    if (tid != 0) hops = 0;
+    s_parked = kept;
+    s_next = total;
+    if (over) s_stop = kTailOver;
   }
   if ((tid & 31) == 0 && hops) atomicAdd(&s_hops, hops);
   __syncthreads();
