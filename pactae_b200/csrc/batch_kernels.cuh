@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(1024, 1) k_batch(BatchInstance *__restrict__ t
         // women propose down their lists; every man ranks a woman by her
         // place in the shared list
         const SharedBids bids{sbid, spos};
-        const auto keep_going = [&]() { return *reinterpret_cast<volatile int *>(&s_status) == 0; };
+        const auto keep_going = [&]() { return !warp_flag(&s_status); };
         int m = -1, pos = 0, S = 1, bad_value = 0;
         Ahead ahead;
         unsigned long long settled = 0;
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(1024, 1) k_batch(BatchInstance *__restrict__ t
                    rank_smem_elems / 2, n, &s_next_man, &s_status);
     } else {
       const SharedBids bids{sbid, spos};
-      const auto keep_going = [&]() { return *reinterpret_cast<volatile int *>(&s_status) == 0; };
+      const auto keep_going = [&]() { return !warp_flag(&s_status); };
       int m = -1, pos = 0, S = 1, bad_value = 0;
       Ahead ahead;
       unsigned long long settled = 0;

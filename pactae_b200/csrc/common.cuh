@@ -113,6 +113,13 @@ __device__ __forceinline__ int ld_volatile_s32(const int *p) {
   return *reinterpret_cast<const volatile int *>(p);
 }
 
+// A flag that another warp may set at any time, read for the whole warp:
+// lanes that each read it for themselves may see different values, and what
+// follows are votes of all of them.
+__device__ __forceinline__ bool warp_flag(const int *flag) {
+  return __any_sync(0xFFFFFFFFu, *reinterpret_cast<const volatile int *>(flag) != 0);
+}
+
 // Grid-strided L2 prefetch of [p, p + bytes), one request per 128-byte line.
 __device__ __forceinline__ void prefetch_l2(const void *p, size_t bytes) {
   const char *base = static_cast<const char *>(p);

@@ -524,9 +524,9 @@ __device__ __forceinline__ RoundCount chains_by_warp(const RoundChains &q) {
   };
   const auto next_man = [&]() {
     int i = 0;
-    if (lane == 0) i = atomicAdd(q.s_next, 1);
+    if (lane == 0) i = *reinterpret_cast<volatile int *>(q.s_stop) ? q.ready : atomicAdd(q.s_next, 1);
     i = __shfl_sync(kFullMask, i, 0);
-    if (i >= q.ready || *reinterpret_cast<volatile int *>(q.s_stop)) return false;
+    if (i >= q.ready) return false;
     m = i < q.slot.parked ? q.parkq[i] : __ldg(q.order + q.slot.new0 + (i - q.slot.parked));
     pos = 0;
     one = kNoCand;
@@ -656,10 +656,10 @@ __device__ __forceinline__ RoundCount chains_by_group(const RoundChains &q) {
     const bool ask = !has && !out;
     if (__any_sync(kFullMask, ask)) {
       int i = 0;
-      if (ask && gl == 0) i = atomicAdd(q.s_next, 1);
+      if (ask && gl == 0) i = *reinterpret_cast<volatile int *>(q.s_stop) ? q.ready : atomicAdd(q.s_next, 1);
       i = __shfl_sync(kFullMask, i, g0);
       if (ask) {
-        has = i < q.ready && !*reinterpret_cast<volatile int *>(q.s_stop);
+        has = i < q.ready;
         out = !has;
         fresh = has;
         if (has) m = i < q.slot.parked ? q.parkq[i] : __ldg(q.order + q.slot.new0 + (i - q.slot.parked));
@@ -886,7 +886,7 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     return true;
   };
   for (bool more = next_man(); more;) {
-    if (*reinterpret_cast<volatile int *>(&s_stop)) break;
+    if (warp_flag(&s_stop)) break;
     const int32_t *row = pref_m + static_cast<size_t>(m) * n;
     const uint16_t *rrow = rankT + static_cast<size_t>(m) * ld;
     bool taken = false;
@@ -909,6 +909,7 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
         }
         old = __shfl_sync(kFullMask, old, j);
         const uint32_t rkj = __shfl_sync(kFullMask, rk, j);
+        __syncwarp();  // the displaced man's position, as lane j would see it
         if ((old >> 16) > rkj) {
           hops++;
           taken = true;

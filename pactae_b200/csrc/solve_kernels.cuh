@@ -1131,7 +1131,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
   __syncthreads();
 
   const SharedBids bids{sbid, spos};
-  const auto keep_going = [&]() { return *reinterpret_cast<volatile int *>(&s_abort) == 0; };
+  const auto keep_going = [&]() { return !warp_flag(&s_abort); };
   int m = -1, pos = 0, S = 1, bad_value = 0;
   Ahead ahead;
   unsigned long long settled = 0;
@@ -1456,7 +1456,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail_qw(const int32_t *__restrict__
     return true;
   };
   for (bool more = next_man(); more;) {
-    const int aborted = *reinterpret_cast<volatile int *>(&s_abort);  // tested at the end of the step
+    const bool aborted = warp_flag(&s_abort);  // tested at the end of the step
     const int r = pos + lane;
     const bool ok = r < Kn && raw != 0xFFFFFFFFu;
     const int w = ok ? static_cast<int>(raw >> 16) : 0;
