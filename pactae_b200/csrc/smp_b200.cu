@@ -840,9 +840,12 @@ int enqueue_check(Ctx &c, const int32_t *match) {
   return c.check_launch("k_check");
 }
 
-// What the last solve or phase sequence on the context left of its rounds and
-// segments: the next one starts without.
+// What the last solve or phase sequence on the context left of its passes,
+// rounds and segments, and of its caller's array: the next one starts without.
 void reset_progress(Ctx &c) {
+  c.pass = kPassLast;
+  c.match_direct = false;
+  c.pass_match = nullptr;
   c.poll_rounds = c.poll_tail = false;
   c.round_step = c.tail_segment = 0;
   c.swapped = false;
@@ -860,7 +863,6 @@ int stage_reset(Ctx &c, int32_t n) {
   c.launches = 0;
   c.qcnt_clean = c.bid_clean = false;
   c.known_mode = -1;
-  c.pass = kPassLast;
   reset_progress(c);
   plan(c);
   return SMP_OK;
@@ -1182,15 +1184,14 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
     c.n = n;
     plan(c);
   }
-  c.pass_flags = flags;
-  c.pass_match = match_out;
   c.check_after = (flags & SMP_F_CHECK) && c.synchronous && n <= kU16MaxN;
   if (((flags & SMP_F_CHECK) && !c.check_after) || !(c.tail_threshold > 0) || c.tail_window_cfg > 0) {
     c.check_after = false;
-    c.pass = kPassLast;
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }
   int rc = do_stage(c, pref_m, pref_w, n, flags);
+  c.pass_flags = flags;
+  c.pass_match = match_out;
   c.match_direct = (flags & SMP_F_DEVICE_PTRS) && n > 0 && kernel_may_write(c, match_out, sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && solve_is_small(c, flags)) {
     c.pass = kPassSmall;
@@ -1293,6 +1294,8 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
 // Statistics and status of a solve whose stream has completed.
 int solve_finish(Ctx &c, uint32_t flags, smp_stats *st) {
   c.phase = 3;
+  c.match_direct = false;  // the caller's array is the caller's again
+  c.pass_match = nullptr;
   fill_stats(c, c.pass != kPassSmall);
   if (c.pass == kPassSmall) {  // one launch, all of it the core
     c.stats.stage_ms = elapsed(c, kEvStageBegin, kEvStageEnd);

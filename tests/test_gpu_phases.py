@@ -44,3 +44,15 @@ def test_phases_again_on_one_staging(kind, n, param, prefix_k):
         for _ in range(3):
             assert np.array_equal(engine.FindStableMatching(), want)
             assert c.stats()["proposals"] == props
+
+
+@pytest.mark.parametrize("n", [300, 900])
+def test_phases_after_a_device_solve_leave_its_match_alone(n):
+    # the array of a call that has returned is not written again
+    with pb.Context() as c:
+        pm, pw = c.generate(pb.SMP_GEN_UNIFORM, n, 6)
+        out, _ = c.solve(pm, pw)
+        want = out.cpu().numpy()
+        out.fill_(-1)
+        assert np.array_equal(phases(c, n), want)
+        assert bool((out == -1).all())
