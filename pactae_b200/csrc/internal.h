@@ -256,6 +256,9 @@ struct Ctx {
   bool tail_ran = false;
   bool swapped = false;  // the men share one list and the women proposed
   int phase = 0;            // 0 staged, 1 prechecked, 2 inited, 3 cored, 4 posted
+  // A solve or a core has used up the precheck's state: init and core after it
+  // start from the precheck again.
+  bool spent = false;
   // The mode the host has read back from the precheck (kModeQuery / kModeRank),
   // or -1: the enqueue functions then skip the kernels that mode would gate
   // off.  -1 (unknown) enqueues everything and the device picks.

@@ -33,7 +33,7 @@ __host__ __device__ constexpr size_t small_smem(int n) {
 
 __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ pref_m,
                                                    const int32_t *__restrict__ pref_w, int n, int K,
-                                                   int allow_perfect, int32_t *__restrict__ match, Control *out) {
+                                                   int allow_perfect, int32_t *match, int32_t *also, Control *out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const size_t n2 = static_cast<size_t>(n) * n;
   uint16_t *list = reinterpret_cast<uint16_t *>(smem_raw);
@@ -73,7 +73,10 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
   const bool perfect = allow_perfect && distinct == n && s_status == 0;
   const int mode = 4 * distinct >= n ? kModeQuery : kModeRank;
   if (perfect) {
-    if (tid < n) match[tid] = first;
+    if (tid < n) {
+      match[tid] = first;
+      if (also) also[tid] = first;
+    }
   } else {
     const int total = static_cast<int>(n2);
     for (int i = tid; i < n; i += 1024) word[i] = 0xFFFFFFFFu;
@@ -153,10 +156,12 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
     __syncthreads();
     if (!s_status && tid < n) {
       const uint32_t v = word[tid];
-      if (v == 0xFFFFFFFFu)
+      if (v == 0xFFFFFFFFu) {
         refuse(tid);
-      else
+      } else {
         match[v & 0xFFFFu] = tid;
+        if (also) also[v & 0xFFFFu] = tid;
+      }
       atomicAdd(&s_props, spos[tid] + 1ull);
       if (spos[tid] >= K) s_deep = 1;
     }

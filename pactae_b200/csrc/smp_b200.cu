@@ -565,6 +565,8 @@ bool writes_match_here(const Ctx &c) {
   return c.match_direct && (c.pass == kPassSmall || (c.pass == kPassQuery && in_rounds(c)));
 }
 int32_t *match_here(const Ctx &c) { return writes_match_here(c) ? c.pass_match : c.d_match.as<int32_t>(); }
+// The context keeps the matching as well (smp_b200_post after a solve).
+int32_t *match_also(const Ctx &c) { return writes_match_here(c) ? c.d_match.as<int32_t>() : nullptr; }
 
 // Segment after segment: the candidate lists on all SMs, then the chains in
 // one CTA with as many list entries per man in shared memory as fit.  Where
@@ -599,11 +601,11 @@ int enqueue_tail_segments(Ctx &c, int count, bool unlimited) {
     else
       k_tail_lists<false><<<grid, kTailListBlock, cut, c.stream>>>(prefix, c.K, bid, c.d_tailq.as<int2>(), b, c.n, ctrl);
     k_tail_q<E><<<1, 1024, tail_q_smem(c.n, E), c.stream>>>(
-        c.pref_m, prefix, c.K, bid, ctrl, b, match_here(c), c.n, s,
+        c.pref_m, prefix, c.K, bid, ctrl, b, match_here(c), match_also(c), c.n, s,
         unlimited && i + 1 == count ? 0 : E > 0 ? kTailSlowExact : kTailSlow);
   }
   k_tail_out<<<std::max(1, std::min(c.sm_count * 8, (c.n + 7) / 8)), 256, 0, c.stream>>>(prefix, c.K, b, match_here(c),
-                                                                                        c.n, ctrl);
+                                                                                        match_also(c), c.n, ctrl);
   c.tail_segment += count;
   c.launches += 2 * count + 1;
   return c.check_launch("k_tail_q");
@@ -642,7 +644,7 @@ int launch_tail_query(Ctx &c) {
   if (verdict == kVerdictOther) return SMP_OK;
   if (verdict == kVerdictPerfect) {
     k_match<<<std::max(1, std::min(c.sm_count * 4, (c.n + 255) / 256)), 256, 0, c.stream>>>(
-        c.pref_m, c.d_bid.as<unsigned long long>(), match_here(c), c.n, c.d_ctrl.as<Control>());
+        c.pref_m, c.d_bid.as<unsigned long long>(), match_here(c), match_also(c), c.n, c.d_ctrl.as<Control>());
     c.launches++;
     return c.check_launch("k_match");
   }
@@ -650,7 +652,7 @@ int launch_tail_query(Ctx &c) {
     if (allow_dynamic_smem(c, k_tail_qw) != cudaSuccess) return c.fail_cuda("k_tail_qw smem attribute");
     k_tail_qw<<<1, 1024, tail_smem_bytes(c.n), c.stream>>>(c.pref_m, c.d_prefix.as<uint32_t>(), c.K,
                                                            c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(),
-                                                           c.d_tailq.as<int2>(), match_here(c), c.n);
+                                                           c.d_tailq.as<int2>(), match_here(c), match_also(c), c.n);
     c.launches++;
     return c.check_launch("k_tail_qw");
   }
@@ -753,7 +755,7 @@ int enqueue_post(Ctx &c) {
   int rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(n));
   if (rc) return rc;
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
-  k_match<<<grid, 256, 0, c.stream>>>(c.pref_m, c.d_bid.as<unsigned long long>(), c.d_match.as<int32_t>(), n,
+  k_match<<<grid, 256, 0, c.stream>>>(c.pref_m, c.d_bid.as<unsigned long long>(), c.d_match.as<int32_t>(), nullptr, n,
                                       c.d_ctrl.as<Control>());
   c.launches++;
   return c.check_launch("k_match");
@@ -856,6 +858,7 @@ int stage_reset(Ctx &c, int32_t n) {
   c.n = n;
   c.staged = false;
   c.rank_valid = false;
+  c.spent = false;
   c.phase = 0;
   c.stats = smp_stats{};
   c.stats.n = n;
@@ -1160,15 +1163,13 @@ bool solve_is_small(const Ctx &c, uint32_t flags) {
 
 int enqueue_small(Ctx &c, int32_t *match_out, uint32_t flags) {
   const bool device = (flags & SMP_F_DEVICE_PTRS) != 0;
-  if (!writes_match_here(c)) {
-    const int rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
-    if (rc) return rc;
-  }
+  int rc = c.d_match.ensure(sizeof(int32_t) * static_cast<size_t>(c.n));
+  if (rc) return rc;
   if (allow_dynamic_smem(c, k_small) != cudaSuccess) return c.fail_cuda("k_small smem attribute");
   k_small<<<1, 1024, small_smem(c.n), c.stream>>>(c.pref_m, c.pref_w, c.n, c.K, (flags & SMP_F_NO_PRECHECK) == 0,
-                                                  match_here(c), c.h_ctrl);
+                                                  match_here(c), match_also(c), c.h_ctrl);
   c.launches++;
-  int rc = c.check_launch("k_small");
+  rc = c.check_launch("k_small");
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   if (!rc && !writes_match_here(c)) rc = copy_match_out(c, match_out, device);
   return rc;
@@ -1294,6 +1295,7 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
 // Statistics and status of a solve whose stream has completed.
 int solve_finish(Ctx &c, uint32_t flags, smp_stats *st) {
   c.phase = 3;
+  c.spent = true;
   c.match_direct = false;  // the caller's array is the caller's again
   c.pass_match = nullptr;
   fill_stats(c, c.pass != kPassSmall);
@@ -1886,6 +1888,7 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
   Ctx &c = ctx->c;
   DeviceGuard g(c.device);
   reset_progress(c);
+  c.spent = false;
   if (cudaEventRecord(c.ev[kEvStageEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   int rc = enqueue_precheck(c, true);
   if (!rc) rc = read_control(c);
@@ -1904,6 +1907,10 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
 int smp_b200_init(smp_ctx *ctx) {
   if (!valid_ctx(ctx) || ctx->c.phase < 1) return SMP_ERR_INVALID_ARG;
   Ctx &c = ctx->c;
+  if (c.spent) {
+    const int rc = smp_b200_precheck(ctx, nullptr);
+    if (rc) return rc;
+  }
   DeviceGuard g(c.device);
   if (cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   int rc = enqueue_init(c);
@@ -1920,6 +1927,10 @@ int smp_b200_init(smp_ctx *ctx) {
 int smp_b200_core(smp_ctx *ctx) {
   if (!valid_ctx(ctx) || ctx->c.phase < 2) return SMP_ERR_INVALID_ARG;
   Ctx &c = ctx->c;
+  if (c.spent) {
+    const int rc = smp_b200_init(ctx);
+    if (rc) return rc;
+  }
   DeviceGuard g(c.device);
   if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   const bool query = c.known_mode == kModeQuery;
@@ -1944,6 +1955,7 @@ int smp_b200_core(smp_ctx *ctx) {
       more = false;
     }
   }
+  c.spent = true;
   if (rc) return rc;
   c.phase = 3;
   c.stats.core_ms = elapsed(c, kEvInitEnd, kEvCoreEnd);
@@ -1963,12 +1975,14 @@ int smp_b200_post(smp_ctx *ctx, int32_t *match_out, uint32_t flags) {
     if (!rc) rc = c.d_bid.ensure(sizeof(unsigned long long) * static_cast<size_t>(c.n));
     if (rc) return rc;
   }
+  // After a solve, or again: d_match holds the matching and h_ctrl the outcome.
+  const bool again = c.phase == 4;
   if (cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  int rc = enqueue_post(c);
+  int rc = again ? SMP_OK : enqueue_post(c);
   if (!rc) rc = copy_match_out(c, match_out, (flags & SMP_F_DEVICE_PTRS) != 0);
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  rc = read_control(c);
+  if (!again) rc = read_control(c);
   if (!rc) rc = c.sync("post");
   if (rc) return rc;
   c.stats.post_ms = elapsed(c, kEvCoreEnd, kEvPostEnd);

@@ -1052,7 +1052,8 @@ __device__ __forceinline__ void coop_load(const unsigned long long *bid, uint32_
 // match[] and the proposal count (sum of final positions + 1) from the
 // shared state, after every chain has ended.  Called by the whole CTA.
 __device__ __forceinline__ void tail_finish(const uint32_t *sbid, const uint16_t *spos, int32_t *__restrict__ match,
-                                            int n, Control *ctrl, unsigned long long *s_props) {
+                                            int n, Control *ctrl, unsigned long long *s_props,
+                                            int32_t *also = nullptr) {
   unsigned long long props = 0;
   for (int w = threadIdx.x; w < n; w += blockDim.x) {
     const uint32_t b = sbid[w];
@@ -1061,6 +1062,7 @@ __device__ __forceinline__ void tail_finish(const uint32_t *sbid, const uint16_t
       continue;
     }
     match[b & 0xFFFFu] = w;
+    if (also) also[b & 0xFFFFu] = w;
   }
   for (int mm = threadIdx.x; mm < n; mm += blockDim.x) props += spos[mm] + 1ull;
 #pragma unroll
@@ -1070,11 +1072,16 @@ __device__ __forceinline__ void tail_finish(const uint32_t *sbid, const uint16_t
   if (threadIdx.x == 0) ctrl->proposals = *s_props;
 }
 
+// also: the context's copy, where match is the caller's array (nullptr: match
+// is the context's).
 __device__ __forceinline__ void write_perfect(const int32_t *__restrict__ pref_m, int32_t *match, int n,
-                                              Control *ctrl) {
+                                              Control *ctrl, int32_t *also = nullptr) {
   const int stride = gridDim.x * blockDim.x;
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += stride)
-    match[m] = __ldg(pref_m + static_cast<size_t>(m) * n);
+  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += stride) {
+    const int w = __ldg(pref_m + static_cast<size_t>(m) * n);
+    match[m] = w;
+    if (also) also[m] = w;
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->proposals = static_cast<unsigned long long>(n);
 }
 
@@ -1403,10 +1410,10 @@ __global__ void __launch_bounds__(1024, 1) k_tail_qw(const int32_t *__restrict__
                                                     const uint32_t *__restrict__ prefix, int K,
                                                     const unsigned long long *__restrict__ bid, Control *ctrl,
                                                     const int2 *__restrict__ tail_queue,
-                                                    int32_t *__restrict__ match, int n) {
+                                                    int32_t *match, int32_t *also, int n) {
   if (ld_volatile_s32(&ctrl->mode) != kModeQuery) return;
   if (ld_volatile_s32(&ctrl->perfect)) {
-    write_perfect(pref_m, match, n, ctrl);
+    write_perfect(pref_m, match, n, ctrl, also);
     return;
   }
   if (!gate_open(kGateMain, ctrl)) return;
@@ -1541,7 +1548,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail_qw(const int32_t *__restrict__
   }
   __syncthreads();
   if (s_abort || ld_volatile_s32(&ctrl->status)) return;
-  tail_finish(sbid, spos, match, n, ctrl, &s_props);
+  tail_finish(sbid, spos, match, n, ctrl, &s_props, also);
 }
 
 // ---------------------------------------------------------------------------
@@ -1570,9 +1577,9 @@ __global__ void k_retry_reset(unsigned long long *bid, int n, Control *ctrl) {
 // Matching from the global bid words (used when no tail kernel runs).
 // ---------------------------------------------------------------------------
 __global__ void k_match(const int32_t *__restrict__ pref_m, const unsigned long long *__restrict__ bid,
-                        int32_t *__restrict__ match, int n, Control *ctrl) {
+                        int32_t *match, int32_t *also, int n, Control *ctrl) {
   if (ld_volatile_s32(&ctrl->perfect)) {
-    write_perfect(pref_m, match, n, ctrl);
+    write_perfect(pref_m, match, n, ctrl, also);
     return;
   }
   if (ld_volatile_s32(&ctrl->status)) return;
@@ -1585,6 +1592,7 @@ __global__ void k_match(const int32_t *__restrict__ pref_m, const unsigned long 
       continue;
     }
     match[bid_man(b)] = w;
+    if (also) also[bid_man(b)] = w;
     props += bid_pos(b) + 1ull;
   }
 #pragma unroll

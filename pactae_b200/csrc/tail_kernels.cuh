@@ -178,12 +178,12 @@ template <int E>
 __global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ pref_m,
                                                     const uint32_t *__restrict__ prefix, int K,
                                                     const unsigned long long *__restrict__ bid, Control *ctrl,
-                                                    TailBufs b, int32_t *__restrict__ match, int n, int segment,
+                                                    TailBufs b, int32_t *match, int32_t *also, int n, int segment,
                                                     int slow_limit) {
   constexpr bool kExact = E > 0;
   constexpr int kAlone = tail_alone(kExact);
   if (segment == 0 && ld_volatile_s32(&ctrl->mode) == kModeQuery && ld_volatile_s32(&ctrl->perfect)) {
-    write_perfect(pref_m, match, n, ctrl);
+    write_perfect(pref_m, match, n, ctrl, also);
     return;
   }
   if (!tail_open(ctrl)) return;
@@ -456,10 +456,10 @@ __global__ void __launch_bounds__(1024, 1) k_tail_q(const int32_t *__restrict__ 
   }
 }
 
-// match[] and the proposal count: a man's position is where the woman he
+// match[] (and also[], see write_perfect) and the proposal count: a man's position is where the woman he
 // ended with stands in his prefix, at or after the entry before `from`.
 __global__ void __launch_bounds__(256) k_tail_out(const uint32_t *__restrict__ prefix, int K, TailBufs b,
-                                                  int32_t *__restrict__ match, int n, Control *ctrl) {
+                                                  int32_t *match, int32_t *also, int n, Control *ctrl) {
   if (ld_volatile_s32(&ctrl->mode) != kModeQuery || !gate_open(kGateMain, ctrl) || !ld_volatile_s32(&ctrl->tail_done)) return;
   const int lane = threadIdx.x & 31;
   const int Kn = min(K, n);
@@ -482,6 +482,7 @@ __global__ void __launch_bounds__(256) k_tail_out(const uint32_t *__restrict__ p
     if (lane == 0) {
       if (found < 0) report(ctrl, kStatusInvalidInput, w);
       match[m] = w;
+      if (also) also[m] = w;
       props += static_cast<unsigned long long>(found + 1);
     }
   }

@@ -56,3 +56,34 @@ def test_phases_after_a_device_solve_leave_its_match_alone(n):
         out.fill_(-1)
         assert np.array_equal(phases(c, n), want)
         assert bool((out == -1).all())
+
+
+# one launch, the one-launch tail, the segments, distinct first choices, the
+# rounds, and men who share one list; each the first call on its context
+@pytest.mark.parametrize("device", [True, False])
+@pytest.mark.parametrize("kind,n,param", [
+    (pb.SMP_GEN_UNIFORM, 97, 0), (pb.SMP_GEN_PERFECT, 40, 0), (pb.SMP_GEN_CONGESTED, 200, 0),
+    (pb.SMP_GEN_UNIFORM, 400, 0), (pb.SMP_GEN_UNIFORM, 900, 0), (pb.SMP_GEN_PERFECT, 900, 0),
+    (pb.SMP_GEN_CORRELATED, 700, 500), (pb.SMP_GEN_CONGESTED, 700, 0),
+])
+def test_phases_that_follow_a_solve(kind, n, param, device):
+    pm, pw = oracle.generate(kind, n, 12, 0, param)
+    want, props = oracle.gs_seq(pm, pw)
+    if device:
+        import torch
+
+        pm, pw = torch.from_numpy(pm).cuda(), torch.from_numpy(pw).cuda()
+    with pb.Context() as c:
+        _, st = c.solve(pm, pw)
+        for _ in range(2):  # post returns what the solve found
+            assert np.array_equal(post(c, n), want)
+            assert (c.stats()["proposals"], c.stats()["mode"]) == (props, st["mode"])
+        # init and core start from the precheck
+        assert lib.smp_b200_init(c.handle) == pb.SMP_OK
+        for _ in range(2):
+            assert lib.smp_b200_core(c.handle) == pb.SMP_OK
+            assert np.array_equal(post(c, n), want) and c.stats()["proposals"] == props
+    with pb.Context() as c:
+        c.solve(pm, pw)
+        assert lib.smp_b200_core(c.handle) == pb.SMP_OK
+        assert np.array_equal(post(c, n), want) and c.stats()["proposals"] == props
