@@ -299,7 +299,8 @@ struct Ctx {
   DeviceBuf d_qlist;
   DeviceBuf gen_keys_a, gen_keys_b, gen_seg, gen_temp, gen_aux;
   Control *h_ctrl = nullptr;  // pinned host copy of the control block
-  int32_t *h_verdict = nullptr;  // pinned, behind it: the precheck's verdict
+  uint32_t *h_verdict = nullptr;  // pinned, behind it: the precheck's verdict (verdict.h)
+  uint32_t solve_number = 0;      // of the last precheck enqueued
   bool synchronous = false;      // the caller waits for it, and for every pass
   bool check_after = false;      // and runs the checker after the last one
   cudaEvent_t ev[10] = {};

@@ -141,10 +141,10 @@ int enqueue_precheck(Ctx &c, bool allow_perfect) {
   // zeroed on the device, never copied from the host block (k_precheck)
   if (cudaMemsetAsync(c.d_ctrl.ptr, 0, zero_bytes(n), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
-  if (c.synchronous) *static_cast<volatile int32_t *>(c.h_verdict) = kVerdictNone;
+  c.solve_number++;
   k_precheck<<<grid, 256, 0, c.stream>>>(c.pref_m, n, seen_of(c), c.d_bid.as<unsigned long long>(),
                                          c.d_ctrl.as<Control>(), allow_perfect ? 1 : 0, c.query_ok ? 1 : 0,
-                                         c.synchronous ? c.h_verdict : nullptr);
+                                         c.synchronous ? c.h_verdict : nullptr, c.solve_number);
   c.qcnt_clean = c.bid_clean = true;
   c.launches++;
   return c.check_launch("k_precheck");
@@ -630,17 +630,18 @@ constexpr int kTailMinN = 768;
 // to the tail are spared its launches (a perfect instance of n = 30000 takes
 // 0.131 ms on the device with eleven of them, 0.053 without).  Bounded: without a verdict the tail is
 // enqueued and gated on the device, as it is where nobody waits.
-int32_t precheck_verdict(const Ctx &c) {
+Verdict precheck_verdict(const Ctx &c) {
   if (!c.synchronous || c.pass != kPassQuery) return kVerdictNone;
   const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
-  const volatile int32_t *verdict = c.h_verdict;
-  while (*verdict == kVerdictNone && std::chrono::steady_clock::now() < until) {
+  const volatile uint32_t *word = c.h_verdict;
+  Verdict v;
+  while ((v = verdict_of(*word, c.solve_number)) == kVerdictNone && std::chrono::steady_clock::now() < until) {
   }
-  return *verdict;
+  return v;
 }
 
 int launch_tail_query(Ctx &c) {
-  const int32_t verdict = precheck_verdict(c);
+  const Verdict verdict = precheck_verdict(c);
   if (verdict == kVerdictOther) return SMP_OK;
   if (verdict == kVerdictPerfect) {
     k_match<<<std::max(1, std::min(c.sm_count * 4, (c.n + 255) / 256)), 256, 0, c.stream>>>(
@@ -1838,7 +1839,7 @@ int smp_b200_create(smp_ctx **out, const smp_cfg *cfg) {
     return SMP_ERR_OOM;
   }
   std::memset(c.h_ctrl, 0, sizeof(Control));
-  c.h_verdict = reinterpret_cast<int32_t *>(c.h_ctrl + 1);
+  c.h_verdict = reinterpret_cast<uint32_t *>(c.h_ctrl + 1);
   *c.h_verdict = 0;
   *out = ctx;
   return SMP_OK;

@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "step.cuh"
+#include "verdict.h"
 
 namespace smpb200 {
 
@@ -84,9 +85,6 @@ __device__ __forceinline__ bool any_unset<int32_t>(uint4 v) {
   return v.x == 0xFFFFFFFFu || v.y == 0xFFFFFFFFu || v.z == 0xFFFFFFFFu || v.w == 0xFFFFFFFFu;
 }
 
-// What k_precheck tells a host that waits for it.
-enum Verdict : int32_t { kVerdictNone = 0, kVerdictQuery = 1, kVerdictPerfect = 2, kVerdictOther = 3 };
-
 // ---------------------------------------------------------------------------
 // Precheck.  Marks each man's first choice in an n-bit bitmap (seen, zeroed
 // by the host).  The last block to finish counts the distinct first choices
@@ -103,7 +101,8 @@ enum Verdict : int32_t { kVerdictNone = 0, kVerdictQuery = 1, kVerdictPerfect = 
 __global__ void __launch_bounds__(256) k_precheck(const int32_t *__restrict__ pref_m, int n,
                                                   uint32_t *__restrict__ seen,
                                                   unsigned long long *__restrict__ bid, Control *ctrl,
-                                                  int allow_perfect, int allow_query, volatile int32_t *verdict) {
+                                                  int allow_perfect, int allow_query, volatile uint32_t *verdict,
+                                                  uint32_t solve) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctrl->free_count = n;
     ctrl->allow_perfect = allow_perfect;
@@ -142,9 +141,10 @@ __global__ void __launch_bounds__(256) k_precheck(const int32_t *__restrict__ pr
     ctrl->mode = (allow_query && 4ll * distinct >= n) ? kModeQuery : kModeRank;
     if (verdict) {  // pinned host memory
       __threadfence_system();
-      *verdict = ctrl->status ? kVerdictOther
-                 : ctrl->perfect ? kVerdictPerfect
-                 : ctrl->mode == kModeQuery ? kVerdictQuery : kVerdictOther;
+      *verdict = verdict_word(solve, ctrl->status                ? kVerdictOther
+                                     : ctrl->perfect             ? kVerdictPerfect
+                                     : ctrl->mode == kModeQuery ? kVerdictQuery
+                                                                 : kVerdictOther);
     }
   }
 }
