@@ -17,6 +17,6 @@ int main() {
     }
     bad += verdict_of(0u, solve) != kVerdictNone;  // before the first
   }
-  std::printf(bad ? "BAD %d\n" : "VERDICT_OK\n", bad);
+  std::printf("%s %d\n", bad ? "BAD" : "VERDICT_OK", bad);
   return bad != 0;
 }
