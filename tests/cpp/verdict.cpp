@@ -1,5 +1,6 @@
 // The precheck's verdict word: a word of another solve is no verdict.
 #include <cstdio>
+#include <initializer_list>
 
 #include "verdict.h"
 
