@@ -218,9 +218,9 @@ typedef struct smp_batch_cfg {
                            /* beside the persistent kernel; 0 = auto (the    */
                            /* autotuner times none and the largest 8, 32 and */
                            /* 128; with tune = -1: none), -1 = none          */
-  int32_t cta_width;       /* out of smp_b200_batch_config: 2 where the      */
-                           /* autotuner runs CTAs of twice block_threads     */
-                           /* (one per SM), else 1; ignored on input         */
+  int32_t cta_width;       /* 2: CTAs of twice block_threads; 0 = auto (the  */
+                           /* autotuner may choose them where it chooses     */
+                           /* block_threads and ctas_per_sm, else 1)         */
 } smp_batch_cfg;
 
 typedef struct smp_batch_stats {
@@ -246,8 +246,8 @@ SMP_B200_API int smp_b200_batch_run(smp_batch *batch, smp_instance *results, smp
 SMP_B200_API int smp_b200_batch_run_plain(smp_batch *batch, smp_instance *results, smp_batch_stats *st);
 SMP_B200_API void smp_b200_batch_destroy(smp_batch *batch);
 /* The shape a batch runs with (after tuning): block_threads, ctas_per_sm,
- * window, use_graph, rank_smem_kb (-1: none), tune (1: chosen by the
- * autotuner, -1: fixed) and threshold_n (-1: no instance is routed to the
+ * window, use_graph, rank_smem_kb (-1: none), cta_width, tune (1: chosen by
+ * the autotuner, -1: fixed) and threshold_n (-1: no instance is routed to the
  * all-SM pipeline). */
 SMP_B200_API int smp_b200_batch_config(const smp_batch *batch, smp_batch_cfg *out);
 /* create + run + destroy; the status and proposals of inst[] are filled in. */

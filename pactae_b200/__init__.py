@@ -311,7 +311,8 @@ class Batch:
     alive while the batch is used."""
 
     def __init__(self, ctx: Context, instances, block_threads: int = 0, ctas_per_sm: int = 0, window: int = 0,
-                 use_graph: bool = True, rank_smem_kb: int = 0, tune: bool = True, threshold_n: int = 0):
+                 use_graph: bool = True, rank_smem_kb: int = 0, tune: bool = True, threshold_n: int = 0,
+                 cta_width: int = 0):
         self.ctx = ctx
         self._keep = list(instances)
         count = len(self._keep)
@@ -333,6 +334,7 @@ class Batch:
         cfg.rank_smem_kb = rank_smem_kb
         cfg.tune = 0 if tune else -1
         cfg.threshold_n = threshold_n
+        cfg.cta_width = cta_width
         handle = ctypes.c_void_p()
         import torch
 
@@ -348,12 +350,20 @@ class Batch:
         _check(fn(self._h, results, ctypes.byref(st)), "smp_b200_batch_run")
         return [r.status for r in results], [r.proposals for r in results], st.as_dict()
 
+    def _config(self) -> smp_batch_cfg:
+        cfg = smp_batch_cfg()
+        _check(lib.smp_b200_batch_config(self._h, ctypes.byref(cfg)), "smp_b200_batch_config")
+        return cfg
+
     def config(self) -> dict:
         """The shape the batch runs with (after tuning), with threshold_n:
         instances above it run the all-SM pipeline (-1: none)."""
-        cfg = smp_batch_cfg()
-        _check(lib.smp_b200_batch_config(self._h, ctypes.byref(cfg)), "smp_b200_batch_config")
-        return cfg.as_dict()
+        return self._config().as_dict()
+
+    @property
+    def cta_width(self) -> int:
+        """2 where the CTAs have twice config()["block_threads"] threads, else 1."""
+        return self._config().cta_width
 
     def run(self) -> tuple[list[int], list[int], dict]:
         """Batched persistent launch: (statuses, proposals, stats)."""

@@ -1,12 +1,12 @@
 // batch.cu -- the batch ABI: many instances in one persistent launch,
 // captured as a CUDA graph, and the one-launch-per-instance baseline.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <numeric>
-#include <tuple>
 #include <vector>
 
 #include "batch_kernels.cuh"
@@ -143,10 +143,24 @@ int apply_shape(smp_batch &b, const Shape &sh) {
   return set_batch_attribute(b);
 }
 
-// Tuned shapes, per device, largest n and batch size (powers of two).
+// Tuned shapes and thresholds, per device, largest n, batch size (powers of
+// two) and the fields the caller fixed (0: left to the autotuner).
+using TuneKey = std::array<int, 8>;
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int>, Shape> g_tuned;
-std::map<std::tuple<int, int, int>, int> g_tuned_thr;
+std::map<TuneKey, Shape> g_tuned;
+std::map<TuneKey, int> g_tuned_thr;
+
+TuneKey tune_key(const smp_batch &b, const Shape &sh, const smp_batch_cfg *cfg) {
+  TuneKey key = {b.ctx->c.device, b.max_n, 31 - __builtin_clz(static_cast<unsigned>(b.count))};
+  if (cfg) {
+    if (cfg->block_threads > 0) key[3] = sh.block;
+    if (cfg->ctas_per_sm > 0) key[4] = sh.per_sm;
+    if (cfg->window > 0) key[5] = sh.subs;
+    key[6] = cfg->rank_smem_kb > 0 ? cfg->rank_smem_kb : cfg->rank_smem_kb < 0 ? -1 : 0;
+    if (cfg->cta_width == 2) key[7] = 2;
+  }
+  return key;
+}
 
 // Runs the kernel over the sample table and returns its device time.
 float time_shape(smp_batch &b, const Shape &sh, BatchInstance *sample, const int32_t *order, int k) {
@@ -191,7 +205,7 @@ Shape autotune(smp_batch &b, Shape start, const smp_batch_cfg *cfg) {
   };
   if (!(cfg && cfg->window > 0))
     for (int subs : {1, 2, 4, 8}) consider({best.block, best.per_sm, subs, best.rank_kb, best.width});
-  if (!(cfg && (cfg->block_threads > 0 || cfg->ctas_per_sm > 0)))
+  if (!(cfg && (cfg->block_threads > 0 || cfg->ctas_per_sm > 0 || cfg->cta_width == 2)))
     for (const Shape &sh : {Shape{512, 1, 1, 0, 2}, {512, 1, 1, 0, 1}, {512, 2, 1, 0, 1}, {256, 2, 1, 0, 1}, {256, 4, 1, 0, 1}})
       consider({sh.block, sh.per_sm, best.subs, best.rank_kb, sh.width});
   if (!(cfg && cfg->rank_smem_kb != 0))
@@ -416,8 +430,9 @@ int smp_b200_batch_create(smp_ctx *ctx, const smp_instance *inst, int32_t count,
   // Shape: fixed fields from cfg, the rest tuned (or defaults with tune = -1).
   Shape sh{512, 2, 1, 32};  // the best shape on the 8192-instance mix
   if (cfg && cfg->block_threads > 0) sh.block = std::min(512, std::max(64, cfg->block_threads / 32 * 32));
+  if (cfg && cfg->cta_width == 2) sh.width = 2;
   if (cfg && cfg->ctas_per_sm > 0) sh.per_sm = std::min(4, cfg->ctas_per_sm);
-  else if (cfg && cfg->block_threads > 0) sh.per_sm = std::max(1, 1024 / sh.block);
+  else if (cfg && (cfg->block_threads > 0 || sh.width == 2)) sh.per_sm = std::max(1, 1024 / (sh.block * sh.width));
   if (cfg && cfg->window > 0) sh.subs = subs_for_window(cfg->window);
   if (cfg && cfg->rank_smem_kb != 0) sh.rank_kb = std::max(0, cfg->rank_smem_kb);
   b->use_graph = !(cfg && cfg->use_graph < 0);
@@ -425,6 +440,7 @@ int smp_b200_batch_create(smp_ctx *ctx, const smp_instance *inst, int32_t count,
                          !(cfg && cfg->block_threads > 0 && cfg->ctas_per_sm > 0 && cfg->window > 0 &&
                            cfg->rank_smem_kb != 0);
   const bool want_thr = !(cfg && cfg->tune < 0) && !(cfg && cfg->threshold_n != 0);
+  const TuneKey key = tune_key(*b, sh, cfg);
   // Without tuning, shrink a default shape that does not fit (large max_n).
   while (!shape_fits(c, b->max_n, sh) && sh.rank_kb > 0) sh.rank_kb -= 32;
   if (!shape_fits(c, b->max_n, sh) && !(cfg && cfg->ctas_per_sm > 0)) sh.per_sm = 1;
@@ -472,7 +488,6 @@ int smp_b200_batch_create(smp_ctx *ctx, const smp_instance *inst, int32_t count,
     return SMP_ERR_CUDA;
   }
   if (want_tune) {
-    const auto key = std::make_tuple(c.device, b->max_n, 31 - __builtin_clz(static_cast<unsigned>(count)));
     bool cached = false;
     {
       std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -497,7 +512,6 @@ int smp_b200_batch_create(smp_ctx *ctx, const smp_instance *inst, int32_t count,
   // Routing to the all-SM pipeline: as configured, or timed on the batch.
   int thr = cfg && cfg->threshold_n > 0 ? cfg->threshold_n : -1;
   if (want_thr) {
-    const auto key = std::make_tuple(c.device, b->max_n, 31 - __builtin_clz(static_cast<unsigned>(count)));
     bool cached = false;
     {
       std::lock_guard<std::mutex> lock(g_tune_mu);
