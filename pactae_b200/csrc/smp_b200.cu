@@ -1194,7 +1194,14 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
   int rc = do_stage(c, pref_m, pref_w, n, flags);
   c.pass_flags = flags;
   c.pass_match = match_out;
-  c.match_direct = (flags & SMP_F_DEVICE_PTRS) && n > 0 && kernel_may_write(c, match_out, sizeof(int32_t) * static_cast<size_t>(n));
+  // (never into the lists: a kernel that writes the matching may still read them)
+  const auto inside = [&](const int32_t *list) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(match_out), b = reinterpret_cast<uintptr_t>(list);
+    const size_t row = sizeof(int32_t) * static_cast<size_t>(n);
+    return a < b + row * n && b < a + row;
+  };
+  c.match_direct = !rc && (flags & SMP_F_DEVICE_PTRS) && !inside(pref_m) && !inside(pref_w) &&
+                   kernel_may_write(c, match_out, sizeof(int32_t) * static_cast<size_t>(n));
   if (!rc && solve_is_small(c, flags)) {
     c.pass = kPassSmall;
     return enqueue_small(c, match_out, flags);

@@ -87,3 +87,15 @@ def test_phases_that_follow_a_solve(kind, n, param, device):
         c.solve(pm, pw)
         assert lib.smp_b200_core(c.handle) == pb.SMP_OK
         assert np.array_equal(post(c, n), want) and c.stats()["proposals"] == props
+
+
+@pytest.mark.parametrize("kind", [pb.SMP_GEN_PERFECT, pb.SMP_GEN_UNIFORM])
+@pytest.mark.parametrize("n", [200, 600, 5000])
+def test_match_may_lie_in_a_list_that_is_not_needed_again(ctx, kind, n):
+    # the matching is copied over a row once everything has been read
+    for side in (0, 1):
+        for row in (0, n // 2, n - 1):
+            lists = ctx.generate(kind, n, 4)
+            want, _ = ctx.solve(*lists)
+            match, _ = ctx.solve(*lists, out=lists[side][row])
+            assert bool((match == want).all()) and match.data_ptr() == lists[side][row].data_ptr()
