@@ -634,6 +634,14 @@ __device__ __forceinline__ RoundCount chains_by_warp(const RoundChains &q) {
 // displacement), here a step's longest chain is (70 windows of 0.74 us where
 // the mean is 30 of 1.1): correlated n = 30000 8.6 -> 7.9 ms, n = 8000 1.54 ->
 // 1.37, SOLO n = 10007 3.3 -> 3.0.  Counts in the first lane of each eight.
+//   Where lists are old a window rejects him whole, and eight lanes take as long
+// for it as a warp for eight.  A group that has passed more than kDeepWindows
+// windows and kDeepPerHop a displacement parks its man at the next one: he is
+// scanned again, and where all men have started so is everyone.  (Where n is not
+// above kCand no list runs out, so nothing else would park him: SOLO n = 600,
+// one chain that passes nine windows a displacement, took 5.9 ms for 1.1.)
+constexpr unsigned int kDeepWindows = 32;
+constexpr unsigned int kDeepPerHop = 4;
 __device__ __forceinline__ RoundCount chains_by_group(const RoundChains &q) {
   const int n = q.n;
   const int cap = q.b.cap;
@@ -647,7 +655,7 @@ __device__ __forceinline__ RoundCount chains_by_group(const RoundChains &q) {
     return r < cap ? *reinterpret_cast<const uint4 *>(q.b.cand + static_cast<uint32_t>(man * cap + r))
                    : make_uint4(kNoCand, kNoCand, kNoCand, kNoCand);
   };
-  unsigned int hops = 0, lost = 0;
+  unsigned int hops = 0, lost = 0, passed = 0;
   bool has = false, out = false;  // a man; no more of them
   bool fresh = false;             // his window is still to be loaded
   int m = 0, pos = 0;             // the man and the list entry to try next
@@ -693,8 +701,8 @@ __device__ __forceinline__ RoundCount chains_by_group(const RoundChains &q) {
     const uint32_t rk = __shfl_sync(kFullMask, fe, src) & 0xFFFFu;
     const uint32_t hw = __shfl_sync(kFullMask, fw, src);
     if (has && !found) {
-      if (!ends) {
-        pos = (pos & ~3) + 32;
+      pos = (pos & ~3) + 32;  // every entry before it has rejected him
+      if (!ends && ++passed <= kDeepWindows + kDeepPerHop * hops) {
         fresh = true;
       } else {
         if (gl == 0) {
@@ -702,7 +710,7 @@ __device__ __forceinline__ RoundCount chains_by_group(const RoundChains &q) {
             report(q.ctrl, kStatusInvalidInput, m);
             *q.s_stop = 1;
           } else {
-            spos[m] = static_cast<uint16_t>(cap - 1);
+            spos[m] = static_cast<uint16_t>(min(pos, cap) - 1);
             q.park[atomicAdd(q.s_parked, 1)] = m;
           }
         }
