@@ -14,6 +14,10 @@
 // every woman; where all first choices are distinct only those are read.
 //
 // n = 97 uniform, from call to return: 136 -> 61 us.
+//   Men who share one list would make all n (n + 1) / 2 proposals, and where the
+// women share one too, all of them displace someone.  One warp takes the women
+// in the list's order instead: each has the best man whom no woman before her
+// has (the only stable matching there is).
 #pragma once
 
 #include "common.cuh"
@@ -109,9 +113,46 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
         list[t] = static_cast<uint16_t>((w << 8) | rank[w * n + m]);
     }
     if (differ) s_differ = 1;
-    // the chains: a warp each, 32 choices at a time (all warps or none: one that
-    // refuses a man in there must not keep lanes of a later one out)
-    if (!__syncthreads_or(s_status != 0)) {
+    // (all warps or none: one that refuses a man in the chains must not keep lanes
+    // of a later one out)
+    const bool refused = __syncthreads_or(s_status != 0);
+    const bool shared = mode == kModeRank && distinct == 1 && n >= 2 && !s_differ;
+    if (!refused && shared) {
+      if (tid < 32) {
+        // a lane keeps men lane, 32 + lane, ...; the next woman's ranks of them are
+        // loaded while this one's best is found
+        constexpr int kMen = kSmallMaxN / 32;
+        uint32_t gone[kMen], r[kMen], next[kMen];  // gone: all ones once taken
+        const auto load = [&](int w, uint32_t (&to)[kMen]) {
+#pragma unroll
+          for (int j = 0; j < kMen; ++j)
+            to[j] = lane + 32 * j < n ? (static_cast<uint32_t>(rank[w * n + lane + 32 * j]) << 16) | (lane + 32 * j) : 0u;
+        };
+#pragma unroll
+        for (int j = 0; j < kMen; ++j) gone[j] = lane + 32 * j < n ? 0u : 0xFFFFFFFFu;
+        int w = list[0] >> 8, after = list[min(1, n - 1)] >> 8;
+        load(w, r);
+        for (int k = 0; k < n; ++k) {
+          load(after, next);
+          const int w2 = after;
+          after = list[min(k + 2, n - 1)] >> 8;
+          uint32_t best = 0xFFFFFFFFu;
+#pragma unroll
+          for (int j = 0; j < kMen; ++j) best = min(best, r[j] | gone[j]);
+          best = __reduce_min_sync(kFullMask, best);
+          const int m = static_cast<int>(best & 0xFFFFu);
+#pragma unroll
+          for (int j = 0; j < kMen; ++j) gone[j] |= m == lane + 32 * j ? 0xFFFFFFFFu : 0u;
+          if (lane == 0) {
+            word[w] = best;  // (a woman the list names twice leaves another free: refused below)
+            spos[m] = static_cast<uint16_t>(k);
+          }
+          w = w2;
+#pragma unroll
+          for (int j = 0; j < kMen; ++j) r[j] = next[j];
+        }
+      }
+    } else if (!refused) {  // the chains: a warp each, 32 choices at a time
       unsigned int hops = 0;
       int m = -1, pos = 0;
       for (;;) {
