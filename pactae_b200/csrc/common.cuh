@@ -35,7 +35,7 @@ struct Control {
   int32_t allow_query;    // host switch: 1 if the query mode may be chosen
   int32_t blocks_done;    // precheck: blocks that finished (the last one decides)
   int32_t distinct;       // precheck: number of distinct first choices
-  int32_t distinct_w;     // k_wdistinct: distinct first choices of the women
+  int32_t distinct_w;     // k_wdistinct, k_swap_pos: distinct first choices of the women
   int32_t use_filter;     // k_wdistinct: k_bulk runs with its shared partner-rank filter
   int32_t swap_fail;      // k_swap_screen: a pref_m row differs from row 0
   unsigned long long proposals;        // sum over men of (final position + 1)
@@ -53,12 +53,10 @@ struct Control {
   int32_t swap_over;      // k_swap_gs: women stopped at the end of what the device holds of their rows
   int32_t round_done;     // k_round: the matching is complete and written
   // the women-proposing screen with the proposals beside it (swap_kernels.cuh)
-  int32_t w_first;        // the women's first choices differ
   int32_t screen_next;    // rows its CTAs have taken beyond their first
   int32_t screen_ctas;    // CTAs of it that have finished
   int32_t screen_done;    // all have
   int32_t swap_out;       // match[] is written
-  int32_t swap_quit;      // a warp of the proposals beside it gave up
   int32_t tail_left;      // k_tail_q: chains that have not ended
   int32_t tail_done;      // none are left and the words are final
   int32_t check_deep;     // k_check_near: some man's wife is not among his first choices

@@ -1064,7 +1064,8 @@ int enqueue_pass_mode(Ctx &c, int mode) {
 
 // Rank-mode men who all make the same first choice may share one list.  The
 // screen checks that on all SMs (and that pref_w's rows are permutations).
-constexpr int kSwapBeside = 1;  // CTAs per SM of the proposals
+constexpr int kSwapBeside = 1;       // CTAs per SM of the proposals beside the screen
+constexpr int kSwapBesideAlike = 2;  // where the women's lists are alike
 bool swap_screen_fits(const Ctx &c) { return swap_screen_smem(c.n) <= c.smem_optin; }
 
 int enqueue_swap_screen(Ctx &c, bool men_screened) {
@@ -1080,16 +1081,17 @@ int enqueue_swap_screen(Ctx &c, bool men_screened) {
   if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
       cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("swap reset");
-  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl, c.pref_w);
+  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl, c.pref_w, seen_of(c));
   uint16_t *near = n <= kU16MaxN ? c.d_swap_near.as<uint16_t>() : nullptr;
   if (near) k_swap_near<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_w, near, n);
-  // the women's proposals beside the screen, which leaves a CTA's place on
-  // each SM: where it fills them, the proposals may not start before it ends
+  // the women's proposals beside the screen, which leaves a CTA's place on each
+  // SM (two where their lists are alike): where it fills them, the proposals may
+  // not start before it ends
   if (cudaEventRecord(c.ev_fork, c.stream) != cudaSuccess ||
       cudaStreamWaitEvent(c.side_stream, c.ev_fork, 0) != cudaSuccess)
     return c.fail_cuda("swap fork");
-  k_swap_gs<<<c.sm_count * kSwapBeside, 256, 0, c.side_stream>>>(c.pref_m, c.pref_w, pos, bid, n, ctrl, nullptr, n, nullptr,
-                                                       nullptr, 0, 1, near);
+  k_swap_gs<<<c.sm_count * kSwapBesideAlike, 256, 0, c.side_stream>>>(
+      c.pref_m, c.pref_w, pos, bid, n, ctrl, nullptr, n, nullptr, nullptr, 0, 1, near, c.sm_count * kSwapBeside);
   rc = c.check_launch("k_swap_gs");
   if (!rc && allow_dynamic_smem(c, k_swap_screen) != cudaSuccess) rc = c.fail_cuda("k_swap_screen smem attribute");
   const size_t screen_smem = swap_screen_smem(n);
@@ -1101,13 +1103,18 @@ int enqueue_swap_screen(Ctx &c, bool men_screened) {
   const int t0 = men_screened ? n : 1;  // the host compared the men's rows already
   if (!rc) {
     k_swap_screen<<<std::max(1, std::min(2 * n - t0, c.sm_count * std::max(per_sm - kSwapBeside, 1))), 256, screen_smem,
-                    c.stream>>>(c.pref_m, c.pref_w, n, ctrl, t0);
+                    c.stream>>>(c.pref_m, c.pref_w, n, ctrl, t0, c.sm_count * std::max(per_sm - kSwapBesideAlike, 1));
     rc = c.check_launch("k_swap_screen");
+    if (!rc && (cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess ||
+                cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess))
+      rc = c.fail_cuda("event");
+    if (!rc) {
+      k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_m, c.pref_w, pos, bid, n, ctrl, nullptr, n, nullptr, nullptr,
+                                                      0, 2, near);
+      rc = c.check_launch("k_swap_gs");
+    }
   }
-  c.launches += near ? 5 : 4;
-  if (!rc && (cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess ||
-              cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess))
-    rc = c.fail_cuda("event");
+  c.launches += near ? 6 : 5;
   // join the side stream, even after an error: its kernel uses the buffers
   if (cudaEventRecord(c.ev_join, c.side_stream) != cudaSuccess ||
       cudaStreamWaitEvent(c.stream, c.ev_join, 0) != cudaSuccess)
@@ -1118,33 +1125,6 @@ int enqueue_swap_screen(Ctx &c, bool men_screened) {
   if (rc) return rc;
   k_swap_outcome<<<grid, 256, 0, c.stream>>>(c.pref_m, c.pref_w, bid, c.d_match.as<int32_t>(), n, ctrl);
   rc = c.check_launch("k_swap_outcome");
-  if (!rc) rc = copy_match_out(c, c.pass_match, (c.pass_flags & SMP_F_DEVICE_PTRS) != 0);
-  if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  return rc ? rc : read_control(c);
-}
-
-// The screen found one shared list, and proposals still to be made: the women
-// differ, but not in their first choices, so those beside the screen gave up.
-int enqueue_swap_solve(Ctx &c) {
-  const int n = c.n;
-  Control *ctrl = c.d_ctrl.as<Control>();
-  unsigned long long *bid = c.d_bid.as<unsigned long long>();
-  c.bid_clean = false;
-  if (cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
-      cudaMemsetAsync(&ctrl->swap_next, 0, sizeof(int32_t), c.stream) != cudaSuccess)
-    return c.fail_cuda("swap bid reset");
-  if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_m, c.pref_w, c.d_swap_pos.as<int32_t>(), bid, n, ctrl, nullptr,
-                                                  n, nullptr, nullptr, 0, 0, nullptr);
-  c.launches++;
-  int rc = c.check_launch("k_swap_gs");
-  if (!rc && cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (!rc && cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (rc) return rc;
-  k_swap_match<<<std::max(1, std::min(c.sm_count * 4, (n + 255) / 256)), 256, 0, c.stream>>>(
-      c.pref_m, bid, c.d_match.as<int32_t>(), n, ctrl);
-  c.launches++;
-  rc = c.check_launch("k_swap_match");
   if (!rc) rc = copy_match_out(c, c.pass_match, (c.pass_flags & SMP_F_DEVICE_PTRS) != 0);
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   return rc ? rc : read_control(c);
@@ -1236,8 +1216,7 @@ int solve_advance(Ctx &c, bool &more) {
   if (c.pass == kPassScreen && !h.swap_fail) {
     c.pass = kPassLast;
     c.swapped = true;
-    more = !h.swap_out;
-    return more ? enqueue_swap_solve(c) : SMP_OK;
+    return SMP_OK;
   }
   more = true;
   c.poll_rounds = in_rounds(c);
@@ -1294,10 +1273,7 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
   swapped = c.h_ctrl->status || !c.h_ctrl->swap_fail;
   if (!swapped || c.h_ctrl->status) return SMP_OK;
   c.swapped = true;
-  if (c.h_ctrl->swap_out) return SMP_OK;
-  rc = enqueue_swap_solve(c);
-  if (!rc) rc = c.sync("solve");
-  return rc;
+  return SMP_OK;
 }
 
 // Statistics and status of a solve whose stream has completed.

@@ -28,17 +28,24 @@
 namespace smpb200 {
 
 // pos[L[r]] = r, with pos preset to -1; an entry out of range or seen twice
-// makes row 0 no permutation.  With pref_w given, w_first says whether the
-// women's first choices differ.
+// makes row 0 no permutation.  With pref_w given, distinct_w counts the women's
+// first choices in the precheck's bitmap, which holds one bit by then (the men
+// share their first choice): the count may be one too low.
 __global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl,
-                           const int32_t *__restrict__ pref_w = nullptr) {
+                           const int32_t *__restrict__ pref_w = nullptr, uint32_t *__restrict__ seen = nullptr) {
+  unsigned firsts = 0;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const int w = __ldg(pref_m + r);
     if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1)
       report(ctrl, kStatusInvalidInput, w);
-    if (pref_w && __ldg(pref_w + static_cast<size_t>(r) * n) != __ldg(pref_w) && !ld_volatile_s32(&ctrl->w_first))
-      ctrl->w_first = 1;
+    if (pref_w) {
+      const int m = __ldg(pref_w + static_cast<size_t>(r) * n);
+      const uint32_t bit = 1u << (m & 31);
+      if (static_cast<unsigned>(m) < static_cast<unsigned>(n) && !(atomicOr(seen + (m >> 5), bit) & bit)) firsts++;
+    }
   }
+  firsts = __reduce_add_sync(kFullMask, firsts);
+  if (firsts && (threadIdx.x & 31) == 0) atomicAdd(&ctrl->distinct_w, static_cast<int>(firsts));
 }
 
 // Rows t = 1 .. n-1 compare pref_m row t with row 0; rows t = n .. 2n-1
@@ -52,6 +59,11 @@ __global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restri
 // bitmap's shared atomics, took 1.85 ms against 1.47 ms at n = 30000.  Where the
 // women share one list too, comparing with row 0 instead of marking: 1.96 -> 1.30.)
 __host__ __device__ constexpr size_t swap_screen_smem(int n) { return ((static_cast<size_t>(n) + 31) / 32) * 4; }
+
+// Fewer than n / 4 distinct first choices (k_swap_pos).
+__device__ __forceinline__ bool women_alike(const Control *ctrl, int n) {
+  return 4ll * ld_volatile_s32(&ctrl->distinct_w) < n;
+}
 
 // Does this thread's share of row t differ from row 0?  Chunk by chunk where
 // both rows start at the same 16-byte offset (all rows when n is a multiple of
@@ -86,7 +98,7 @@ __device__ __forceinline__ bool row_differs(const int32_t *__restrict__ pref, in
 
 __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__ pref_m,
                                                      const int32_t *__restrict__ pref_w, int n, Control *ctrl,
-                                                     int t0) {
+                                                     int t0, int alike_cta) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *seen = reinterpret_cast<uint32_t *>(smem_raw);
   __shared__ int s_stop;
@@ -99,13 +111,16 @@ __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__
   int bad_value = 0;
   // Rows are taken in turn, each CTA's next one while it works on the last: a
   // CTA that waits for the proposals' CTA to leave its SM then takes fewer.
+  // Those from alike_cta on leave after their first where the women's lists are
+  // alike: a second CTA of the proposals gets their place.
   int next = t0 + static_cast<int>(blockIdx.x);
+  const bool leaves = static_cast<int>(blockIdx.x) >= alike_cta && women_alike(ctrl, n);
   for (;;) {
     if (tid == 0) {
       s_row = next;
       s_stop = next >= 2 * n || ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status);
       s_wsame = !ld_volatile_s32(&ctrl->w_differ);
-      next = t0 + static_cast<int>(gridDim.x) + atomicAdd(&ctrl->screen_next, 1);
+      next = leaves ? 2 * n : t0 + static_cast<int>(gridDim.x) + atomicAdd(&ctrl->screen_next, 1);
     }
     __syncthreads();
     if (s_stop) break;
@@ -201,26 +216,39 @@ __global__ void __launch_bounds__(256) k_swap_near(const int32_t *__restrict__ p
 // position 0).  Gale-Shapley's result does not depend on that order.  An
 // entry out of range is reported; a woman who runs out of her whole row
 // (input that is not a permutation) too.
-//   beside: the screen runs at the same time.  The proposals are a chain of L2
+//   beside = 1: the screen runs at the same time.  The proposals are a chain of L2
 // round trips that leaves the memory idle, the screen a stream that leaves
 // the SMs idle: n = 30000 congested took 1.31 ms and then 0.82 ms.  An entry
 // that is not a permutation's is the screen's to report here; the proposals
 // give up when it has found that the men's lists differ, that the input is
 // invalid, or that the women share one list too (they would make n (n + 1) / 2
 // contended proposals) -- at once if even their first choices are all alike.
+// Two CTAs per SM where the women's lists are alike (women_alike: the proposals
+// contend, and there are many times more of them), one where they are not and
+// the screen sets the time: it leaves them that much room.
+//   beside = 2: after the screen, what is left of the proposals, with four CTAs
+// per SM.  (n = 30000, women correlated with sigma 0.2 / 0.01 / 0.0003: 3.4, 5.2
+// and 17.9 ms all after the screen; 3.7, 13.0 and 49 with one CTA per SM beside it
+// and to the end; 2.8, 4.5 and 14.8 so.)
 __global__ void __launch_bounds__(256) k_swap_gs(const int32_t *__restrict__ pref_m,
                                                  const int32_t *__restrict__ pref_w,
                                                  const int32_t *__restrict__ pos,
                                                  unsigned long long *__restrict__ bid, int n, Control *ctrl,
                                                  const uint8_t *__restrict__ full, int depth,
                                                  int2 *__restrict__ over, const int2 *__restrict__ start,
-                                                 int start_count, int beside, const uint16_t *__restrict__ near) {
+                                                 int start_count, int beside, const uint16_t *__restrict__ near,
+                                                 int alike_cta = 0) {
   const int lane = threadIdx.x & 31;
   const int total = start ? start_count : n;
   int w = -1, r0 = 0;
   uint32_t key = 0;
   unsigned steps = 0;
-  if (beside && !ld_volatile_s32(&ctrl->w_first)) return;
+  if (beside == 1 && (ld_volatile_s32(&ctrl->distinct_w) <= 1 ||
+                      (static_cast<int>(blockIdx.x) >= alike_cta && !women_alike(ctrl, n))))
+    return;
+  if (beside == 2 && (ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status) ||
+                      !ld_volatile_s32(&ctrl->w_differ)))
+    return;
   for (;;) {
     // Now and then only: thousands of warps reading these flags at every step
     // would queue at one L2 slice.
@@ -229,10 +257,7 @@ __global__ void __launch_bounds__(256) k_swap_gs(const int32_t *__restrict__ pre
       if (lane == 0)
         stop = ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status) ||
                (ld_volatile_s32(&ctrl->screen_done) && !ld_volatile_s32(&ctrl->w_differ));
-      if (__shfl_sync(kFullMask, stop, 0)) {
-        if (lane == 0) atomicExch(&ctrl->swap_quit, 1);
-        return;
-      }
+      if (__shfl_sync(kFullMask, stop, 0)) return;
     }
     if (w < 0) {
       int i = 0;
@@ -355,14 +380,12 @@ __global__ void k_swap_mark_full(uint8_t *__restrict__ full, const int32_t *__re
 // The outcome of the screen and the proposals beside it: nothing where the
 // men's lists differ or the input is invalid; the pairing rank for rank where
 // the women share one list too; else match[m] = the woman m holds.  swap_out
-// says that match[] is complete (the host runs the proposals alone if they
-// gave up without cause: women who differ, but not in their first choice).
+// says that match[] is complete.
 __global__ void k_swap_outcome(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
                                const unsigned long long *__restrict__ bid, int32_t *__restrict__ match, int n,
                                Control *ctrl) {
   if (ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status)) return;
   const bool alike = !ld_volatile_s32(&ctrl->w_differ);
-  if (!alike && (!ld_volatile_s32(&ctrl->w_first) || ld_volatile_s32(&ctrl->swap_quit))) return;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     if (alike) {
       match[__ldg(pref_w + k)] = __ldg(pref_m + k);
