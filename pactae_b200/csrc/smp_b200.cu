@@ -160,6 +160,15 @@ size_t rank_matrix_bytes(const Ctx &c) { return static_cast<size_t>(c.n) * rank_
 // one SM holds the bids; else through k_bulk.
 bool in_rounds(const Ctx &c) { return c.rank_bytes == 2 && c.tail_threshold > 0; }
 
+// The men start by popularity (k_order_*) in the rounds, and in k_bulk from this
+// n on, unless k_wdistinct has chosen its filtered variant: below it the two launches cost more than they save (rank mode without a
+// tail, correlated n = 500 / 1500 / 6000: 303, 453 and 1737 us without, 321, 496
+// and 1793 with; n = 40000 25.2 and 24.7 ms, both sides one list 206 and 69).
+constexpr int kOrderMinN = 8192;
+bool ordered(const Ctx &c) { return in_rounds(c) || c.n >= kOrderMinN; }
+bool filter_fits(const Ctx &c) { return sizeof(uint32_t) * static_cast<size_t>(c.n) + 1024 <= c.smem_optin; }
+const int32_t *men_order(const Ctx &c) { return ordered(c) ? c.d_order.as<int32_t>() : nullptr; }
+
 // Rows of int32 ranks have ld = n.
 template <typename RankT>
 int enqueue_invert(Ctx &c, const int32_t *pref_w, RankT *rank, size_t ld, int gate) {
@@ -232,9 +241,15 @@ int order_buffers(Ctx &c) {
 // man-major (d_rankT); where k_bulk proposes with uint16 ranks, by position too.
 int enqueue_rank(Ctx &c, int gate) {
   int rc = c.d_rankT.ensure(rank_matrix_bytes(c));
-  if (!rc) rc = order_buffers(c);
+  if (!rc && ordered(c)) rc = order_buffers(c);
   if (!rc) rc = enqueue_invert_any(c, gate);
-  if (!rc) rc = enqueue_order(c, gate);
+  if (!rc && !in_rounds(c) && gate == kGateModeRank && filter_fits(c)) {
+    // decides on the device which variant of k_bulk runs
+    k_wdistinct<<<1, 1024, sizeof(uint32_t) * ((c.n + 31) / 32), c.stream>>>(c.pref_w, c.n, c.d_ctrl.as<Control>());
+    c.launches++;
+    rc = c.check_launch("k_wdistinct");
+  }
+  if (!rc && ordered(c)) rc = enqueue_order(c, gate == kGateModeRank ? kGateOrder : gate);
   if (rc) return rc;
   const int tiles = (c.n + 63) / 64;
   const int grid = static_cast<int>(std::min<long long>(static_cast<long long>(c.sm_count) * 4,
@@ -468,14 +483,9 @@ int launch_bulk(Ctx &c, int round) {
   const RankT *rank = proposal_ranks<RankT>(c);
   const uint32_t *prefix = c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr;
   const int rank_threshold = c.tail_threshold > 0 ? std::min(c.tail_threshold, c.tail_threshold_rank) : 0;
-  const size_t filter = sizeof(uint32_t) * static_cast<size_t>(c.n);
-  if (!in_rounds(c) && round == 0 && c.known_mode != kModeQuery && filter + 1024 <= c.smem_optin) {  // the filter fits
-    // k_wdistinct decides on the device which of the two variants runs
-    k_wdistinct<<<1, 1024, sizeof(uint32_t) * ((c.n + 31) / 32), c.stream>>>(c.pref_w, c.n, c.d_ctrl.as<Control>());
-    c.launches++;
-    int rc = c.check_launch("k_wdistinct");
-    if (rc) return rc;
-    const auto kernel = k_bulk<RankT, kSub, true>;
+  if (!in_rounds(c) && round == 0 && c.known_mode != kModeQuery && filter_fits(c)) {
+    const size_t filter = sizeof(uint32_t) * static_cast<size_t>(c.n);
+    const auto kernel = k_bulk<RankT, kSub, true>;  // the women are unlike: no order helps
     if (allow_dynamic_smem(c, kernel) !=
         cudaSuccess)
       return c.fail_cuda("k_bulk smem attribute");
@@ -486,16 +496,27 @@ int launch_bulk(Ctx &c, int round) {
     }
     kernel<<<c.sm_count * std::max(per_sm, 1), kFilterBlock, filter, c.stream>>>(
         c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-        c.d_order.as<int32_t>(), c.n, c.tail_threshold, rank_threshold, round, -1);
+        nullptr, c.n, c.tail_threshold, rank_threshold, round, -1);
     c.launches++;
-    rc = c.check_launch("k_bulk (filtered)");
+    const int rc = c.check_launch("k_bulk (filtered)");
     if (rc) return rc;
   }
-  k_bulk<RankT, kSub><<<resident_grid(c, k_bulk<RankT, kSub>, 256), 256, 0, c.stream>>>(
-      c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-      c.d_order.as<int32_t>(), c.n, c.tail_threshold, rank_threshold, round, in_rounds(c) ? kModeQuery : c.known_mode);
-  c.launches++;
-  return c.check_launch("k_bulk");
+  // Query-mode men start as they are numbered; the ordered variant's take-up took
+  // 5 % of a query-mode bulk (n = 6000 without a tail: 1.85 and 1.95 ms).
+  const auto launch = [&](auto kernel, int only_mode) {
+    kernel<<<resident_grid(c, kernel, 256), 256, 0, c.stream>>>(
+        c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
+        men_order(c), c.n, c.tail_threshold, rank_threshold, round, only_mode);
+    c.launches++;
+    return c.check_launch("k_bulk");
+  };
+  if (in_rounds(c)) return launch(k_bulk<RankT, kSub>, kModeQuery);
+  if (!ordered(c)) return launch(k_bulk<RankT, kSub>, c.known_mode);
+  int rc = SMP_OK;
+  const bool query = round == 0 && c.query_ok;
+  if (query && c.known_mode != kModeRank) rc = launch(k_bulk<RankT, kSub>, kModeQuery);
+  if (!rc && c.known_mode != kModeQuery) rc = launch(k_bulk<RankT, kSub, false, true>, query ? kModeRank : c.known_mode);
+  return rc;
 }
 
 template <typename RankT, int kSub>
@@ -506,7 +527,7 @@ int launch_tail(Ctx &c, int round, int only_mode) {
   if (allow_dynamic_smem(c, k_tail<RankT, kSub>) != cudaSuccess) return c.fail_cuda("k_tail smem attribute");
   k_tail<RankT, kSub><<<1, 1024, smem, c.stream>>>(c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(),
                                                    c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-                                                   c.d_order.as<int32_t>(), c.d_match.as<int32_t>(), c.n, round, only_mode, kCoopChains);
+                                                   men_order(c), c.d_match.as<int32_t>(), c.n, round, only_mode, kCoopChains);
   c.launches++;
   int rc = c.check_launch("k_tail");
   if (rc) return rc;
@@ -976,7 +997,7 @@ int reserve_buffers(Ctx &c, int32_t n) {
   int rc = c.d_ctrl.ensure(zero_bytes(n));
   if (!rc) rc = init_buffers(c);
   if (!rc) rc = c.d_rankT.ensure(rank_matrix_bytes(c));
-  if (!rc) rc = order_buffers(c);
+  if (!rc && ordered(c)) rc = order_buffers(c);
   if (!rc && in_rounds(c)) rc = c.d_round.ensure(round_bytes(n));
   if (!rc && c.rank_bytes == 2 && !in_rounds(c)) rc = c.d_pr.ensure(static_cast<size_t>(n) * n * 2);
   if (!rc && c.query_ok && n <= kTailMaxN) rc = c.d_tail.ensure(tail_bytes(n));

@@ -46,6 +46,7 @@ enum Gate : int {
   kGateModeRank = 2,   // round 0 in rank mode
   kGateModeQuery = 3,  // round 0 in query mode
   kGateRetry = 4,      // the rank-mode round after a query-mode abort
+  kGateOrder = 5,      // round 0 in rank mode, but not through the filtered bulk
   kGateNoRank = 6,     // the checker after a solve that built no rank matrix
 };
 
@@ -58,6 +59,7 @@ __device__ __forceinline__ bool gate_open(int gate, const Control *c) {
     case kGateMain: return true;
     case kGateModeRank: return ld_volatile_s32(&c->mode) == kModeRank;
     case kGateModeQuery: return ld_volatile_s32(&c->mode) == kModeQuery;
+    case kGateOrder: return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->use_filter);
     case kGateRetry: return ld_volatile_s32(&c->retry) != 0;
     default: return false;
   }
@@ -916,7 +918,8 @@ __global__ void __launch_bounds__(1024) k_wdistinct(const int32_t *__restrict__ 
   }
 }
 
-template <typename RankT, int kMaxSub, bool kFilter = false>
+// kOrdered: rank-mode men start in `order` (round_kernels.cuh), else as numbered.
+template <typename RankT, int kMaxSub, bool kFilter = false, bool kOrdered = false>
 __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
     k_bulk(const int32_t *__restrict__ pref_m, const RankT *__restrict__ rank, const uint32_t *__restrict__ prefix,
            int K, unsigned long long *bid, Control *ctrl, int2 *tail_queue, const int32_t *__restrict__ order, int n,
@@ -966,7 +969,7 @@ __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
       if (lane == 0 && ld_relaxed_s32(&ctrl->free_count) > tail_threshold) v = atomicAdd(&ctrl->next_man, 1);
       v = __shfl_sync(kFullMask, v, 0);
       if (v >= n) break;
-      m = query ? v : __ldg(order + v);
+      m = !kOrdered || query ? v : __ldg(order + v);
       pos = 0;
       S = 1;
     }
@@ -1155,7 +1158,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
         pos = e.y;
       } else {
         m = first_unstarted + (i - queued);
-        if (!query) m = __ldg(order + m);
+        if (!query && order) m = __ldg(order + m);
         pos = 0;
       }
       S = 1;
