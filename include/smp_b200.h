@@ -106,12 +106,14 @@ typedef struct smp_cfg {
   int32_t prefix_k;        /* width of the per-man (woman, rank) prefix; 0 = auto,  */
                            /* -1 = none                                             */
   int32_t tail_threshold;  /* free men at which the single-CTA tail takes over;     */
-                           /* 0 = auto, -1 = never                                  */
+                           /* 0 = auto, -1 = never (and no rank mode in rounds)     */
   int32_t bulk_window;     /* widest look-ahead of the all-SM kernel, in choices    */
-                           /* per warp step (32, 64, 128, 256); 0 = auto            */
+                           /* per warp step (32, 64, 128, 256); 0 = auto.  Rank     */
+                           /* mode in rounds (uint16 ranks, n up to 38000) has none */
   uint64_t hbm_budget;     /* bytes the batch / serving paths may hold resident;    */
                            /* 0 = 64 GiB                                            */
-  int32_t tail_window;     /* the same for the tail kernel; 0 = auto                */
+  int32_t tail_window;     /* the same for the tail kernel of int32 ranks; 0 = auto */
+                           /* (uint16 ranks have tails without a window)            */
   int32_t mode;            /* 0 = auto, 1 = the men's rank-matrix mode only         */
   int32_t rank_bytes;      /* bytes per rank-matrix entry: 0 = auto (2 up to        */
                            /* n = 65535, else 4), 4 = int32 ranks at any n (the     */

@@ -778,7 +778,7 @@ int enqueue_post(Ctx &c) {
   if (rc) return rc;
   const int grid = std::max(1, std::min(c.sm_count * 4, (n + 255) / 256));
   k_match<<<grid, 256, 0, c.stream>>>(c.pref_m, c.d_bid.as<unsigned long long>(), c.d_match.as<int32_t>(), nullptr, n,
-                                      c.d_ctrl.as<Control>());
+                                      c.d_ctrl.as<Control>(), c.pass == kPassQuery ? kModeQuery : -1);
   c.launches++;
   return c.check_launch("k_match");
 }
@@ -1056,10 +1056,12 @@ int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t 
 // keep their gates, so the device still decides what runs.
 //   The checker (SMP_F_CHECK) must see the final matching: a synchronous solve
 // runs it after its passes, the others enqueue it behind the fully gated
-// pipeline, in one pass.  So do a disabled tail and a configured tail window
-// (whose tail kernel serves either mode), and int32 ranks with the checker,
-// which reads them.  (Checked solves in the gated pipeline: uniform n = 1500
-// 0.49 ms for 0.28 in passes, congested n = 6000 3.1 for 0.52.)
+// pipeline, in one pass.  So do int32 ranks with the checker, which reads them.
+// (Checked solves in the gated pipeline: uniform n = 1500 0.49 ms for 0.28 in
+// passes, congested n = 6000 3.1 for 0.52.)  A tail that is configured away keeps
+// the gated pipeline too: correlated n = 97 / 500 190 and 282 us, 211 and 303 to
+// 324 in passes.  Where n is too large for one the passes gain: n = 40000 perfect
+// 0.17 -> 0.12 ms, congested 19.5 -> 2.3.
 
 namespace {
 
@@ -1159,8 +1161,7 @@ namespace {
 // that only the larger pipelines heed.
 bool solve_is_small(const Ctx &c, uint32_t flags) {
   return c.n >= 1 && c.n <= kSmallMaxN && small_smem(c.n) + 256 <= c.smem_optin && c.prefix_k_cfg == 0 &&
-         c.tail_threshold_cfg == 0 && c.bulk_window_cfg == 0 && c.tail_window_cfg == 0 && c.mode_cfg == 0 &&
-         c.rank_bytes_cfg == 0 && !(flags & (SMP_F_CHECK | SMP_F_VALIDATE));
+         c.tail_threshold_cfg == 0 && c.bulk_window_cfg == 0 && c.mode_cfg == 0 && c.rank_bytes_cfg == 0 && !(flags & (SMP_F_CHECK | SMP_F_VALIDATE));
 }
 
 int enqueue_small(Ctx &c, int32_t *match_out, uint32_t flags) {
@@ -1188,7 +1189,7 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
     plan(c);
   }
   c.check_after = (flags & SMP_F_CHECK) && c.synchronous && n <= kU16MaxN;
-  if (((flags & SMP_F_CHECK) && !c.check_after) || !(c.tail_threshold > 0) || c.tail_window_cfg > 0) {
+  if (((flags & SMP_F_CHECK) && !c.check_after) || c.tail_threshold_cfg < 0) {
     c.check_after = false;
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }

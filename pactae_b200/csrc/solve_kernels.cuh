@@ -1577,14 +1577,16 @@ __global__ void k_retry_reset(unsigned long long *bid, int n, Control *ctrl) {
 }
 
 // ---------------------------------------------------------------------------
-// Matching from the global bid words (used when no tail kernel runs).
+// Matching from the global bid words (used when no tail kernel runs).  only_mode
+// >= 0: after proposals enqueued for that mode alone.
 // ---------------------------------------------------------------------------
 __global__ void k_match(const int32_t *__restrict__ pref_m, const unsigned long long *__restrict__ bid,
-                        int32_t *match, int32_t *also, int n, Control *ctrl) {
+                        int32_t *match, int32_t *also, int n, Control *ctrl, int only_mode = -1) {
   if (ld_volatile_s32(&ctrl->perfect)) {
     write_perfect(pref_m, match, n, ctrl, also);
     return;
   }
+  if (only_mode >= 0 && (ld_volatile_s32(&ctrl->mode) != only_mode || ld_volatile_s32(&ctrl->retry))) return;
   if (ld_volatile_s32(&ctrl->status)) return;
   unsigned long long props = 0;
   const int stride = gridDim.x * blockDim.x;
