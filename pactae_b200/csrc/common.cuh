@@ -35,7 +35,9 @@ struct Control {
   int32_t allow_query;    // host switch: 1 if the query mode may be chosen
   int32_t blocks_done;    // precheck: blocks that finished (the last one decides)
   int32_t distinct;       // precheck: number of distinct first choices
-  int32_t distinct_w;     // k_wdistinct, k_swap_pos: distinct first choices of the women
+  int32_t distinct_w;     // rank mode: distinct first choices of the women
+  int32_t distinct_mid;   // distinct choices in the middle of the men's lists,
+  int32_t same_mid;       // and neighbours who make the same choice there
   int32_t use_filter;     // k_wdistinct: k_bulk runs with its shared partner-rank filter
   int32_t swap_fail;      // k_swap_screen: a pref_m row differs from row 0
   unsigned long long proposals;        // sum over men of (final position + 1)

@@ -243,6 +243,7 @@ struct Ctx {
   // State of the staged solve.
   int n = 0;
   bool staged = false;
+  bool lists_here = false;  // both lists are whole on the device
   const int32_t *pref_m = nullptr;  // device pointers the solve reads
   const int32_t *pref_w = nullptr;
   int K = 0;               // prefix width (0 = none)
@@ -255,6 +256,7 @@ struct Ctx {
   bool rank_valid = false;  // d_rank holds the inversion of pref_w
   bool tail_ran = false;
   bool swapped = false;  // the men share one list and the women proposed
+  bool bulk_rank = false;  // uint16 ranks, but rank mode through k_bulk and k_tail
   int phase = 0;            // 0 staged, 1 prechecked, 2 inited, 3 cored, 4 posted
   // A solve or a core has used up the precheck's state: init and core after it
   // start from the precheck again.

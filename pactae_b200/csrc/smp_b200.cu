@@ -125,6 +125,31 @@ void plan(Ctx &c) {
   c.tail_threshold_rank = c.tail_threshold_cfg > 0 ? c.tail_threshold_cfg : kDefaultRankTailThreshold;
 }
 
+// Rank mode runs in rounds (round_kernels.cuh) when the ranks are uint16 and
+// one SM holds the bids; else through k_bulk.
+bool rounds_fit(const Ctx &c) { return c.rank_bytes == 2 && c.tail_threshold > 0; }
+bool in_rounds(const Ctx &c) { return rounds_fit(c) && !c.bulk_rank; }
+// The rounds lose to k_bulk, k_tail and k_tail_coop where the men's lists are alike
+// (at most n / 3 distinct choices in the middle of them) and the women's are not (at
+// least n / 4 distinct first choices): no starting order helps, a man who starts
+// displaces others all down the list, and one SM resolves n ln n displacements
+// through lists that are soon old where k_bulk has all SMs.  Women uniform, men
+// correlated, n = 5000 / 12000 / 24000, sigma 0.01: rounds 2.3, 7.3 and 20.3 ms,
+// bulk 0.9, 2.4, 6.3; sigma 0.05 2.3, 6.9, 18.1 and 1.5, 4.0, 9.1; sigma 0.2 (mid
+// choices 0.5 n) 1.8, 5.5, 14.1 and 3.8, 13.8, 29; at n = 1500 / 1000, sigma 0.05,
+// 659 and 442 us against 558 and 450.  Where most men have the very same list
+// the filtered bulk serves them, and pays from a larger n on: one man off, n = 2000
+// / 2560 / 12000 / 24000: 0.91, 1.19, 7.1, 17.9 ms and 0.95, 1.16, 4.4, 9.7; a
+// fiftieth of 5000 2.3 and 2.1.
+constexpr int kBulkRankMinN = 1280;
+constexpr int kBulkSameMinN = 2304;
+bool men_mostly_same(const Ctx &c) { return 4ll * c.h_ctrl->same_mid >= c.n; }
+bool bulk_rank_pays(const Ctx &c) {
+  const Control &h = *c.h_ctrl;
+  return rounds_fit(c) && 4ll * h.distinct_w >= c.n && 3ll * h.distinct_mid <= c.n &&
+         c.n >= (men_mostly_same(c) ? kBulkSameMinN : kBulkRankMinN);
+}
+
 // What a solve needs zeroed, in one buffer and one reset: the control block,
 // the query buckets' counts and the precheck's bitmap.
 constexpr size_t kCtrlBytes = (sizeof(Control) + 255) & ~static_cast<size_t>(255);
@@ -150,22 +175,41 @@ int enqueue_precheck(Ctx &c, bool allow_perfect) {
   return c.check_launch("k_precheck");
 }
 
+// The statistics bulk_rank_pays and the women's proposals go by, where no query
+// pass counts them (k_qscatter).  men: their lists are on the device too.
+int enqueue_alike(Ctx &c, bool men) {
+  k_alike<<<std::max(1, std::min(c.sm_count, (c.n + 255) / 256)), 256, 0, c.stream>>>(
+      men ? c.pref_m : nullptr, c.pref_w, c.n, reinterpret_cast<uint32_t *>(qcnt_of(c)), c.d_ctrl.as<Control>());
+  c.launches++;
+  return c.check_launch("k_alike");
+}
+
+// Sends the rank mode through k_bulk where that pays, by the control block read
+// back; its filtered variant as k_wdistinct would, and where most men have the
+// same list (a fiftieth of 24000 off: 9.4 ms filtered, 13.8 not; correlated men, sigma
+// 0.05: 9.6 and 9.1).
+int choose_rank_path(Ctx &c) {
+  c.bulk_rank = bulk_rank_pays(c);
+  const bool filter = c.h_ctrl->distinct <= kFilterMaxDistinct || men_mostly_same(c);
+  if (c.bulk_rank && filter &&  // (not zero for the kernels: the word was zero)
+      cudaMemsetAsync(&c.d_ctrl.as<Control>()->use_filter, 1, 1, c.stream) != cudaSuccess)
+    return c.fail_cuda("filter flag");
+  return SMP_OK;
+}
+
 // Entries per row of the rank matrices: uint16 rows are padded to 16 bytes.
 size_t rank_ld(const Ctx &c) {
   return c.rank_bytes == 2 ? (static_cast<size_t>(c.n) + 7) & ~static_cast<size_t>(7) : static_cast<size_t>(c.n);
 }
 size_t rank_matrix_bytes(const Ctx &c) { return static_cast<size_t>(c.n) * rank_ld(c) * c.rank_bytes; }
 
-// Rank mode runs in rounds (round_kernels.cuh) when the ranks are uint16 and
-// one SM holds the bids; else through k_bulk.
-bool in_rounds(const Ctx &c) { return c.rank_bytes == 2 && c.tail_threshold > 0; }
 
 // The men start by popularity (k_order_*) in the rounds, and in k_bulk from this
 // n on, unless k_wdistinct has chosen its filtered variant: below it the two launches cost more than they save (rank mode without a
 // tail, correlated n = 500 / 1500 / 6000: 303, 453 and 1737 us without, 321, 496
 // and 1793 with; n = 40000 25.2 and 24.7 ms, both sides one list 206 and 69).
 constexpr int kOrderMinN = 8192;
-bool ordered(const Ctx &c) { return in_rounds(c) || c.n >= kOrderMinN; }
+bool ordered(const Ctx &c) { return in_rounds(c) || (!c.bulk_rank && c.n >= kOrderMinN); }
 bool filter_fits(const Ctx &c) { return sizeof(uint32_t) * static_cast<size_t>(c.n) + 1024 <= c.smem_optin; }
 const int32_t *men_order(const Ctx &c) { return ordered(c) ? c.d_order.as<int32_t>() : nullptr; }
 
@@ -236,6 +280,12 @@ int order_buffers(Ctx &c) {
   return rc ? rc : c.d_score.ensure(sizeof(uint32_t) * static_cast<size_t>(c.n));
 }
 
+int enqueue_wdistinct(Ctx &c) {
+  k_wdistinct<<<1, 1024, sizeof(uint32_t) * ((c.n + 31) / 32), c.stream>>>(c.pref_w, c.n, c.d_ctrl.as<Control>());
+  c.launches++;
+  return c.check_launch("k_wdistinct");
+}
+
 // The rank matrices a solve's proposals read: inverted (woman-major, kept for
 // the checker), the men's starting order taken from it, and transposed to
 // man-major (d_rankT); where k_bulk proposes with uint16 ranks, by position too.
@@ -243,11 +293,8 @@ int enqueue_rank(Ctx &c, int gate) {
   int rc = c.d_rankT.ensure(rank_matrix_bytes(c));
   if (!rc && ordered(c)) rc = order_buffers(c);
   if (!rc) rc = enqueue_invert_any(c, gate);
-  if (!rc && !in_rounds(c) && gate == kGateModeRank && filter_fits(c)) {
-    // decides on the device which variant of k_bulk runs
-    k_wdistinct<<<1, 1024, sizeof(uint32_t) * ((c.n + 31) / 32), c.stream>>>(c.pref_w, c.n, c.d_ctrl.as<Control>());
-    c.launches++;
-    rc = c.check_launch("k_wdistinct");
+  if (!rc && !rounds_fit(c) && gate == kGateModeRank && filter_fits(c)) {
+    rc = enqueue_wdistinct(c);  // decides on the device which variant of k_bulk runs
   }
   if (!rc && ordered(c)) rc = enqueue_order(c, gate == kGateModeRank ? kGateOrder : gate);
   if (rc) return rc;
@@ -377,7 +424,7 @@ int enqueue_query_index(Ctx &c) {
   c.qcnt_clean = false;
   const int grid = static_cast<int>(std::min<size_t>(static_cast<size_t>(c.sm_count) * 16, (total + 255) / 256));
   k_qscatter<<<grid, 256, 0, c.stream>>>(c.pref_m, n, c.K, qcap, qcnt_of(c), c.d_qlist.as<uint32_t>(),
-                                         c.d_ctrl.as<Control>());
+                                         c.d_ctrl.as<Control>(), c.lists_here ? c.pref_w : nullptr);
   c.launches++;
   return c.check_launch("k_qscatter");
 }
@@ -735,7 +782,7 @@ int enqueue_round(Ctx &c, int round) {
   if constexpr (std::is_same<RankT, int32_t>::value) {
     if (c.tail_threshold > 0) return launch_tail_window<RankT>(c, c.tail_window, round, -1);
   }
-  return SMP_OK;
+  return c.bulk_rank ? launch_tail<uint16_t, 8>(c, round, -1) : SMP_OK;
 }
 
 // Rank-mode retry round; every kernel of it returns at once unless the
@@ -873,6 +920,7 @@ void reset_progress(Ctx &c) {
   c.poll_rounds = c.poll_tail = false;
   c.round_step = c.tail_segment = 0;
   c.swapped = false;
+  c.bulk_rank = false;
 }
 
 // Per-solve state reset and plan for size n.
@@ -919,7 +967,7 @@ int do_stage(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n, ui
     c.pref_w = c.d_pref_w.as<int32_t>();
   }
   if (cudaEventRecord(c.ev[kEvStageEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
-  c.staged = true;
+  c.staged = c.lists_here = true;
   return SMP_OK;
 }
 
@@ -999,7 +1047,7 @@ int reserve_buffers(Ctx &c, int32_t n) {
   if (!rc) rc = c.d_rankT.ensure(rank_matrix_bytes(c));
   if (!rc && ordered(c)) rc = order_buffers(c);
   if (!rc && in_rounds(c)) rc = c.d_round.ensure(round_bytes(n));
-  if (!rc && c.rank_bytes == 2 && !in_rounds(c)) rc = c.d_pr.ensure(static_cast<size_t>(n) * n * 2);
+  if (!rc && c.rank_bytes == 2 && (!in_rounds(c) || n >= kBulkRankMinN)) rc = c.d_pr.ensure(static_cast<size_t>(n) * n * 2);
   if (!rc && c.query_ok && n <= kTailMaxN) rc = c.d_tail.ensure(tail_bytes(n));
   if (!rc && c.query_ok)
     rc = c.d_qlist.ensure(sizeof(uint32_t) * static_cast<size_t>(n) * query_capacity(n, c.K));
@@ -1104,7 +1152,9 @@ int enqueue_swap_screen(Ctx &c, bool men_screened) {
   if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
       cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("swap reset");
-  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl, c.pref_w, seen_of(c));
+  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl);
+  if (!c.query_ok && !rounds_fit(c)) rc = enqueue_alike(c, false);  // not counted yet
+  if (rc) return rc;
   uint16_t *near = n <= kU16MaxN ? c.d_swap_near.as<uint16_t>() : nullptr;
   if (near) k_swap_near<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_w, near, n);
   // the women's proposals beside the screen, which leaves a CTA's place on each
@@ -1214,7 +1264,9 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
   if (rc) return rc;
   c.pass = c.query_ok ? kPassQuery : kPassPrecheck;
   c.poll_tail = true;
-  return c.query_ok ? enqueue_pass_mode(c, kModeQuery) : read_control(c);
+  if (c.query_ok) return enqueue_pass_mode(c, kModeQuery);
+  if (rounds_fit(c)) rc = enqueue_alike(c, true);
+  return rc ? rc : read_control(c);
 }
 
 int solve_advance(Ctx &c, bool &more) {
@@ -1248,11 +1300,17 @@ int solve_advance(Ctx &c, bool &more) {
     const int rc = c.rank_bytes == 2 ? enqueue_retry_round<uint16_t>(c) : enqueue_retry_round<int32_t>(c);
     return rc ? rc : enqueue_pass_end(c);
   }
-  // one first choice for every man: perhaps one list for every man
+  // one first choice for every man: perhaps one list for every man (and if a
+  // query pass has looked, one choice in the middle)
   if (c.pass != kPassScreen && !h.perfect && h.mode == kModeRank && h.distinct == 1 && c.n >= 2 && c.mode_cfg == 0 &&
-      swap_screen_fits(c)) {
+      (!queried || h.same_mid == c.n) && swap_screen_fits(c)) {
     c.pass = kPassScreen;
     return enqueue_swap_screen(c, false);
+  }
+  if (!h.perfect) {
+    const int rc = choose_rank_path(c);
+    if (rc) return rc;
+    c.poll_rounds = in_rounds(c);
   }
   c.pass = kPassLast;
   if (!h.perfect) return enqueue_pass_mode(c, h.mode);
@@ -1289,7 +1347,8 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
   if (!swap_screen_fits(c)) return SMP_OK;
   c.pass_flags = flags;
   c.pass_match = match_out;
-  int rc = enqueue_swap_screen(c, true);
+  int rc = enqueue_alike(c, false);
+  if (!rc) rc = enqueue_swap_screen(c, true);
   if (!rc) rc = c.sync("swap screen");
   if (rc) return rc;
   swapped = c.h_ctrl->status || !c.h_ctrl->swap_fail;
@@ -1636,6 +1695,7 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
     return c.fail_cuda("pref_m prefix copy");
   if (cudaEventRecord(c.ev[kEvStageEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   c.staged = true;
+  c.lists_here = false;
   rc = enqueue_precheck(c, (flags & SMP_F_NO_PRECHECK) == 0);
   if (!rc) rc = read_control(c);
   if (!rc) rc = c.sync("precheck");
@@ -1695,6 +1755,13 @@ int solve_streamed(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t
       rc = c.fail_cuda("event");
     if (!rc && shared && !swapped) rc = solve_swapped(c, flags, match_out, swapped);
     const bool perfect = c.h_ctrl->perfect != 0;
+    if (!rc && !swapped && !perfect && rounds_fit(c)) {
+      if (!shared) rc = enqueue_alike(c, true);  // the lists are here now
+      if (!rc) rc = read_control(c);
+      if (!rc) rc = c.sync("lists");
+      if (!rc) rc = choose_rank_path(c);
+      c.poll_rounds = in_rounds(c);
+    }
     if (perfect) c.tail_ran = false;  // k_match writes the first choices
     if (!rc && !swapped && !perfect) rc = enqueue_init(c);
     if (!rc && !swapped && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
@@ -1897,6 +1964,7 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
   c.spent = false;
   if (cudaEventRecord(c.ev[kEvStageEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   int rc = enqueue_precheck(c, true);
+  if (!rc && rounds_fit(c) && c.lists_here) rc = enqueue_alike(c, true);
   if (!rc) rc = read_control(c);
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
@@ -1906,7 +1974,9 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
   c.stats.precheck_ms = elapsed(c, kEvStageEnd, kEvPrecheckEnd);
   if (is_perfect) *is_perfect = c.h_ctrl->perfect;
   // init and core enqueue this mode's kernels only
-  c.known_mode = in_rounds(c) && !c.h_ctrl->status && !c.h_ctrl->perfect ? c.h_ctrl->mode : -1;
+  c.known_mode = rounds_fit(c) && !c.h_ctrl->status && !c.h_ctrl->perfect ? c.h_ctrl->mode : -1;
+  if (c.known_mode == kModeRank) rc = choose_rank_path(c);
+  if (rc) return rc;
   return control_status(c);
 }
 
@@ -1940,7 +2010,7 @@ int smp_b200_core(smp_ctx *ctx) {
   DeviceGuard g(c.device);
   if (cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   const bool query = c.known_mode == kModeQuery;
-  c.poll_tail = c.poll_rounds = c.known_mode >= 0;
+  c.poll_tail = c.poll_rounds = c.known_mode >= 0 && !c.bulk_rank;
   c.round_step = c.tail_segment = 0;  // this call waits for what it enqueues itself
   int rc = enqueue_core(c);
   for (bool more = true; !rc && more;) {

@@ -87,6 +87,41 @@ __device__ __forceinline__ bool any_unset<int32_t>(uint4 v) {
   return v.x == 0xFFFFFFFFu || v.y == 0xFFFFFFFFu || v.z == 0xFFFFFFFFu || v.w == 0xFFFFFFFFu;
 }
 
+// How alike the lists of a rank-mode instance are: the distinct first choices of
+// the women, and the distinct entries in the middle of the men's lists (not with
+// pref_m = nullptr), in two bitmaps of zeros one after the other; and how many men
+// have the same there as the man after them.
+__device__ __forceinline__ void count_alike(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
+                                            int n, uint32_t *bitmaps, Control *ctrl) {
+  unsigned women = 0, mid = 0, same = 0;
+  const auto fresh = [&](uint32_t *bitmap, int v) {
+    const uint32_t bit = 1u << (v & 31);
+    return static_cast<unsigned>(v) < static_cast<unsigned>(n) && !(atomicOr(bitmap + (v >> 5), bit) & bit);
+  };
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const size_t row = static_cast<size_t>(r) * n;
+    const int w = __ldg(pref_w + row);
+    const int v = pref_m ? __ldg(pref_m + row + n / 2) : -1;
+    const int u = pref_m ? __ldg(pref_m + (r + 1 < n ? row + n : 0) + n / 2) : -2;
+    women += fresh(bitmaps, w);
+    mid += fresh(bitmaps + ((n + 31) >> 5), v);
+    same += v == u;
+  }
+  women = __reduce_add_sync(kFullMask, women);
+  mid = __reduce_add_sync(kFullMask, mid);
+  same = __reduce_add_sync(kFullMask, same);
+  if ((threadIdx.x & 31) == 0) {
+    if (women) atomicAdd(&ctrl->distinct_w, static_cast<int>(women));
+    if (mid) atomicAdd(&ctrl->distinct_mid, static_cast<int>(mid));
+    if (same) atomicAdd(&ctrl->same_mid, static_cast<int>(same));
+  }
+}
+
+__global__ void __launch_bounds__(256) k_alike(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
+                                               int n, uint32_t *bitmaps, Control *ctrl) {
+  if (gate_open(kGateModeRank, ctrl)) count_alike(pref_m, pref_w, n, bitmaps, ctrl);
+}
+
 // ---------------------------------------------------------------------------
 // Precheck.  Marks each man's first choice in an n-bit bitmap (seen, zeroed
 // by the host).  The last block to finish counts the distinct first choices
@@ -446,9 +481,15 @@ __global__ void __launch_bounds__(512) k_validate_rows(const int32_t *__restrict
 // bucket.  The rank matrix is never written: pref_w is read once and nothing
 // n^2-sized is stored.  qcnt is zeroed by the host.
 // ---------------------------------------------------------------------------
+// A rank-mode instance has no use for it: its lists are compared instead (pref_w
+// on the device, else nullptr).
 __global__ void k_qscatter(const int32_t *__restrict__ pref_m, int n, int K, int qcap, int32_t *__restrict__ qcnt,
-                           uint32_t *__restrict__ qlist, Control *ctrl) {
-  if (!gate_open(kGateModeQuery, ctrl)) return;
+                           uint32_t *__restrict__ qlist, Control *ctrl, const int32_t *__restrict__ pref_w) {
+  if (!gate_open(kGateModeQuery, ctrl)) {
+    if (pref_w && gate_open(kGateModeRank, ctrl))
+      count_alike(pref_m, pref_w, n, reinterpret_cast<uint32_t *>(qcnt), ctrl);
+    return;
+  }
   const size_t total = static_cast<size_t>(n) * K;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {

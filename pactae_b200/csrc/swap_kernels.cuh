@@ -28,24 +28,13 @@
 namespace smpb200 {
 
 // pos[L[r]] = r, with pos preset to -1; an entry out of range or seen twice
-// makes row 0 no permutation.  With pref_w given, distinct_w counts the women's
-// first choices in the precheck's bitmap, which holds one bit by then (the men
-// share their first choice): the count may be one too low.
-__global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl,
-                           const int32_t *__restrict__ pref_w = nullptr, uint32_t *__restrict__ seen = nullptr) {
-  unsigned firsts = 0;
+// makes row 0 no permutation.
+__global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const int w = __ldg(pref_m + r);
     if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1)
       report(ctrl, kStatusInvalidInput, w);
-    if (pref_w) {
-      const int m = __ldg(pref_w + static_cast<size_t>(r) * n);
-      const uint32_t bit = 1u << (m & 31);
-      if (static_cast<unsigned>(m) < static_cast<unsigned>(n) && !(atomicOr(seen + (m >> 5), bit) & bit)) firsts++;
-    }
   }
-  firsts = __reduce_add_sync(kFullMask, firsts);
-  if (firsts && (threadIdx.x & 31) == 0) atomicAdd(&ctrl->distinct_w, static_cast<int>(firsts));
 }
 
 // Rows t = 1 .. n-1 compare pref_m row t with row 0; rows t = n .. 2n-1
@@ -60,7 +49,7 @@ __global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restri
 // women share one list too, comparing with row 0 instead of marking: 1.96 -> 1.30.)
 __host__ __device__ constexpr size_t swap_screen_smem(int n) { return ((static_cast<size_t>(n) + 31) / 32) * 4; }
 
-// Fewer than n / 4 distinct first choices (k_swap_pos).
+// Fewer than n / 4 distinct first choices (count_alike).
 __device__ __forceinline__ bool women_alike(const Control *ctrl, int n) {
   return 4ll * ld_volatile_s32(&ctrl->distinct_w) < n;
 }
