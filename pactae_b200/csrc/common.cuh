@@ -59,6 +59,9 @@ struct Control {
   int32_t screen_ctas;    // CTAs of it that have finished
   int32_t screen_done;    // all have
   int32_t swap_out;       // match[] is written
+  // a solve in one fixed sequence (k_turn)
+  int32_t swap_try;       // the men may share one list
+  int32_t rank_bulk;      // rank mode goes through k_bulk
   int32_t tail_left;      // k_tail_q: chains that have not ended
   int32_t tail_done;      // none are left and the words are final
   int32_t check_deep;     // k_check_near: some man's wife is not among his first choices

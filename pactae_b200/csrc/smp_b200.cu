@@ -141,14 +141,7 @@ bool in_rounds(const Ctx &c) { return rounds_fit(c) && !c.bulk_rank; }
 // the filtered bulk serves them, and pays from a larger n on: one man off, n = 2000
 // / 2560 / 12000 / 24000: 0.91, 1.19, 7.1, 17.9 ms and 0.95, 1.16, 4.4, 9.7; a
 // fiftieth of 5000 2.3 and 2.1.
-constexpr int kBulkRankMinN = 1280;
-constexpr int kBulkSameMinN = 2304;
-bool men_mostly_same(const Ctx &c) { return 4ll * c.h_ctrl->same_mid >= c.n; }
-bool bulk_rank_pays(const Ctx &c) {
-  const Control &h = *c.h_ctrl;
-  return rounds_fit(c) && 4ll * h.distinct_w >= c.n && 3ll * h.distinct_mid <= c.n &&
-         c.n >= (men_mostly_same(c) ? kBulkSameMinN : kBulkRankMinN);
-}
+bool bulk_rank_pays(const Ctx &c) { return rounds_fit(c) && rank_bulk_pays(*c.h_ctrl, c.n); }
 
 // What a solve needs zeroed, in one buffer and one reset: the control block,
 // the query buckets' counts and the precheck's bitmap.
@@ -190,7 +183,7 @@ int enqueue_alike(Ctx &c, bool men) {
 // 0.05: 9.6 and 9.1).
 int choose_rank_path(Ctx &c) {
   c.bulk_rank = bulk_rank_pays(c);
-  const bool filter = c.h_ctrl->distinct <= kFilterMaxDistinct || men_mostly_same(c);
+  const bool filter = rank_bulk_filtered(*c.h_ctrl, c.n);
   if (c.bulk_rank && filter &&  // (not zero for the kernels: the word was zero)
       cudaMemsetAsync(&c.d_ctrl.as<Control>()->use_filter, 1, 1, c.stream) != cudaSuccess)
     return c.fail_cuda("filter flag");
@@ -286,18 +279,7 @@ int enqueue_wdistinct(Ctx &c) {
   return c.check_launch("k_wdistinct");
 }
 
-// The rank matrices a solve's proposals read: inverted (woman-major, kept for
-// the checker), the men's starting order taken from it, and transposed to
-// man-major (d_rankT); where k_bulk proposes with uint16 ranks, by position too.
-int enqueue_rank(Ctx &c, int gate) {
-  int rc = c.d_rankT.ensure(rank_matrix_bytes(c));
-  if (!rc && ordered(c)) rc = order_buffers(c);
-  if (!rc) rc = enqueue_invert_any(c, gate);
-  if (!rc && !rounds_fit(c) && gate == kGateModeRank && filter_fits(c)) {
-    rc = enqueue_wdistinct(c);  // decides on the device which variant of k_bulk runs
-  }
-  if (!rc && ordered(c)) rc = enqueue_order(c, gate == kGateModeRank ? kGateOrder : gate);
-  if (rc) return rc;
+int enqueue_transpose(Ctx &c, int gate) {
   const int tiles = (c.n + 63) / 64;
   const int grid = static_cast<int>(std::min<long long>(static_cast<long long>(c.sm_count) * 4,
                                                         static_cast<long long>(tiles) * tiles));
@@ -308,10 +290,12 @@ int enqueue_rank(Ctx &c, int gate) {
     k_transpose<int32_t><<<grid, 512, 0, c.stream>>>(c.d_rank.as<int32_t>(), c.d_rankT.as<int32_t>(), c.n,
                                                      c.d_ctrl.as<Control>(), gate);
   c.launches++;
-  rc = c.check_launch("k_transpose");
-  if (rc || c.rank_bytes != 2 || in_rounds(c)) return rc;
-  // uint16 ranks: k_bulk reads them by position (pr)
-  rc = c.d_pr.ensure(static_cast<size_t>(c.n) * c.n * 2);
+  return c.check_launch("k_transpose");
+}
+
+// uint16 ranks by position, which k_bulk reads.
+int enqueue_pr(Ctx &c, int gate) {
+  const int rc = c.d_pr.ensure(static_cast<size_t>(c.n) * c.n * 2);
   if (rc) return rc;
   const size_t smem = row_smem_bytes<uint16_t>(c.n);
   if (allow_dynamic_smem(c, k_pr) != cudaSuccess) return c.fail_cuda("k_pr smem attribute");
@@ -325,6 +309,20 @@ int enqueue_rank(Ctx &c, int gate) {
       c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr, c.K > 0 ? c.K : 0, c.n, c.d_ctrl.as<Control>(), gate);
   c.launches++;
   return c.check_launch("k_pr");
+}
+
+// The rank matrices a solve's proposals read: inverted (woman-major, kept for
+// the checker), the men's starting order taken from it, and transposed to
+// man-major (d_rankT); where k_bulk proposes with uint16 ranks, by position too.
+int enqueue_rank(Ctx &c, int gate) {
+  int rc = c.d_rankT.ensure(rank_matrix_bytes(c));
+  if (!rc && ordered(c)) rc = order_buffers(c);
+  if (!rc) rc = enqueue_invert_any(c, gate);
+  if (!rc && !rounds_fit(c) && gate == kGateModeRank && filter_fits(c))
+    rc = enqueue_wdistinct(c);  // decides on the device which variant of k_bulk runs
+  if (!rc && ordered(c)) rc = enqueue_order(c, gate == kGateModeRank ? kGateOrder : gate);
+  if (!rc) rc = enqueue_transpose(c, gate);
+  return rc || c.rank_bytes != 2 || in_rounds(c) ? rc : enqueue_pr(c, gate);
 }
 
 // The rounds' buffers, one allocation: candidate lists, words and positions,
@@ -360,7 +358,7 @@ RoundBufs round_bufs(const Ctx &c) {
 // (c.poll_rounds) gets kRoundExtra more and adds steps until round_done;
 // otherwise kRoundExtraBlind follow, then the last step, which ends any solve.
 constexpr int kRoundExtra = 1;
-constexpr int kRoundExtraBlind = 12;
+constexpr int kRoundExtraBlind = 2;  // (12: 20 to 30 us more whatever the lists, and no family of the generator faster)
 constexpr int kRoundMore = 8;
 
 int enqueue_round_steps(Ctx &c, int gate, int count) {
@@ -490,6 +488,8 @@ int init_buffers(Ctx &c) {
   return SMP_OK;
 }
 
+bool swap_screen_fits(const Ctx &c) { return swap_screen_smem(c.n) <= c.smem_optin; }
+
 // The stream that runs beside the context's, with its fork and join events
 // (created on first use).
 int side_stream(Ctx &c) {
@@ -525,44 +525,56 @@ int enqueue_init(Ctx &c) {
   return SMP_OK;
 }
 
+// Free women left when rank-mode men move to the one-CTA tail.
+int rank_tail_threshold(const Ctx &c) {
+  return c.tail_threshold > 0 ? std::min(c.tail_threshold, c.tail_threshold_rank) : 0;
+}
+
+template <typename RankT, int kSub>
+int launch_bulk_filtered(Ctx &c, int round) {
+  const size_t filter = sizeof(uint32_t) * static_cast<size_t>(c.n);
+  const auto kernel = k_bulk<RankT, kSub, true>;  // the women are unlike: no order helps
+  if (allow_dynamic_smem(c, kernel) !=
+      cudaSuccess)
+    return c.fail_cuda("k_bulk smem attribute");
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFilterBlock, filter) != cudaSuccess) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
+  kernel<<<c.sm_count * std::max(per_sm, 1), kFilterBlock, filter, c.stream>>>(
+      c.pref_m, proposal_ranks<RankT>(c), c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr, c.K,
+      c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(), nullptr, c.n, c.tail_threshold,
+      rank_tail_threshold(c), round, -1);
+  c.launches++;
+  return c.check_launch("k_bulk (filtered)");
+}
+
+template <typename RankT, int kSub, bool kOrdered = false>
+int launch_bulk_open(Ctx &c, int round, int only_mode) {
+  const auto kernel = k_bulk<RankT, kSub, false, kOrdered>;
+  kernel<<<resident_grid(c, kernel, 256), 256, 0, c.stream>>>(
+      c.pref_m, proposal_ranks<RankT>(c), c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr, c.K,
+      c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(), kOrdered ? men_order(c) : nullptr,
+      c.n, c.tail_threshold, rank_tail_threshold(c), round, only_mode);
+  c.launches++;
+  return c.check_launch("k_bulk");
+}
+
 template <typename RankT, int kSub>
 int launch_bulk(Ctx &c, int round) {
-  const RankT *rank = proposal_ranks<RankT>(c);
-  const uint32_t *prefix = c.K > 0 ? c.d_prefix.as<uint32_t>() : nullptr;
-  const int rank_threshold = c.tail_threshold > 0 ? std::min(c.tail_threshold, c.tail_threshold_rank) : 0;
-  if (!in_rounds(c) && round == 0 && c.known_mode != kModeQuery && filter_fits(c)) {
-    const size_t filter = sizeof(uint32_t) * static_cast<size_t>(c.n);
-    const auto kernel = k_bulk<RankT, kSub, true>;  // the women are unlike: no order helps
-    if (allow_dynamic_smem(c, kernel) !=
-        cudaSuccess)
-      return c.fail_cuda("k_bulk smem attribute");
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFilterBlock, filter) != cudaSuccess) {
-      cudaGetLastError();
-      per_sm = 1;
-    }
-    kernel<<<c.sm_count * std::max(per_sm, 1), kFilterBlock, filter, c.stream>>>(
-        c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-        nullptr, c.n, c.tail_threshold, rank_threshold, round, -1);
-    c.launches++;
-    const int rc = c.check_launch("k_bulk (filtered)");
-    if (rc) return rc;
-  }
+  int rc = SMP_OK;
+  if (!in_rounds(c) && round == 0 && c.known_mode != kModeQuery && filter_fits(c))
+    rc = launch_bulk_filtered<RankT, kSub>(c, round);
+  if (rc) return rc;
   // Query-mode men start as they are numbered; the ordered variant's take-up took
   // 5 % of a query-mode bulk (n = 6000 without a tail: 1.85 and 1.95 ms).
-  const auto launch = [&](auto kernel, int only_mode) {
-    kernel<<<resident_grid(c, kernel, 256), 256, 0, c.stream>>>(
-        c.pref_m, rank, prefix, c.K, c.d_bid.as<unsigned long long>(), c.d_ctrl.as<Control>(), c.d_tailq.as<int2>(),
-        men_order(c), c.n, c.tail_threshold, rank_threshold, round, only_mode);
-    c.launches++;
-    return c.check_launch("k_bulk");
-  };
-  if (in_rounds(c)) return launch(k_bulk<RankT, kSub>, kModeQuery);
-  if (!ordered(c)) return launch(k_bulk<RankT, kSub>, c.known_mode);
-  int rc = SMP_OK;
+  if (in_rounds(c)) return launch_bulk_open<RankT, kSub>(c, round, kModeQuery);
+  if (!ordered(c)) return launch_bulk_open<RankT, kSub>(c, round, c.known_mode);
   const bool query = round == 0 && c.query_ok;
-  if (query && c.known_mode != kModeRank) rc = launch(k_bulk<RankT, kSub>, kModeQuery);
-  if (!rc && c.known_mode != kModeQuery) rc = launch(k_bulk<RankT, kSub, false, true>, query ? kModeRank : c.known_mode);
+  if (query && c.known_mode != kModeRank) rc = launch_bulk_open<RankT, kSub>(c, round, kModeQuery);
+  if (!rc && c.known_mode != kModeQuery)
+    rc = launch_bulk_open<RankT, kSub, true>(c, round, query ? kModeRank : c.known_mode);
   return rc;
 }
 
@@ -1058,6 +1070,63 @@ int reserve_buffers(Ctx &c, int32_t n) {
   return rc;
 }
 
+namespace {
+
+// Init and core of a solve in one fixed sequence, uint16 ranks: the query mode, then
+// (k_turn) one rank mode for its retry and for the instances that start in it --
+// men who share one list, k_bulk, or rounds.  What the device does not take is an
+// empty launch, 2 to 3 us.  (Routed in a batch, n = 600 uniform / 9001 congested /
+// correlated: 269 us, 4.7 ms and 1.73 ms with a rank mode of its own for the retry,
+// twelve spare steps and shared lists left to the rounds; 173 us, 0.74 and 1.62 so.)
+int enqueue_fixed(Ctx &c) {
+  const int n = c.n;
+  Control *ctrl = c.d_ctrl.as<Control>();
+  int rc = init_buffers(c);
+  if (!rc) rc = swap_buffers(c);
+  if (!rc) rc = enqueue_query(c);
+  if (rc) return rc;
+  if (cudaEventRecord(c.ev[kEvInvertEnd], c.stream) != cudaSuccess ||
+      cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess)
+    return c.fail_cuda("event");
+  c.tail_ran = true;
+  rc = enqueue_bulk<uint16_t>(c, 0);
+  if (!rc && cudaEventRecord(c.ev[kEvBulkEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+  if (!rc) rc = launch_tail_query(c);
+  if (rc) return rc;
+  const bool share = c.mode_cfg == 0 && swap_screen_fits(c);
+  const bool bulk = n >= kBulkRankMinN;
+  int32_t *pos = c.d_swap_pos.as<int32_t>();
+  unsigned long long *bid = c.d_bid.as<unsigned long long>();
+  k_turn<<<1, 1024, 0, c.stream>>>(c.pref_m, bid, pos, n, ctrl, share, bulk);
+  c.launches++;
+  rc = c.check_launch("k_turn");
+  if (!rc && share) {
+    if (allow_dynamic_smem(c, k_swap_screen) != cudaSuccess) return c.fail_cuda("k_swap_screen smem attribute");
+    const int screen = std::min(2 * n - 1, c.sm_count * 7);
+    k_swap_screen<<<screen, 256, swap_screen_smem(n), c.stream>>>(c.pref_m, c.pref_w, n, ctrl, 1, screen, 1);
+    k_swap_gs<<<c.sm_count * 4, 256, 0, c.stream>>>(c.pref_m, c.pref_w, pos, bid, n, ctrl, nullptr, n, nullptr, nullptr,
+                                                    0, 2, nullptr);
+    k_swap_outcome<<<std::max(1, std::min(c.sm_count, (n + 255) / 256)), 256, 0, c.stream>>>(
+        c.pref_m, c.pref_w, bid, c.d_match.as<int32_t>(), n, ctrl, 1);
+    c.launches += 3;
+    rc = c.check_launch("k_swap_outcome");
+  }
+  if (!rc) rc = c.d_rankT.ensure(rank_matrix_bytes(c));
+  if (!rc) rc = order_buffers(c);
+  if (!rc) rc = enqueue_invert_any(c, kGateModeRank);
+  if (!rc) rc = enqueue_order(c, kGateRounds);
+  if (!rc) rc = enqueue_transpose(c, kGateModeRank);
+  if (!rc && bulk) {
+    rc = enqueue_pr(c, kGateBulk);
+    if (!rc) rc = launch_bulk_filtered<uint16_t, 8>(c, 0);
+    if (!rc) rc = launch_bulk_open<uint16_t, 8>(c, 0, kOnlyRankBulk);
+    if (!rc) rc = launch_tail<uint16_t, 8>(c, 0, kOnlyRankBulk);
+  }
+  return rc ? rc : enqueue_rounds(c, kGateRounds);
+}
+
+}  // namespace
+
 // Enqueues a whole solve on c.stream with no host round trip (stage,
 // precheck, init, core, post, the match copy, optional check, control
 // readback).  The caller synchronises the stream, then calls solve_finish.
@@ -1069,9 +1138,13 @@ int solve_enqueue(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t 
   rc = enqueue_precheck(c, (flags & SMP_F_NO_PRECHECK) == 0);
   if (!rc && (flags & SMP_F_VALIDATE)) rc = enqueue_validate(c);
   if (!rc && cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (!rc) rc = enqueue_init(c);
-  if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
-  if (!rc) rc = enqueue_core(c);
+  if (!rc && rounds_fit(c) && c.query_ok) {
+    rc = enqueue_fixed(c);
+  } else {
+    if (!rc) rc = enqueue_init(c);
+    if (!rc && cudaEventRecord(c.ev[kEvInitEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
+    if (!rc) rc = enqueue_core(c);
+  }
   if (!rc && cudaEventRecord(c.ev[kEvCoreEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
   if (!rc) rc = enqueue_post(c);
   if (!rc && (flags & SMP_F_DEVICE_PTRS)) rc = copy_match_out(c, match_out, true);
@@ -1137,7 +1210,6 @@ int enqueue_pass_mode(Ctx &c, int mode) {
 // screen checks that on all SMs (and that pref_w's rows are permutations).
 constexpr int kSwapBeside = 1;       // CTAs per SM of the proposals beside the screen
 constexpr int kSwapBesideAlike = 2;  // where the women's lists are alike
-bool swap_screen_fits(const Ctx &c) { return swap_screen_smem(c.n) <= c.smem_optin; }
 
 int enqueue_swap_screen(Ctx &c, bool men_screened) {
   const int n = c.n;

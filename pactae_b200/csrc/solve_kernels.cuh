@@ -47,6 +47,8 @@ enum Gate : int {
   kGateModeQuery = 3,  // round 0 in query mode
   kGateRetry = 4,      // the rank-mode round after a query-mode abort
   kGateOrder = 5,      // round 0 in rank mode, but not through the filtered bulk
+  kGateRounds = 7,     // a fixed sequence's rank mode, in rounds
+  kGateBulk = 8,       // through k_bulk
   kGateNoRank = 6,     // the checker after a solve that built no rank matrix
 };
 
@@ -57,9 +59,13 @@ __device__ __forceinline__ bool gate_open(int gate, const Control *c) {
   if (perfect || ld_volatile_s32(&c->status)) return false;
   switch (gate) {
     case kGateMain: return true;
-    case kGateModeRank: return ld_volatile_s32(&c->mode) == kModeRank;
+    case kGateModeRank: return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->swap_out);
     case kGateModeQuery: return ld_volatile_s32(&c->mode) == kModeQuery;
     case kGateOrder: return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->use_filter);
+    case kGateRounds:
+    case kGateBulk:
+      return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->swap_out) &&
+             (ld_volatile_s32(&c->rank_bulk) != 0) == (gate == kGateBulk);
     case kGateRetry: return ld_volatile_s32(&c->retry) != 0;
     default: return false;
   }
@@ -924,6 +930,8 @@ __global__ void __launch_bounds__(256) k_widen16_rows(const uint16_t *__restrict
 // per SM); else GlobalBids.  Both variants are enqueued and the device runs
 // the one k_wdistinct chose (ctrl->use_filter).
 constexpr int kFilterBlock = 768;
+// (only_mode of k_bulk and k_tail, beside the modes and -1)
+constexpr int kOnlyRankBulk = 2;
 constexpr int kFilterMaxDistinct = 16;
 
 // ---------------------------------------------------------------------------
@@ -974,7 +982,7 @@ __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
     // barrier.
     __shared__ int s_go;
     if (threadIdx.x == 0)
-      s_go = round == 0 && ld_volatile_s32(&ctrl->use_filter) && gate_open(kGateMain, ctrl) &&
+      s_go = round == 0 && ld_volatile_s32(&ctrl->use_filter) && gate_open(kGateModeRank, ctrl) &&
              !ld_volatile_s32(&ctrl->retry);
     __syncthreads();
     if (!s_go) return;
@@ -985,7 +993,9 @@ __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
     if (round == 0 && ld_volatile_s32(&ctrl->retry)) return;  // a query bucket overflowed
     if (round == 0 && ld_volatile_s32(&ctrl->use_filter)) return;  // the filtered variant runs
     // enqueued for one mode only (the host has not read the precheck yet)
-    if (round == 0 && only_mode >= 0 && ld_volatile_s32(&ctrl->mode) != only_mode) return;
+    if (round == 0 && only_mode == kOnlyRankBulk && !gate_open(kGateBulk, ctrl)) return;
+    if (round == 0 && (only_mode == kModeRank || only_mode == kModeQuery) && ld_volatile_s32(&ctrl->mode) != only_mode)
+      return;
   }
   const bool query = round == 0 && ld_volatile_s32(&ctrl->mode) == kModeQuery;
   // Free women left when the men move to the one-CTA tail: rank-mode
@@ -1138,8 +1148,7 @@ __device__ __forceinline__ void write_perfect(const int32_t *__restrict__ pref_m
 // proposal count.  In query mode a man beyond his prefix sets the retry flag
 // and every warp stops.
 // round 0: gate Main (and no retry pending); round 1: gate Retry.
-// only_mode >= 0 runs the kernel only when the precheck chose that mode, so
-// the host can enqueue a narrow and a wide variant and the device keeps one.
+// only_mode = kOnlyRankBulk: in a fixed sequence, where k_turn chose k_bulk.
 // ---------------------------------------------------------------------------
 template <typename RankT, int kMaxSub>
 __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pref_m,
@@ -1150,7 +1159,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
                                                   const int32_t *__restrict__ order,
                                                   int32_t *__restrict__ match, int n, int round,
                                                   int only_mode, int coop_chains) {
-  if (only_mode >= 0 && round == 0 && ld_volatile_s32(&ctrl->mode) != only_mode) return;
+  if (only_mode == kOnlyRankBulk && !gate_open(kGateBulk, ctrl)) return;
   if (round == 0 && ld_volatile_s32(&ctrl->perfect)) {
     write_perfect(pref_m, match, n, ctrl);
     return;
@@ -1599,8 +1608,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail_qw(const int32_t *__restrict__
 // Start of the rank-mode retry round: every woman free again, counters reset.
 // One CTA.
 // ---------------------------------------------------------------------------
-__global__ void k_retry_reset(unsigned long long *bid, int n, Control *ctrl) {
-  if (!gate_open(kGateRetry, ctrl)) return;
+__device__ __forceinline__ void retry_reset(unsigned long long *bid, int n, Control *ctrl) {
   for (int w = threadIdx.x; w < n; w += blockDim.x) bid[w] = kFree;
   if (threadIdx.x == 0) {
     ctrl->mode = kModeRank;
@@ -1614,6 +1622,50 @@ __global__ void k_retry_reset(unsigned long long *bid, int n, Control *ctrl) {
     ctrl->tail_hops = 0;
     ctrl->coop_count = 0;
     ctrl->use_filter = 0;
+  }
+}
+
+__global__ void k_retry_reset(unsigned long long *bid, int n, Control *ctrl) {
+  if (gate_open(kGateRetry, ctrl)) retry_reset(bid, n, ctrl);
+}
+
+// What the rank mode of an instance goes through (bulk_rank_pays in smp_b200.cu says
+// why and what was measured).
+constexpr int kBulkRankMinN = 1280;
+constexpr int kBulkSameMinN = 2304;
+__host__ __device__ __forceinline__ bool men_mostly_same(const Control &c, int n) { return 4ll * c.same_mid >= n; }
+__host__ __device__ __forceinline__ bool rank_bulk_pays(const Control &c, int n) {
+  return 4ll * c.distinct_w >= n && 3ll * c.distinct_mid <= n &&
+         n >= (men_mostly_same(c, n) ? kBulkSameMinN : kBulkRankMinN);
+}
+__host__ __device__ __forceinline__ bool rank_bulk_filtered(const Control &c, int n) {
+  return c.distinct <= kFilterMaxDistinct || men_mostly_same(c, n);
+}
+
+// The turn of a fixed sequence from the query mode to the rank mode, one CTA: the
+// retry's reset, or which way a rank-mode instance takes; where the men may share
+// one list, pos = its inverse (k_swap_pos).
+__global__ void __launch_bounds__(1024) k_turn(const int32_t *__restrict__ pref_m, unsigned long long *bid, int32_t *pos,
+                                               int n, Control *ctrl, int may_share, int may_bulk) {
+  if (!gate_open(kGateMain, ctrl)) return;
+  if (ld_volatile_s32(&ctrl->retry)) {
+    retry_reset(bid, n, ctrl);
+    return;
+  }
+  if (ld_volatile_s32(&ctrl->mode) != kModeRank) return;
+  const bool share = may_share && n >= 2 && ctrl->distinct == 1 && ctrl->same_mid == n;
+  if (threadIdx.x == 0) {
+    ctrl->swap_try = share;
+    ctrl->rank_bulk = may_bulk && rank_bulk_pays(*ctrl, n);
+    ctrl->use_filter = ctrl->rank_bulk && rank_bulk_filtered(*ctrl, n);
+  }
+  if (!share) return;
+  for (int w = threadIdx.x; w < n; w += 1024) pos[w] = -1;
+  __syncthreads();
+  for (int r = threadIdx.x; r < n; r += 1024) {
+    const int w = __ldg(pref_m + r);
+    if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1)
+      report(ctrl, kStatusInvalidInput, w);
   }
 }
 

@@ -87,7 +87,8 @@ __device__ __forceinline__ bool row_differs(const int32_t *__restrict__ pref, in
 
 __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__ pref_m,
                                                      const int32_t *__restrict__ pref_w, int n, Control *ctrl,
-                                                     int t0, int alike_cta) {
+                                                     int t0, int alike_cta, int only_try = 0) {
+  if (only_try && !ld_volatile_s32(&ctrl->swap_try)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *seen = reinterpret_cast<uint32_t *>(smem_raw);
   __shared__ int s_stop;
@@ -372,7 +373,8 @@ __global__ void k_swap_mark_full(uint8_t *__restrict__ full, const int32_t *__re
 // says that match[] is complete.
 __global__ void k_swap_outcome(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
                                const unsigned long long *__restrict__ bid, int32_t *__restrict__ match, int n,
-                               Control *ctrl) {
+                               Control *ctrl, int only_try = 0) {
+  if (only_try && !ld_volatile_s32(&ctrl->swap_try)) return;
   if (ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status)) return;
   const bool alike = !ld_volatile_s32(&ctrl->w_differ);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
