@@ -220,7 +220,7 @@ __device__ __forceinline__ void hard_order(const int32_t *__restrict__ pref_w, u
   for (int i = tid; i < kHardBuckets; i += nthr) hist[i] = 0;
   __syncthreads();
   for (int i = 0; i < kHardSamples; ++i) {
-    const int32_t *row = pref_w + static_cast<size_t>(static_cast<long long>(i) * n / kHardSamples) * n;
+    const int32_t *row = pref_w + static_cast<size_t>(order_sample(i, kHardSamples, n)) * n;
     for (int r = tid; r < n; r += nthr) {
       const int m = __ldg(row + r);
       if (static_cast<unsigned>(m) < static_cast<unsigned>(n)) atomicAdd(score + m, static_cast<uint32_t>(r));

@@ -159,6 +159,20 @@ __device__ __forceinline__ uint32_t atom_min_relaxed_shared(uint32_t *p, uint32_
 }
 
 // ---------------------------------------------------------------------------
+// The women whose ranks of the men set a starting order: the i-th of `samples`
+// stands somewhere in her part of the n, at a place that follows no pattern, so
+// that women who are numbered by some rule are not sampled by it.
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ int order_sample(int i, int samples, int n) {
+  const int from = static_cast<int>(static_cast<long long>(i) * n / samples);
+  const int to = static_cast<int>(static_cast<long long>(i + 1) * n / samples);
+  uint32_t h = static_cast<uint32_t>(i + 1) * 0x9E3779B9u;
+  h = (h ^ (h >> 15)) * 0x85EBCA6Bu;
+  h ^= h >> 13;
+  return from + static_cast<int>(h % static_cast<uint32_t>(to - from));
+}
+
+// ---------------------------------------------------------------------------
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11), the counter-based
 // generator behind every seeded workload.
 // ---------------------------------------------------------------------------

@@ -58,6 +58,8 @@ namespace smpb200 {
 // spread over the rank matrix, in kOrderBuckets steps; k_order_sort counts
 // the buckets and lays the men out bucket by bucket.  The order within a
 // bucket is arbitrary: any order gives the same matching.
+// (Men liked in one order by the women numbered i n / 64 and in the reverse by all
+// others, n = 4000: 78 ms with those sampled, 3.2 as it is.)
 // ---------------------------------------------------------------------------
 constexpr uint32_t kOrderBuckets = 8192;
 constexpr int kOrderSamples = 64;
@@ -71,7 +73,7 @@ __global__ void __launch_bounds__(256) k_order_score(const RankT *__restrict__ r
     unsigned long long sum = 0;
 #pragma unroll 16
     for (int i = 0; i < samples; ++i) {
-      const size_t w = static_cast<size_t>(static_cast<long long>(i) * n / samples);
+      const size_t w = static_cast<size_t>(order_sample(i, samples, n));
       sum += static_cast<uint32_t>(__ldg(rank + w * ld + m));
     }
     const unsigned long long b = sum * kOrderBuckets / (static_cast<unsigned long long>(n) * samples);

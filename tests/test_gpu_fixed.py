@@ -13,6 +13,15 @@ import pactae_b200 as pb
 pytestmark = pytest.mark.gpu
 
 
+def order_sample(i, samples, n):
+    """The women whose ranks set the starting order (common.cuh)."""
+    start, end = i * n // samples, (i + 1) * n // samples
+    h = (i + 1) * 0x9E3779B9 & 0xFFFFFFFF
+    h = (h ^ (h >> 15)) * 0x85EBCA6B & 0xFFFFFFFF
+    h ^= h >> 13
+    return start + h % (end - start)
+
+
 def worst_order(n):
     # The 64 women whose ranks set the starting order like the men in one order, all
     # others in the reverse: every man who starts displaces all who started before
@@ -21,7 +30,7 @@ def worst_order(n):
     pm[n // 2, [n - 2, n - 1]] = pm[n // 2, [n - 1, n - 2]]  # not one shared list
     pw = np.tile(np.arange(n, dtype=np.int32)[::-1], (n, 1))
     for i in range(64):
-        pw[i * n // 64] = np.arange(n, dtype=np.int32)
+        pw[order_sample(i, 64, n)] = np.arange(n, dtype=np.int32)
     return pm, pw
 
 
@@ -85,6 +94,15 @@ def test_fixed_sequence(ctx, case):
                 status, proposals, _ = batch.run()
                 assert status == [0, 0] and proposals[0] == props
                 assert np.array_equal(insts[0][2].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [700, 1500, 5000])
+def test_worst_order_in_steps_that_are_added(n):
+    pm, pw = worst_order(n)
+    want, props = oracle.gs_seq(pm, pw)
+    with pb.Context() as c:
+        match, st = c.solve(pm, pw)
+        assert np.array_equal(match, want) and st["proposals"] == props and st["mode"] == 0
 
 
 @pytest.mark.parametrize("case", ["uniform 400", "correlated 3001", "shared 2501", "near shared 2501", "men alike 1281"])
