@@ -126,24 +126,31 @@ typedef struct smp_stats {
   int64_t proposals;       /* Gale-Shapley proposals (equal for every execution)    */
   int64_t blocking_pairs;  /* from smp_b200_check / SMP_F_CHECK; -1 if not run     */
   int64_t tail_proposals;  /* the share of proposals settled by the tail kernel     */
+                           /* (0 in rounds and in one-launch solves, which have no  */
+                           /* tail; so are tail_men, tail_hops and tail_ms)         */
   int32_t n;
   int32_t perfect;         /* 1 if the precheck short-circuited the solve          */
   int32_t tail_men;        /* free men handed to the tail kernel                   */
   int32_t rank_bytes;      /* bytes per rank-matrix entry (2 or 4)                  */
   int32_t kernel_launches; /* kernels the call launched                            */
-  int32_t bulk_hops;       /* accepted proposals in the all-SM kernel              */
+  int32_t bulk_hops;       /* accepted proposals in the all-SM kernel, in rounds or */
+                           /* in a one-launch solve (not counted where the women    */
+                           /* proposed)                                             */
   int32_t tail_hops;       /* accepted proposals in the tail kernel                */
   int32_t mode;            /* 0 rank-matrix mode, 1 query mode, 2 query then rank, */
                            /* 3 the men share one list and the women proposed      */
   float stage_ms;          /* host->device copy of the inputs                       */
-  float precheck_ms;       /* device time of each phase (CUDA events)              */
+  float precheck_ms;       /* device time of each phase (CUDA events); a solve in   */
+                           /* one launch (n up to 256) fills core_ms and total_ms   */
   float init_ms;
   float core_ms;
   float post_ms;
   float check_ms;
   float total_ms;          /* precheck + init + core + post                        */
-  float invert_ms;         /* rank inversion / prefix query kernels (part of init) */
-  float bulk_ms;           /* all-SM proposal kernel (part of core)                */
+  float invert_ms;         /* rank inversion / prefix query kernels (part of init); */
+                           /* mode 3: the screen, beside which the women propose    */
+  float bulk_ms;           /* all-SM proposal kernel or rounds (part of core);      */
+                           /* mode 3: the proposals left after the screen           */
   float tail_ms;           /* single-CTA tail kernel (part of core)                */
   float reserved[2];
 } smp_stats;

@@ -21,16 +21,21 @@ constexpr int kModeQuery = 1;  // prefix answered straight from pref_w rows, no 
 // Per-solve control block in device memory.  Kernels of one solve share it;
 // the host writes its initial value (free_count = n, the allow_* switches)
 // before the solve.
-struct Control {
+struct alignas(16) Control {
+  // what the gates read (gate_open): two 16-byte words
   int32_t status;         // first error a kernel saw (kStatus*), 0 if none
   int32_t perfect;        // precheck: every first choice distinct (and allowed)
+  int32_t mode;           // kModeRank or kModeQuery
+  int32_t retry;          // query mode met a man beyond his prefix: rerun in rank mode
+  int32_t use_filter;     // k_bulk runs with its shared partner-rank filter
+  int32_t swap_out;       // men who share one list: match[] is written
+  int32_t rank_bulk;      // a fixed sequence's rank mode goes through k_bulk (k_turn)
+  int32_t swap_try;       // a fixed sequence: the men may share one list (k_turn)
   int32_t next_man;       // bulk kernel: next man that has not proposed yet
   int32_t free_count;     // women that have not received a proposal yet
   int32_t tail_count;     // men handed from the bulk kernel to the tail kernel
   int32_t tail_men;       // men the tail kernel started chains for
   int32_t bad_value;      // first out-of-range preference value seen
-  int32_t mode;           // kModeRank or kModeQuery
-  int32_t retry;          // query mode met a man beyond his prefix: rerun in rank mode
   int32_t allow_perfect;  // host switch: 0 disables the distinct-first-choices shortcut
   int32_t allow_query;    // host switch: 1 if the query mode may be chosen
   int32_t blocks_done;    // precheck: blocks that finished (the last one decides)
@@ -38,7 +43,6 @@ struct Control {
   int32_t distinct_w;     // rank mode: distinct first choices of the women
   int32_t distinct_mid;   // distinct choices in the middle of the men's lists,
   int32_t same_mid;       // and neighbours who make the same choice there
-  int32_t use_filter;     // k_wdistinct: k_bulk runs with its shared partner-rank filter
   int32_t swap_fail;      // k_swap_screen: a pref_m row differs from row 0
   unsigned long long proposals;        // sum over men of (final position + 1)
   unsigned long long blocking;         // checker: blocking pairs
@@ -58,10 +62,6 @@ struct Control {
   int32_t screen_next;    // rows its CTAs have taken beyond their first
   int32_t screen_ctas;    // CTAs of it that have finished
   int32_t screen_done;    // all have
-  int32_t swap_out;       // match[] is written
-  // a solve in one fixed sequence (k_turn)
-  int32_t swap_try;       // the men may share one list
-  int32_t rank_bulk;      // rank mode goes through k_bulk
   int32_t tail_left;      // k_tail_q: chains that have not ended
   int32_t tail_done;      // none are left and the words are final
   int32_t check_deep;     // k_check_near: some man's wife is not among his first choices
@@ -121,6 +121,15 @@ __device__ __forceinline__ int ld_volatile_s32(const int *p) {
 // follows are votes of all of them.
 __device__ __forceinline__ bool warp_flag(const int *flag) {
   return __any_sync(0xFFFFFFFFu, *reinterpret_cast<const volatile int *>(flag) != 0);
+}
+
+__device__ __forceinline__ int4 ld_volatile_v4(const int *p) {
+  int4 v;
+  asm volatile("ld.volatile.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
 }
 
 // Grid-strided L2 prefetch of [p, p + bytes), one request per 128-byte line.

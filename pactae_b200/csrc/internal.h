@@ -253,7 +253,6 @@ struct Ctx {
   int bulk_window = 256;   // look-ahead choices per warp step
   int tail_window = 256;
   int rank_bytes = 2;
-  bool rank_valid = false;  // d_rank holds the inversion of pref_w
   bool tail_ran = false;
   bool swapped = false;  // the men share one list and the women proposed
   bool bulk_rank = false;  // uint16 ranks, but rank mode through k_bulk and k_tail

@@ -67,7 +67,7 @@ constexpr int kOrderSamples = 64;
 template <typename RankT>
 __global__ void __launch_bounds__(256) k_order_score(const RankT *__restrict__ rank, size_t ld,
                                                      uint32_t *__restrict__ score, int n, Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   const int samples = min(n, kOrderSamples);
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
     unsigned long long sum = 0;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) k_order_score(const RankT *__restrict__ r
 // One CTA.
 __global__ void __launch_bounds__(1024) k_order_sort(const uint32_t *__restrict__ score, int32_t *__restrict__ order,
                                                      int n, Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   __shared__ uint32_t hist[kOrderBuckets];
   __shared__ uint32_t warp_sum[32];
   const int tid = threadIdx.x;
@@ -149,8 +149,6 @@ struct RoundCtl {
   int32_t arrived[2];  // CTAs of step t that have scanned their men
   int32_t checked[2];  // rows of step t's new men taken for their range check
   int32_t done;        // the matching is complete and written
-  int32_t steps;       // steps that ran
-  int32_t refreshes;
   int32_t calm;        // 1: few proposals of the step before came too late; -1: many did at four times the chains
 };
 
@@ -824,8 +822,6 @@ __global__ void __launch_bounds__(kRoundBlock, 1)
     b.ctl->slot[(t & 1) ^ 1] = nx;
     b.ctl->arrived[(t & 1) ^ 1] = 0;
     b.ctl->checked[(t & 1) ^ 1] = 0;
-    b.ctl->steps = t + 1;
-    b.ctl->refreshes += nx.refresh;
     const bool few = s_lost * (calm ? kCalmGroup : kCalmWarp) < s_hops;
     if (few && b.ctl->calm == 0)
       b.ctl->calm = 1;

@@ -939,7 +939,6 @@ void reset_progress(Ctx &c) {
 int stage_reset(Ctx &c, int32_t n) {
   c.n = n;
   c.staged = false;
-  c.rank_valid = false;
   c.spent = false;
   c.phase = 0;
   c.stats = smp_stats{};
@@ -1113,9 +1112,9 @@ int enqueue_fixed(Ctx &c) {
   }
   if (!rc) rc = c.d_rankT.ensure(rank_matrix_bytes(c));
   if (!rc) rc = order_buffers(c);
-  if (!rc) rc = enqueue_invert_any(c, kGateModeRank);
+  if (!rc) rc = enqueue_invert_any(c, kGateFixedRank);
   if (!rc) rc = enqueue_order(c, kGateRounds);
-  if (!rc) rc = enqueue_transpose(c, kGateModeRank);
+  if (!rc) rc = enqueue_transpose(c, kGateFixedRank);
   if (!rc && bulk) {
     rc = enqueue_pr(c, kGateBulk);
     if (!rc) rc = launch_bulk_filtered<uint16_t, 8>(c, 0);
@@ -2170,7 +2169,6 @@ int smp_b200_invert(smp_ctx *ctx, const int32_t *pref_w, int32_t n, int32_t *ran
   c.n = n;
   c.phase = 0;
   c.staged = false;
-  c.rank_valid = false;
   const size_t bytes = sizeof(int32_t) * static_cast<size_t>(n) * n;
   int rc = c.d_ctrl.ensure(sizeof(Control));
   if (rc) return rc;

@@ -24,9 +24,10 @@
 //                   w among a man's first K choices are qlist[w*qcap ..] (qcnt[w])
 //   bid             u64 [n] (see common.cuh)
 //
-// Every kernel opens with a gate (below) read from the control block, so the
-// host enqueues the whole pipeline once and the device decides which parts
-// run: no host round trip inside a solve.
+// Every kernel opens with a gate (below) read from the control block: a solve in
+// one fixed sequence is enqueued whole and the device decides which parts run.
+// A solve in passes enqueues the kernels of one mode and reads the control block
+// back before the next; the gates hold there too.
 #pragma once
 
 #include <type_traits>
@@ -45,30 +46,45 @@ enum Gate : int {
   kGateMain = 1,       // round 0 of a solve: not perfect, no error seen
   kGateModeRank = 2,   // round 0 in rank mode
   kGateModeQuery = 3,  // round 0 in query mode
+  kGateQuery = 10,     // and no retry pending
   kGateRetry = 4,      // the rank-mode round after a query-mode abort
   kGateOrder = 5,      // round 0 in rank mode, but not through the filtered bulk
-  kGateRounds = 7,     // a fixed sequence's rank mode, in rounds
-  kGateBulk = 8,       // through k_bulk
   kGateNoRank = 6,     // the checker after a solve that built no rank matrix
+  kGateFixedRank = 7,  // a fixed sequence's rank mode (k_turn),
+  kGateRounds = 8,     // in rounds
+  kGateBulk = 9,       // or through k_bulk
 };
 
 __device__ __forceinline__ bool gate_open(int gate, const Control *c) {
   if (gate == kGateAlways) return true;
-  const int perfect = ld_volatile_s32(&c->perfect);
-  if (gate == kGateNoRank) return perfect != 0 || ld_volatile_s32(&c->mode) == kModeQuery;
-  if (perfect || ld_volatile_s32(&c->status)) return false;
+  const int4 g = ld_volatile_v4(&c->status);  // status, perfect, mode, retry
+  if (gate == kGateNoRank) return g.y != 0 || g.z == kModeQuery;
+  if (g.y || g.x) return false;
   switch (gate) {
     case kGateMain: return true;
-    case kGateModeRank: return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->swap_out);
-    case kGateModeQuery: return ld_volatile_s32(&c->mode) == kModeQuery;
-    case kGateOrder: return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->use_filter);
-    case kGateRounds:
-    case kGateBulk:
-      return ld_volatile_s32(&c->mode) == kModeRank && !ld_volatile_s32(&c->swap_out) &&
-             (ld_volatile_s32(&c->rank_bulk) != 0) == (gate == kGateBulk);
-    case kGateRetry: return ld_volatile_s32(&c->retry) != 0;
+    case kGateModeRank: return g.z == kModeRank;
+    case kGateModeQuery: return g.z == kModeQuery;
+    case kGateQuery: return g.z == kModeQuery && !g.w;
+    case kGateRetry: return g.w != 0;
+    default: break;
+  }
+  if (g.z != kModeRank) return false;
+  const int4 h = ld_volatile_v4(&c->use_filter);  // use_filter, swap_out, rank_bulk, swap_try
+  switch (gate) {
+    case kGateOrder: return !h.x;
+    case kGateFixedRank: return !h.y;
+    case kGateRounds: return !h.y && !h.z;
+    case kGateBulk: return !h.y && h.z;
     default: return false;
   }
+}
+
+// The same, read once for the CTA.  An open or closed gate costs a request for every
+// warp that looks, all to one L2 slice: with 16 warps a CTA looking, flag by flag, a
+// gated transpose took 10 us.  (And threads that each look may see an error that
+// another CTA reports meanwhile, or not, before a barrier.)
+__device__ __forceinline__ bool cta_gate_open(int gate, const Control *c) {
+  return __syncthreads_or(threadIdx.x == 0 && gate_open(gate, c));
 }
 
 // Unset marker of a rank slot during inversion: never a valid rank (uint16
@@ -125,7 +141,7 @@ __device__ __forceinline__ void count_alike(const int32_t *__restrict__ pref_m, 
 
 __global__ void __launch_bounds__(256) k_alike(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
                                                int n, uint32_t *bitmaps, Control *ctrl) {
-  if (gate_open(kGateModeRank, ctrl)) count_alike(pref_m, pref_w, n, bitmaps, ctrl);
+  if (cta_gate_open(kGateModeRank, ctrl)) count_alike(pref_m, pref_w, n, bitmaps, ctrl);
 }
 
 // ---------------------------------------------------------------------------
@@ -259,7 +275,7 @@ __device__ __forceinline__ void load_row(const int32_t *__restrict__ row, RankT 
 template <typename RankT>
 __global__ void __launch_bounds__(512) k_invert(const int32_t *__restrict__ pref_w, RankT *__restrict__ rank,
                                                 size_t ld, int n, Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RankT *sbuf = reinterpret_cast<RankT *>(smem_raw);
   constexpr int kPerVec = 16 / sizeof(RankT);
@@ -303,7 +319,7 @@ __global__ void __launch_bounds__(512) k_invert(const int32_t *__restrict__ pref
 // sits at the output row's offset from a 16-byte boundary.
 __global__ void __launch_bounds__(512) k_invert_wide(const int32_t *__restrict__ pref_w, int32_t *__restrict__ rank,
                                                      int n, Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint16_t *sbuf = reinterpret_cast<uint16_t *>(smem_raw);
   bool bad = false;
@@ -342,7 +358,7 @@ __global__ void __launch_bounds__(512) k_invert_wide(const int32_t *__restrict__
 // global memory, then verify rank[w][pref_w[w][r]] == r in a second pass.
 __global__ void k_invert_global(const int32_t *__restrict__ pref_w, int32_t *__restrict__ rank, int n,
                                 Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   const size_t total = static_cast<size_t>(n) * n;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -358,7 +374,7 @@ __global__ void k_invert_global(const int32_t *__restrict__ pref_w, int32_t *__r
 }
 __global__ void k_invert_verify(const int32_t *__restrict__ pref_w, const int32_t *__restrict__ rank, int n,
                                 Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   const size_t total = static_cast<size_t>(n) * n;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -384,7 +400,7 @@ __global__ void k_invert_verify(const int32_t *__restrict__ pref_w, const int32_
 // past n are written as 0xFFFF.
 __global__ void __launch_bounds__(512) k_transpose16(const uint16_t *__restrict__ src, uint16_t *__restrict__ dst,
                                                      size_t ld, int n, Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   __shared__ uint16_t tile[64][66];
   const int row = threadIdx.x >> 3, ch = threadIdx.x & 7;  // 64 rows x 8 chunks of 8 entries
   const int tiles = (n + 63) / 64;
@@ -417,7 +433,7 @@ __global__ void __launch_bounds__(512) k_transpose16(const uint16_t *__restrict_
 template <typename T>
 __global__ void __launch_bounds__(512) k_transpose(const T *__restrict__ src, T *__restrict__ dst, int n,
                                                    Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   __shared__ T tile[64][65];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 16
   const int tiles = (n + 63) / 64;
@@ -491,11 +507,12 @@ __global__ void __launch_bounds__(512) k_validate_rows(const int32_t *__restrict
 // on the device, else nullptr).
 __global__ void k_qscatter(const int32_t *__restrict__ pref_m, int n, int K, int qcap, int32_t *__restrict__ qcnt,
                            uint32_t *__restrict__ qlist, Control *ctrl, const int32_t *__restrict__ pref_w) {
-  if (!gate_open(kGateModeQuery, ctrl)) {
-    if (pref_w && gate_open(kGateModeRank, ctrl))
-      count_alike(pref_m, pref_w, n, reinterpret_cast<uint32_t *>(qcnt), ctrl);
-    return;
-  }
+  __shared__ int s_way;
+  if (threadIdx.x == 0)
+    s_way = gate_open(kGateModeQuery, ctrl) ? 1 : pref_w && gate_open(kGateModeRank, ctrl) ? 2 : 0;
+  __syncthreads();
+  if (s_way == 2) count_alike(pref_m, pref_w, n, reinterpret_cast<uint32_t *>(qcnt), ctrl);
+  if (s_way != 1) return;
   const size_t total = static_cast<size_t>(n) * K;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -520,7 +537,7 @@ __global__ void __launch_bounds__(512) k_qinvert(const int32_t *__restrict__ pre
                                                  const int32_t *__restrict__ qcnt,
                                                  const uint32_t *__restrict__ qlist,
                                                  uint32_t *__restrict__ prefix, Control *ctrl, int w0, int w1) {
-  if (!gate_open(kGateModeQuery, ctrl) || ld_volatile_s32(&ctrl->retry)) return;
+  if (!cta_gate_open(kGateQuery, ctrl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint16_t *srow = reinterpret_cast<uint16_t *>(smem_raw);
   const int chunks = (n + 7) / 8;
@@ -609,7 +626,7 @@ __global__ void __launch_bounds__(kThreads) k_qinvert_c(const int32_t *__restric
                                                       const int32_t *__restrict__ qcnt,
                                                       const uint32_t *__restrict__ qlist,
                                                       uint32_t *__restrict__ prefix, Control *ctrl, int w0, int w1) {
-  if (!gate_open(kGateModeQuery, ctrl) || ld_volatile_s32(&ctrl->retry)) return;
+  if (!cta_gate_open(kGateQuery, ctrl)) return;
   int w = w0 + static_cast<int>(blockIdx.x);
   if (w >= w1) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -708,7 +725,7 @@ __host__ __device__ constexpr int rank_layout() {
 __global__ void __launch_bounds__(512) k_pr(const int32_t *__restrict__ pref_m, const uint16_t *__restrict__ rankT,
                                             size_t ld, uint16_t *__restrict__ pr, uint32_t *__restrict__ prefix, int K, int n,
                                             Control *ctrl, int gate) {
-  if (!gate_open(gate, ctrl)) return;
+  if (!cta_gate_open(gate, ctrl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x;
   const int nthr = blockDim.x;
@@ -789,7 +806,7 @@ __global__ void __launch_bounds__(256) k_qinvert_p16(const uint16_t *__restrict_
                                                      const int32_t *__restrict__ qcnt,
                                                      const uint32_t *__restrict__ qlist,
                                                      uint32_t *__restrict__ prefix, Control *ctrl, int w0, int w1) {
-  if (!gate_open(kGateModeQuery, ctrl) || ld_volatile_s32(&ctrl->retry)) return;
+  if (!cta_gate_open(kGateQuery, ctrl)) return;
   int w = w0 + static_cast<int>(blockIdx.x);
   if (w >= w1) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -982,20 +999,23 @@ __global__ void __launch_bounds__(kFilter ? kFilterBlock : 256)
     // barrier.
     __shared__ int s_go;
     if (threadIdx.x == 0)
-      s_go = round == 0 && ld_volatile_s32(&ctrl->use_filter) && gate_open(kGateModeRank, ctrl) &&
+      s_go = round == 0 && ld_volatile_s32(&ctrl->use_filter) && gate_open(kGateFixedRank, ctrl) &&
              !ld_volatile_s32(&ctrl->retry);
     __syncthreads();
     if (!s_go) return;
     for (int w = threadIdx.x; w < n; w += blockDim.x) lrank[w] = 0xFFFFFFFFu;
     __syncthreads();
   } else {
-    if (!gate_open(round == 0 ? kGateMain : kGateRetry, ctrl)) return;
-    if (round == 0 && ld_volatile_s32(&ctrl->retry)) return;  // a query bucket overflowed
-    if (round == 0 && ld_volatile_s32(&ctrl->use_filter)) return;  // the filtered variant runs
-    // enqueued for one mode only (the host has not read the precheck yet)
-    if (round == 0 && only_mode == kOnlyRankBulk && !gate_open(kGateBulk, ctrl)) return;
-    if (round == 0 && (only_mode == kModeRank || only_mode == kModeQuery) && ld_volatile_s32(&ctrl->mode) != only_mode)
-      return;
+    const auto closed = [&]() {
+      if (!gate_open(round == 0 ? kGateMain : kGateRetry, ctrl)) return true;
+      if (round != 0) return false;
+      // a query bucket overflowed, or the filtered variant runs
+      if (ld_volatile_s32(&ctrl->retry) || ld_volatile_s32(&ctrl->use_filter)) return true;
+      // enqueued for one mode only (the host has not read the precheck yet)
+      if (only_mode == kOnlyRankBulk) return !gate_open(kGateBulk, ctrl);
+      return only_mode >= 0 && ld_volatile_s32(&ctrl->mode) != only_mode;
+    };
+    if (__syncthreads_or(threadIdx.x == 0 && closed())) return;
   }
   const bool query = round == 0 && ld_volatile_s32(&ctrl->mode) == kModeQuery;
   // Free women left when the men move to the one-CTA tail: rank-mode
@@ -1145,8 +1165,8 @@ __device__ __forceinline__ void write_perfect(const int32_t *__restrict__ pref_m
 // 2-byte array (SharedBids).  Warps take men from the bulk kernel's queue and
 // from the men that never proposed, and follow their chains with every bid
 // read and atomic inside the SM.  At the end the CTA writes match[] and the
-// proposal count.  In query mode a man beyond his prefix sets the retry flag
-// and every warp stops.
+// proposal count.  Rank mode only (int32 ranks, and uint16 ones through k_bulk):
+// the query mode's tails are k_tail_qw and k_tail_q.
 // round 0: gate Main (and no retry pending); round 1: gate Retry.
 // only_mode = kOnlyRankBulk: in a fixed sequence, where k_turn chose k_bulk.
 // ---------------------------------------------------------------------------
@@ -1166,12 +1186,10 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
   }
   if (!gate_open(round == 0 ? kGateMain : kGateRetry, ctrl)) return;
   if (round == 0 && ld_volatile_s32(&ctrl->retry)) return;
-  const bool query = round == 0 && ld_volatile_s32(&ctrl->mode) == kModeQuery;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *sbid = reinterpret_cast<uint32_t *>(smem_raw);
   uint16_t *spos = reinterpret_cast<uint16_t *>(smem_raw + static_cast<size_t>(n) * 4);
   __shared__ int s_next;
-  __shared__ int s_abort;
   __shared__ int s_busy;  // warps carrying a chain
   __shared__ unsigned long long s_props;
   const int tid = threadIdx.x;
@@ -1183,7 +1201,6 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
   tail_setup(bid, sbid, spos, n);
   if (tid == 0) {
     s_next = 0;
-    s_abort = 0;
     s_busy = 0;
     s_props = 0;
     ctrl->tail_men = total;
@@ -1191,7 +1208,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
   __syncthreads();
 
   const SharedBids bids{sbid, spos};
-  const auto keep_going = [&]() { return !warp_flag(&s_abort); };
+  const auto keep_going = []() { return true; };
   int m = -1, pos = 0, S = 1, bad_value = 0;
   Ahead ahead;
   unsigned long long settled = 0;
@@ -1208,7 +1225,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
         pos = e.y;
       } else {
         m = first_unstarted + (i - queued);
-        if (!query && order) m = __ldg(order + m);
+        if (order) m = __ldg(order + m);
         pos = 0;
       }
       S = 1;
@@ -1231,16 +1248,11 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
       }
     }
     const int rc = man_step<kMaxSub, (kMaxSub < 8), true, (kMaxSub == 8 ? 8 : 1), rank_layout<RankT>()>(
-        bids, keep_going, pref_m, rank, prefix, K, n, query, lane, m, pos, S, ahead, settled,
+        bids, keep_going, pref_m, rank, prefix, K, n, false, lane, m, pos, S, ahead, settled,
                                      hops, bad_value);
     if (rc == kStepMatchedFree && lane == 0) atomicSub(&s_busy, 1);
     if (rc == kStepMoved || rc == kStepMatchedFree) continue;
-    if (rc == kStepBad) {
-      if (lane == 0) report(ctrl, kStatusInvalidInput, bad_value);
-    } else if (rc == kStepBeyond && lane == 0) {
-      s_abort = 1;
-      atomicExch(&ctrl->retry, 1);
-    }
+    if (lane == 0) report(ctrl, kStatusInvalidInput, bad_value);
     break;
   }
   if (lane == 0 && settled) {
@@ -1248,7 +1260,7 @@ __global__ void __launch_bounds__(1024, 1) k_tail(const int32_t *__restrict__ pr
     atomicAdd(&ctrl->tail_hops, hops);
   }
   __syncthreads();
-  if (s_abort || ld_volatile_s32(&ctrl->status)) return;
+  if (ld_volatile_s32(&ctrl->status)) return;
   if (ld_volatile_s32(&ctrl->coop_count) > 0) {
     // chains handed over: the shared state goes to k_tail_coop through the
     // bid buffer, which this kernel no longer reads

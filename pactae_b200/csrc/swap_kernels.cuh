@@ -88,7 +88,7 @@ __device__ __forceinline__ bool row_differs(const int32_t *__restrict__ pref, in
 __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__ pref_m,
                                                      const int32_t *__restrict__ pref_w, int n, Control *ctrl,
                                                      int t0, int alike_cta, int only_try = 0) {
-  if (only_try && !ld_volatile_s32(&ctrl->swap_try)) return;
+  if (only_try && !__syncthreads_or(threadIdx.x == 0 && ld_volatile_s32(&ctrl->swap_try))) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *seen = reinterpret_cast<uint32_t *>(smem_raw);
   __shared__ int s_stop;
@@ -102,9 +102,11 @@ __global__ void __launch_bounds__(256) k_swap_screen(const int32_t *__restrict__
   // Rows are taken in turn, each CTA's next one while it works on the last: a
   // CTA that waits for the proposals' CTA to leave its SM then takes fewer.
   // Those from alike_cta on leave after their first where the women's lists are
-  // alike: a second CTA of the proposals gets their place.
+  // alike (and not all the same, as it seems): a second CTA of the proposals gets
+  // their place.
   int next = t0 + static_cast<int>(blockIdx.x);
-  const bool leaves = static_cast<int>(blockIdx.x) >= alike_cta && women_alike(ctrl, n);
+  const bool leaves = tid == 0 && static_cast<int>(blockIdx.x) >= alike_cta && women_alike(ctrl, n) &&
+                      ld_volatile_s32(&ctrl->distinct_w) > 1;
   for (;;) {
     if (tid == 0) {
       s_row = next;
@@ -233,12 +235,15 @@ __global__ void __launch_bounds__(256) k_swap_gs(const int32_t *__restrict__ pre
   int w = -1, r0 = 0;
   uint32_t key = 0;
   unsigned steps = 0;
-  if (beside == 1 && (ld_volatile_s32(&ctrl->distinct_w) <= 1 ||
-                      (static_cast<int>(blockIdx.x) >= alike_cta && !women_alike(ctrl, n))))
-    return;
-  if (beside == 2 && (ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status) ||
-                      !ld_volatile_s32(&ctrl->w_differ)))
-    return;
+  if (beside) {  // (one look for the CTA, as with the gates)
+    int closed = 0;
+    if (threadIdx.x == 0 && beside == 1)
+      closed = ld_volatile_s32(&ctrl->distinct_w) <= 1 ||
+               (static_cast<int>(blockIdx.x) >= alike_cta && !women_alike(ctrl, n));
+    if (threadIdx.x == 0 && beside == 2)
+      closed = ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status) || !ld_volatile_s32(&ctrl->w_differ);
+    if (__syncthreads_or(closed)) return;
+  }
   for (;;) {
     // Now and then only: thousands of warps reading these flags at every step
     // would queue at one L2 slice.
