@@ -231,6 +231,8 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   int sm_count = 148;
   size_t smem_optin = 0;  // max dynamic shared memory per block
+  size_t wide_smem = 0;   // CTAs of k_invert_wide an SM holds with so much shared memory
+  int wide_per_sm = 0;
   int prefix_k_cfg = 0;
   int tail_threshold_cfg = 0;
   int bulk_window_cfg = 0;

@@ -29,7 +29,8 @@
 // positions, so none of this shows in the outputs.
 //
 // Measured on one B200 against k_bulk, k_tail and k_tail_coop over ranks by
-// position, which still serve int32 ranks and lists whose bids no SM holds:
+// position, which still serve int32 ranks, lists whose bids no SM holds, and men
+// who are alike among women who are not (bulk_rank_pays in smp_b200.cu):
 // RANDOM(5) n = 15013 18.7 -> 4.0 ms (18.7 M displacements -> 98 thousand),
 // n = 30000 58.8 -> 9.6; SOLO n = 10007 43.6 -> 3.0; correlated n = 30000
 // 10.8 -> 7.9, n = 2000 0.57 -> 0.53, n = 97 0.25 -> 0.22.  A step of the

@@ -146,6 +146,9 @@ bool bulk_rank_pays(const Ctx &c) { return rounds_fit(c) && rank_bulk_pays(*c.h_
 // What a solve needs zeroed, in one buffer and one reset: the control block,
 // the query buckets' counts and the precheck's bitmap.
 constexpr size_t kCtrlBytes = (sizeof(Control) + 255) & ~static_cast<size_t>(255);
+// What the host reads back and other calls reset: all but the chains that k_tail
+// hands over, which coop_count says are there.
+constexpr size_t kCtrlHead = offsetof(Control, coop_chain);
 size_t zero_bytes(int n) {
   return kCtrlBytes + sizeof(int32_t) * (static_cast<size_t>(n) + (static_cast<size_t>(n) + 31) / 32);
 }
@@ -215,12 +218,16 @@ int enqueue_invert(Ctx &c, const int32_t *pref_w, RankT *rank, size_t ld, int ga
     if (n <= kU16MaxN) {  // int32 output from a uint16 shared row
       if (allow_dynamic_smem(c, k_invert_wide) != cudaSuccess)
         return c.fail_cuda("k_invert_wide smem attribute");
-      int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_invert_wide, 512, smem16) != cudaSuccess) {
-        cudaGetLastError();
-        per_sm = 1;
+      if (c.wide_smem != smem16) {  // (asking takes a microsecond of a small call's 42)
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_invert_wide, 512, smem16) != cudaSuccess) {
+          cudaGetLastError();
+          per_sm = 1;
+        }
+        c.wide_smem = smem16;
+        c.wide_per_sm = std::max(per_sm, 1);
       }
-      const int grid = std::min(n, c.sm_count * std::max(per_sm, 1));
+      const int grid = std::min(n, c.sm_count * c.wide_per_sm);
       k_invert_wide<<<grid, 512, smem16, c.stream>>>(pref_w, rank, n, c.d_ctrl.as<Control>(), gate);
       c.launches++;
       return c.check_launch("k_invert_wide");
@@ -852,7 +859,7 @@ int copy_match_out(Ctx &c, int32_t *match_out, bool device) {
 }
 
 int read_control(Ctx &c) {
-  if (cudaMemcpyAsync(c.h_ctrl, c.d_ctrl.ptr, sizeof(Control), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess)
+  if (cudaMemcpyAsync(c.h_ctrl, c.d_ctrl.ptr, kCtrlHead, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess)
     return c.fail_cuda("control readback");
   return SMP_OK;
 }
@@ -2035,7 +2042,7 @@ int smp_b200_precheck(smp_ctx *ctx, int32_t *is_perfect) {
   c.spent = false;
   if (cudaEventRecord(c.ev[kEvStageEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   int rc = enqueue_precheck(c, true);
-  if (!rc && rounds_fit(c) && c.lists_here) rc = enqueue_alike(c, true);
+  if (!rc && rounds_fit(c) && c.lists_here && c.n >= kBulkRankMinN) rc = enqueue_alike(c, true);
   if (!rc) rc = read_control(c);
   if (rc) return rc;
   if (cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
@@ -2183,7 +2190,7 @@ int smp_b200_invert(smp_ctx *ctx, const int32_t *pref_w, int32_t n, int32_t *ran
     src = c.d_pref_w.as<int32_t>();
     dst = c.d_rank.as<int32_t>();
   }
-  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, sizeof(Control), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
+  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, kCtrlHead, c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   if (cudaEventRecord(c.ev[kEvPrecheckEnd], c.stream) != cudaSuccess) return c.fail_cuda("event");
   rc = enqueue_invert<int32_t>(c, src, dst, static_cast<size_t>(n), kGateAlways);
   if (rc) return rc;
@@ -2219,7 +2226,7 @@ int smp_b200_check(smp_ctx *ctx, const int32_t *pref_m, const int32_t *pref_w, i
       return c.fail_cuda("match copy");
     dmatch = c.d_match.as<int32_t>();
   }
-  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, sizeof(Control), c.stream) != cudaSuccess) return c.fail_cuda("control reset");
+  if (cudaMemsetAsync(c.d_ctrl.ptr, 0, kCtrlHead, c.stream) != cudaSuccess) return c.fail_cuda("control reset");
   if (cudaEventRecord(c.ev[kEvCheckBegin], c.stream) != cudaSuccess) return c.fail_cuda("event");
   if (n > kU16MaxN) {
     rc = enqueue_precheck(c, false);  // reports first choices out of range
