@@ -199,11 +199,11 @@ size_t rank_ld(const Ctx &c) {
 }
 size_t rank_matrix_bytes(const Ctx &c) { return static_cast<size_t>(c.n) * rank_ld(c) * c.rank_bytes; }
 
-
 // The men start by popularity (k_order_*) in the rounds, and in k_bulk from this
-// n on, unless k_wdistinct has chosen its filtered variant: below it the two launches cost more than they save (rank mode without a
-// tail, correlated n = 500 / 1500 / 6000: 303, 453 and 1737 us without, 321, 496
-// and 1793 with; n = 40000 25.2 and 24.7 ms, both sides one list 206 and 69).
+// n on, unless k_wdistinct has chosen its filtered variant: below it the two
+// launches cost more than they save (rank mode without a tail, correlated n = 500 /
+// 1500 / 6000: 303, 453 and 1737 us without, 321, 496 and 1793 with; n = 40000 25.2
+// and 24.7 ms, both sides one list 206 and 69).
 constexpr int kOrderMinN = 8192;
 bool ordered(const Ctx &c) { return in_rounds(c) || (!c.bulk_rank && c.n >= kOrderMinN); }
 bool filter_fits(const Ctx &c) { return sizeof(uint32_t) * static_cast<size_t>(c.n) + 1024 <= c.smem_optin; }
@@ -365,7 +365,7 @@ RoundBufs round_bufs(const Ctx &c) {
 // (c.poll_rounds) gets kRoundExtra more and adds steps until round_done;
 // otherwise kRoundExtraBlind follow, then the last step, which ends any solve.
 constexpr int kRoundExtra = 1;
-constexpr int kRoundExtraBlind = 2;  // (12: 20 to 30 us more whatever the lists, and no family of the generator faster)
+constexpr int kRoundExtraBlind = 2;  // (12: 20 to 30 us more, and no family of the generator faster)
 constexpr int kRoundMore = 8;
 
 int enqueue_round_steps(Ctx &c, int gate, int count) {
@@ -1289,7 +1289,8 @@ namespace {
 // that only the larger pipelines heed.
 bool solve_is_small(const Ctx &c, uint32_t flags) {
   return c.n >= 1 && c.n <= kSmallMaxN && small_smem(c.n) + 256 <= c.smem_optin && c.prefix_k_cfg == 0 &&
-         c.tail_threshold_cfg == 0 && c.bulk_window_cfg == 0 && c.mode_cfg == 0 && c.rank_bytes_cfg == 0 && !(flags & (SMP_F_CHECK | SMP_F_VALIDATE));
+         c.tail_threshold_cfg == 0 && c.bulk_window_cfg == 0 && c.mode_cfg == 0 && c.rank_bytes_cfg == 0 &&
+         !(flags & (SMP_F_CHECK | SMP_F_VALIDATE));
 }
 
 int enqueue_small(Ctx &c, int32_t *match_out, uint32_t flags) {
@@ -1430,8 +1431,7 @@ int solve_swapped(Ctx &c, uint32_t flags, int32_t *match_out, bool &swapped) {
   if (!rc) rc = c.sync("swap screen");
   if (rc) return rc;
   swapped = c.h_ctrl->status || !c.h_ctrl->swap_fail;
-  if (!swapped || c.h_ctrl->status) return SMP_OK;
-  c.swapped = true;
+  c.swapped = swapped && !c.h_ctrl->status;
   return SMP_OK;
 }
 
