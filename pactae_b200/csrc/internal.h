@@ -257,6 +257,10 @@ struct Ctx {
   int rank_bytes = 2;
   bool tail_ran = false;
   bool swapped = false;  // the men share one list and the women proposed
+  // Men who all make the same first choice may share the first man's list, which
+  // is then refused if it is no permutation.  Not by a checked solve, a served
+  // request or a routed instance, which take the men's own proposals for an answer.
+  bool first_man = false;
   bool bulk_rank = false;  // uint16 ranks, but rank mode through k_bulk and k_tail
   int phase = 0;            // 0 staged, 1 prechecked, 2 inited, 3 cored, 4 posted
   // A solve or a core has used up the precheck's state: init and core after it

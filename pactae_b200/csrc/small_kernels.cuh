@@ -37,7 +37,8 @@ __host__ __device__ constexpr size_t small_smem(int n) {
 
 __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ pref_m,
                                                    const int32_t *__restrict__ pref_w, int n, int K,
-                                                   int allow_perfect, int32_t *match, int32_t *also, Control *out) {
+                                                   int allow_perfect, int32_t *match, int32_t *also, Control *out,
+                                                   int first_man) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const size_t n2 = static_cast<size_t>(n) * n;
   uint16_t *list = reinterpret_cast<uint16_t *>(smem_raw);
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
   uint16_t *spos = reinterpret_cast<uint16_t *>(word + n);
   __shared__ int s_distinct, s_differ, s_status, s_bad, s_next, s_deep, s_late;
   __shared__ unsigned int s_hops;
+  __shared__ uint32_t s_row0[kSmallMaxN / 32];  // women the first man's list has named
   __shared__ unsigned long long s_props;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -58,6 +60,7 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
     s_hops = 0;
     s_props = 0;
   }
+  if (tid < kSmallMaxN / 32) s_row0[tid] = 0;
   for (int i = tid; i < 8 * n; i += 1024) seen[i] = 0;
   for (int i = tid; i < n; i += 1024) {
     word[i] = 0xFFFFFFFFu;
@@ -109,8 +112,14 @@ __global__ void __launch_bounds__(1024, 1) k_small(const int32_t *__restrict__ p
         else
           refuse(w);
         list[t] = 0;
-      } else
+      } else {
+        const uint32_t bit = 1u << (w & 31);
+        if (m == 0 && distinct == 1 && mode == kModeRank && (atomicOr(s_row0 + (w >> 5), bit) & bit)) {
+          if (first_man) refuse(w);
+          differ = true;  // no list to share
+        }
         list[t] = static_cast<uint16_t>((w << 8) | rank[w * n + m]);
+      }
     }
     if (differ) s_differ = 1;
     // (all warps or none: one that refuses a man in the chains must not keep lanes

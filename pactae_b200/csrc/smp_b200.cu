@@ -429,7 +429,8 @@ int enqueue_query_index(Ctx &c) {
   c.qcnt_clean = false;
   const int grid = static_cast<int>(std::min<size_t>(static_cast<size_t>(c.sm_count) * 16, (total + 255) / 256));
   k_qscatter<<<grid, 256, 0, c.stream>>>(c.pref_m, n, c.K, qcap, qcnt_of(c), c.d_qlist.as<uint32_t>(),
-                                         c.d_ctrl.as<Control>(), c.lists_here ? c.pref_w : nullptr);
+                                         c.d_ctrl.as<Control>(), c.lists_here ? c.pref_w : nullptr,
+                                         c.first_man && n > 2);
   c.launches++;
   return c.check_launch("k_qscatter");
 }
@@ -938,7 +939,7 @@ void reset_progress(Ctx &c) {
   c.pass_match = nullptr;
   c.poll_rounds = c.poll_tail = false;
   c.round_step = c.tail_segment = 0;
-  c.swapped = false;
+  c.swapped = c.first_man = false;
   c.bulk_rank = false;
 }
 
@@ -1230,7 +1231,7 @@ int enqueue_swap_screen(Ctx &c, bool men_screened) {
   if (cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
       cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("swap reset");
-  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl);
+  k_swap_pos<<<grid, 256, 0, c.stream>>>(c.pref_m, pos, n, ctrl, men_screened || c.first_man);
   if (!c.query_ok && !rounds_fit(c)) rc = enqueue_alike(c, false);  // not counted yet
   if (rc) return rc;
   uint16_t *near = n <= kU16MaxN ? c.d_swap_near.as<uint16_t>() : nullptr;
@@ -1299,7 +1300,7 @@ int enqueue_small(Ctx &c, int32_t *match_out, uint32_t flags) {
   if (rc) return rc;
   if (allow_dynamic_smem(c, k_small) != cudaSuccess) return c.fail_cuda("k_small smem attribute");
   k_small<<<1, 1024, small_smem(c.n), c.stream>>>(c.pref_m, c.pref_w, c.n, c.K, (flags & SMP_F_NO_PRECHECK) == 0,
-                                                  match_here(c), match_also(c), c.h_ctrl);
+                                                  match_here(c), match_also(c), c.h_ctrl, c.first_man);
   c.launches++;
   rc = c.check_launch("k_small");
   if (!rc && cudaEventRecord(c.ev[kEvPostEnd], c.stream) != cudaSuccess) rc = c.fail_cuda("event");
@@ -1323,6 +1324,8 @@ int solve_begin(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, int32_t n,
     return solve_enqueue(c, pref_m, pref_w, n, match_out, flags);
   }
   int rc = do_stage(c, pref_m, pref_w, n, flags);
+  c.first_man = c.synchronous && !(flags & SMP_F_CHECK) && c.mode_cfg == 0 && c.tail_window_cfg == 0 &&
+                swap_screen_fits(c);
   c.pass_flags = flags;
   c.pass_match = match_out;
   // (never into the lists: a kernel that writes the matching may still read them)
@@ -1382,7 +1385,7 @@ int solve_advance(Ctx &c, bool &more) {
   // one first choice for every man: perhaps one list for every man (and if a
   // query pass has looked, one choice in the middle)
   if (c.pass != kPassScreen && !h.perfect && h.mode == kModeRank && h.distinct == 1 && c.n >= 2 && c.mode_cfg == 0 &&
-      (!queried || h.same_mid == c.n) && swap_screen_fits(c)) {
+      (!queried || h.same_mid == c.n || (c.first_man && c.n == 2)) && swap_screen_fits(c)) {
     c.pass = kPassScreen;
     return enqueue_swap_screen(c, false);
   }
@@ -1668,7 +1671,7 @@ int solve_shared_host(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, uint
         cudaMemsetAsync(pos, 0xFF, sizeof(int32_t) * static_cast<size_t>(n), c.stream) != cudaSuccess ||
         cudaMemsetAsync(d_rows, 0, sizeof(int32_t), c.stream) != cudaSuccess)  // the row list {0}
       return c.fail_cuda("shared lists copy");
-    k_swap_pos<<<grid, 256, 0, c.stream>>>(dm, pos, n, ctrl);
+    k_swap_pos<<<grid, 256, 0, c.stream>>>(dm, pos, n, ctrl, 1);
     k_swap_rows_check<<<1, 256, check_smem, c.stream>>>(dw, n, d_rows, 1, n, ctrl);
     c.launches += 2;
     rc = c.check_launch("k_swap_rows_check");
@@ -1695,7 +1698,7 @@ int solve_shared_host(Ctx &c, const int32_t *pref_m, const int32_t *pref_w, uint
       cudaMemsetAsync(full, 0, static_cast<size_t>(n), c.stream) != cudaSuccess ||
       cudaMemsetAsync(bid, 0xFF, sizeof(unsigned long long) * static_cast<size_t>(n), c.stream) != cudaSuccess)
     return c.fail_cuda("swap reset");
-  k_swap_pos<<<grid, 256, 0, c.stream>>>(dm, pos, n, ctrl);
+  k_swap_pos<<<grid, 256, 0, c.stream>>>(dm, pos, n, ctrl, 1);
   k_swap_rows_check<<<row_grid, 256, check_smem, c.stream>>>(dw, n, nullptr, n, kw, ctrl);
   c.launches += 2;
   rc = c.check_launch("k_swap_rows_check");

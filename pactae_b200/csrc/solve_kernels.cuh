@@ -112,9 +112,10 @@ __device__ __forceinline__ bool any_unset<int32_t>(uint4 v) {
 // How alike the lists of a rank-mode instance are: the distinct first choices of
 // the women, and the distinct entries in the middle of the men's lists (not with
 // pref_m = nullptr), in two bitmaps of zeros one after the other; and how many men
-// have the same there as the man after them.
+// have the same there as the man after them.  first_man: the first man's list is to
+// be a permutation (a third bitmap: n > 2).
 __device__ __forceinline__ void count_alike(const int32_t *__restrict__ pref_m, const int32_t *__restrict__ pref_w,
-                                            int n, uint32_t *bitmaps, Control *ctrl) {
+                                            int n, uint32_t *bitmaps, Control *ctrl, bool first_man = false) {
   unsigned women = 0, mid = 0, same = 0;
   const auto fresh = [&](uint32_t *bitmap, int v) {
     const uint32_t bit = 1u << (v & 31);
@@ -128,6 +129,10 @@ __device__ __forceinline__ void count_alike(const int32_t *__restrict__ pref_m, 
     women += fresh(bitmaps, w);
     mid += fresh(bitmaps + ((n + 31) >> 5), v);
     same += v == u;
+    if (first_man) {
+      const int x = __ldg(pref_m + r);
+      if (!fresh(bitmaps + 2 * ((n + 31) >> 5), x)) report(ctrl, kStatusInvalidInput, x);
+    }
   }
   women = __reduce_add_sync(kFullMask, women);
   mid = __reduce_add_sync(kFullMask, mid);
@@ -506,12 +511,16 @@ __global__ void __launch_bounds__(512) k_validate_rows(const int32_t *__restrict
 // A rank-mode instance has no use for it: its lists are compared instead (pref_w
 // on the device, else nullptr).
 __global__ void k_qscatter(const int32_t *__restrict__ pref_m, int n, int K, int qcap, int32_t *__restrict__ qcnt,
-                           uint32_t *__restrict__ qlist, Control *ctrl, const int32_t *__restrict__ pref_w) {
+                           uint32_t *__restrict__ qlist, Control *ctrl, const int32_t *__restrict__ pref_w,
+                           int first_man) {
   __shared__ int s_way;
   if (threadIdx.x == 0)
-    s_way = gate_open(kGateModeQuery, ctrl) ? 1 : pref_w && gate_open(kGateModeRank, ctrl) ? 2 : 0;
+    s_way = gate_open(kGateModeQuery, ctrl)                       ? 1
+            : !pref_w || !gate_open(kGateModeRank, ctrl)          ? 0
+            : first_man && ld_volatile_s32(&ctrl->distinct) == 1 ? 3
+                                                                  : 2;
   __syncthreads();
-  if (s_way == 2) count_alike(pref_m, pref_w, n, reinterpret_cast<uint32_t *>(qcnt), ctrl);
+  if (s_way >= 2) count_alike(pref_m, pref_w, n, reinterpret_cast<uint32_t *>(qcnt), ctrl, s_way == 3);
   if (s_way != 1) return;
   const size_t total = static_cast<size_t>(n) * K;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -1667,18 +1676,19 @@ __global__ void __launch_bounds__(1024) k_turn(const int32_t *__restrict__ pref_
   if (ld_volatile_s32(&ctrl->mode) != kModeRank) return;
   const bool share = may_share && n >= 2 && ctrl->distinct == 1 && ctrl->same_mid == n;
   if (threadIdx.x == 0) {
-    ctrl->swap_try = share;
     ctrl->rank_bulk = may_bulk && rank_bulk_pays(*ctrl, n);
     ctrl->use_filter = ctrl->rank_bulk && rank_bulk_filtered(*ctrl, n);
   }
   if (!share) return;
   for (int w = threadIdx.x; w < n; w += 1024) pos[w] = -1;
   __syncthreads();
+  bool bad = false;  // no permutation: the men's own proposals find out what it does
   for (int r = threadIdx.x; r < n; r += 1024) {
     const int w = __ldg(pref_m + r);
-    if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1)
-      report(ctrl, kStatusInvalidInput, w);
+    bad |= static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1;
   }
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) ctrl->swap_try = !bad;
 }
 
 // ---------------------------------------------------------------------------

@@ -28,12 +28,17 @@
 namespace smpb200 {
 
 // pos[L[r]] = r, with pos preset to -1; an entry out of range or seen twice
-// makes row 0 no permutation.
-__global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl) {
+// makes row 0 no permutation: invalid input (refuse), or no list to share.
+__global__ void k_swap_pos(const int32_t *__restrict__ pref_m, int32_t *__restrict__ pos, int n, Control *ctrl,
+                           int refuse) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const int w = __ldg(pref_m + r);
-    if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1)
-      report(ctrl, kStatusInvalidInput, w);
+    if (static_cast<unsigned>(w) >= static_cast<unsigned>(n) || atomicCAS(pos + w, -1, r) != -1) {
+      if (refuse)
+        report(ctrl, kStatusInvalidInput, w);
+      else
+        ctrl->swap_fail = 1;
+    }
   }
 }
 
@@ -238,7 +243,8 @@ __global__ void __launch_bounds__(256) k_swap_gs(const int32_t *__restrict__ pre
   if (beside) {  // (one look for the CTA, as with the gates)
     int closed = 0;
     if (threadIdx.x == 0 && beside == 1)
-      closed = ld_volatile_s32(&ctrl->distinct_w) <= 1 ||
+      closed = ld_volatile_s32(&ctrl->distinct_w) <= 1 || ld_volatile_s32(&ctrl->swap_fail) ||
+               ld_volatile_s32(&ctrl->status) ||
                (static_cast<int>(blockIdx.x) >= alike_cta && !women_alike(ctrl, n));
     if (threadIdx.x == 0 && beside == 2)
       closed = ld_volatile_s32(&ctrl->swap_fail) || ld_volatile_s32(&ctrl->status) || !ld_volatile_s32(&ctrl->w_differ);
